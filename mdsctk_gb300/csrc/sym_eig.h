@@ -111,8 +111,11 @@ inline void tridiagonalise(std::vector<double> a, int m, std::vector<double>& di
 }
 
 // One implicit QR step with a Wilkinson shift on the unreduced block
-// [lo, hi] of (diag, off), the rotations applied to the columns of z.
-inline void qr_step(std::vector<double>& diag, std::vector<double>& off, int lo, int hi, std::vector<double>& z,
+// [lo, hi] of (diag, off), the rotations applied to the columns of Z, which
+// are the rows of zt: two contiguous rows per rotation. (On Z's own columns,
+// a stride of m, the rotations were most of a solve: 4.5 ms at m = 101
+// against 1.5 ms, same operations in the same order.)
+inline void qr_step(std::vector<double>& diag, std::vector<double>& off, int lo, int hi, std::vector<double>& zt,
                     int m) {
   // shift: the eigenvalue of the trailing 2x2 block closer to diag[hi]
   const double t = off[hi - 1];
@@ -142,11 +145,12 @@ inline void qr_step(std::vector<double>& diag, std::vector<double>& off, int lo,
       y = bulge;
     }
     // Z <- Z R^T on columns k, k+1
+    double* __restrict__ z0 = &zt[(size_t)k * m];
+    double* __restrict__ z1 = z0 + m;
     for (int i = 0; i < m; ++i) {
-      double* row = &z[(size_t)i * m];
-      const double zk = row[k], zk1 = row[k + 1];
-      row[k] = c * zk + s * zk1;
-      row[k + 1] = -s * zk + c * zk1;
+      const double zk = z0[i], zk1 = z1[i];
+      z0[i] = c * zk + s * zk1;
+      z1[i] = -s * zk + c * zk1;
     }
   }
 }
@@ -156,8 +160,10 @@ inline void qr_step(std::vector<double>& diag, std::vector<double>& off, int lo,
 // z (row-major m x m). Returns false if some eigenvalue needs more than 60
 // QR steps (never seen on projected Lanczos matrices).
 inline bool sym_eig(const std::vector<double>& a, int m, std::vector<double>& w, std::vector<double>& z) {
-  std::vector<double> diag, off;
+  std::vector<double> diag, off, zt((size_t)m * m);
   tridiagonalise(a, m, diag, off, z);
+  for (int r = 0; r < m; ++r)
+    for (int c = 0; c < m; ++c) zt[(size_t)c * m + r] = z[(size_t)r * m + c];
   const double eps = std::numeric_limits<double>::epsilon();
   const double tiny = std::numeric_limits<double>::min();
   int hi = m - 1, steps = 0;
@@ -173,18 +179,16 @@ inline bool sym_eig(const std::vector<double>& a, int m, std::vector<double>& w,
     while (lo > 0 && std::fabs(off[lo - 1]) > eps * (std::fabs(diag[lo - 1]) + std::fabs(diag[lo])) + tiny) --lo;
     if (lo > 0) off[lo - 1] = 0.0;
     if (++steps > 60) return false;
-    qr_step(diag, off, lo, hi, z, m);
+    qr_step(diag, off, lo, hi, zt, m);
   }
   std::vector<int> ord(m);
   for (int i = 0; i < m; ++i) ord[i] = i;
   std::sort(ord.begin(), ord.end(), [&](int x, int y) { return diag[x] < diag[y]; });
   w.resize(m);
-  std::vector<double> z2((size_t)m * m);
   for (int c = 0; c < m; ++c) {
     w[c] = diag[ord[c]];
-    for (int r = 0; r < m; ++r) z2[(size_t)r * m + c] = z[(size_t)r * m + ord[c]];
+    for (int r = 0; r < m; ++r) z[(size_t)r * m + c] = zt[(size_t)ord[c] * m + r];
   }
-  z.swap(z2);
   return true;
 }
 
