@@ -11,14 +11,15 @@
 //     w = exp(-d^2 / 2 sigma^2); degrees as decomp_sparse.cpp:162-169 (each
 //     stored entry adds w to both its row and its column, a diagonal entry
 //     twice); entries scaled by d_r^-1/2 d_c^-1/2.
-//  2. SpMV: FP64, one warp per row of the expanded CSR.
+//  2. SpMV: FP64, several lanes per row of the expanded CSR.
 //  3. Thick-restart Lanczos (Wu & Simon 2000; equivalent to ARPACK's
 //     implicitly restarted Lanczos for symmetric matrices) keeping ARPACK's
 //     contract: which='LA', nev, ncv, tol (0 = machine epsilon, converged
 //     when the Ritz estimate <= tol * max(eps^(2/3), |theta|)), maxiter
 //     restarts, start vector from a fixed seed. Full reorthogonalisation
-//     (classical Gram-Schmidt applied twice) by FP64 GEMV kernels; the
-//     projected matrix (ncv x ncv, arrowhead + tridiagonal) is solved on the
+//     (classical Gram-Schmidt, a second time where ARPACK's test asks for
+//     it), the steps of a cycle in one cooperative launch; the projected
+//     matrix (ncv x ncv, arrowhead + tridiagonal) is solved on the
 //     host by Householder tridiagonalisation and implicit symmetric QR steps
 //     with Wilkinson shifts (sym_eig.h).
 //  4. Eigenvalues descending, eigenvectors in the same order, residuals
@@ -449,6 +450,323 @@ __global__ void k_lz_finish_scale(const double* __restrict__ h1, const double* _
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = s_brk ? 0.0 : w[i] * s_scale;
 }
+
+// ---------------------------------------------------------------------------
+// The Lanczos steps j0..m-1 of a cycle in one cooperative launch
+// ---------------------------------------------------------------------------
+// Bound: the FP64 pipe (1.6 FMA a clock and SM, measured) and the latency of
+// the reductions between the steps' passes. Each block owns a range of rows
+// for the whole launch and keeps their piece of the basis in shared memory
+// (all of it up to n x columns of about 30 MB; columns past that stay in
+// global memory, in L2), so a step reads no basis vector from memory:
+//   1. w = A v_j - beta_(j-1) v_(j-1) - alpha_(j-1) v_j on the block's rows.
+//      The recurrence's known term and the last step's alpha, close to this
+//      one's, go first (the projection below adds the rest), so that the
+//      projection removes little and ARPACK's test (dsaitr, after Daniel,
+//      Gragg, Kaufman and Stewart: a second pass when the first leaves ||w||
+//      <= 0.717 of its norm) rarely asks for a second pass; without them it
+//      asked for one in nearly every step.
+//   2. h = V^T w and ||w||^2: partial sums per block, summed over the four
+//      blocks of a cluster, then by every block over the clusters (every
+//      block adding all blocks' sums itself would cost 2.8 us of FP64 pipe).
+//   3. w -= V h, ||w||^2 (again where the test asks), beta_j; w goes out
+//      unnormalised and the next product scales its sums by 1 / beta_j, so
+//      a step has two grid barriers (1.2 us each).
+// All sums are in a fixed order: results are deterministic.
+// 8 graph-launched kernels per step took 45 us (n = 2,000, 101 columns) and
+// 53 us (n = 20,001); this takes 16.6 and 25.8 us, of which at n = 20,001 the
+// product's gathers from L2 7.7, the projections 3.9, the subtraction 4.0 (the
+// FP64 pipe's 3.1 each) and the reductions between them the rest.
+// Every wait for other blocks gives up after about a second, sets *err, and
+// the block returns (a cluster barrier does not wait for returned blocks).
+#define LZ_THREADS 512
+#define LZ_WARPS (LZ_THREADS / 32)
+#define LZ_CLUSTER 4
+#define LZ_MINROWS 32  // rows per block below which more blocks only add to the reductions
+
+struct LzArgs {
+  const int64_t* rp;
+  const int* col;
+  const double* w;   // operator (CSR)
+  int n;
+  double* V;         // locked columns, then the basis v_0..v_m, leading dimension ld
+  int64_t ld;
+  int nlock, j0, m;
+  int cs, rs;        // basis columns kept in shared memory, their stride in rows
+  double brk_tol;
+  double* wbuf;      // [2][n]
+  double* part1;     // [blocks][ldp]
+  double* part2;     // [ldp][clusters]
+  double* npart;     // [blocks]
+  int ldp;
+  double* alpha;
+  double* beta;
+  int* brk;
+  unsigned* bar;     // arrivals at the grid barrier (zeroed before the launch)
+  int* err;
+};
+
+// Shared memory besides the basis: h, partial sums of the projections (at
+// most max(32, ncols / 4) tasks of 4 columns) and of the subtraction, the
+// cross-warp sums.
+static size_t lz_fixed_smem(int ncols) {
+  const size_t dots = (size_t)(2 * LZ_WARPS + (ncols + 4) / 4) * 4;
+  return sizeof(double) * ((size_t)ncols + 1 + dots + 2 * LZ_WARPS * 16 + 64);
+}
+
+__device__ __forceinline__ void lz_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ bool lz_grid_sync(const LzArgs& a, unsigned& arrivals, int* s_ok) {
+  arrivals += gridDim.x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.bar), "r"(1u) : "memory");
+    const long long t0 = clock64();
+    unsigned v;
+    while (true) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+      if (v >= arrivals) break;
+      if (clock64() - t0 > 2000000000ll) {  // about a second
+        atomicExch(a.err, 1);
+        ok = 0;
+        break;
+      }
+    }
+    __threadfence();
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+__global__ void __launch_bounds__(LZ_THREADS, 1) k_lz_cycle(const LzArgs a) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int s_ok, s_again, s_broke;
+  __shared__ double s_before, s_alpha, s_beta, s_scale;  // (by warp 0: scalars that every warp computed would cost FP64 pipe)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = blockIdx.x, G = gridDim.x;
+  const int ncl = G / LZ_CLUSTER, cl = b / LZ_CLUSTER, cr = b % LZ_CLUSTER;
+  const int r0 = (int)((int64_t)a.n * b / G), R = (int)((int64_t)a.n * (b + 1) / G) - r0;
+  double* sV = sm;                              // [cs][rs]
+  double* hs = sV + (size_t)a.cs * a.rs;        // [ncols + 1]
+  double* red = hs + (a.nlock + a.m + 1);       // [64]
+  double* ps = red + 64;                        // [2 LZ_WARPS][16]
+  double* sp = ps + 2 * LZ_WARPS * 16;          // dots partial sums
+  unsigned arrivals = 0;
+  const int have = a.nlock + a.j0 + 1;          // columns on entry
+  for (int c = warp; c < min(have, a.cs); c += LZ_WARPS)
+    for (int r = lane; r < R; r += 32) sV[(size_t)c * a.rs + r] = a.V[(int64_t)c * a.ld + r0 + r];
+  auto colp = [&](int c) -> const double* {
+    return c < a.cs ? sV + (size_t)c * a.rs : a.V + (int64_t)c * a.ld + r0;
+  };
+  // Projections of the block's rows of w onto the columns [0, nc) and, with
+  // norm, w onto itself, over all blocks, into hs[0..nc]. Groups of 8 lanes
+  // take a column each, so a sum needs three shuffles instead of five (each
+  // costs an FP64 add of the whole warp); the rows are split among tasks
+  // only where there are fewer column groups than warps.
+  auto dots = [&](const double* w, int nc, bool norm) -> bool {
+    const int ncn = nc + (norm ? 1 : 0);
+    const int ngrp = (ncn + 3) / 4, RC = max(1, min(8, LZ_WARPS / ngrp));
+    const int per = ((R + RC - 1) / RC + 7) & ~7;
+    for (int task = warp; task < ngrp * RC; task += LZ_WARPS) {
+      const int g = task % ngrp, rc = task / ngrp, l8 = lane & 7;
+      const int c = 4 * g + (lane >> 3);
+      const double* v = c < nc ? colp(c) : w;
+      const int e = c < ncn ? min(R, (rc + 1) * per) : 0;
+      double s = 0.0;
+      for (int r = rc * per + l8; r < e; r += 8) s += v[r] * w[r];
+      for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (l8 == 0 && c < ncn) sp[rc * ngrp * 4 + c] = s;
+    }
+    __syncthreads();
+    for (int c = tid; c < ncn; c += LZ_THREADS) {
+      double s = 0.0;
+      for (int rc = 0; rc < RC; ++rc) s += sp[rc * ngrp * 4 + c];
+      a.part1[(int64_t)b * a.ldp + c] = s;
+    }
+    lz_cluster_sync();
+    for (int c = cr + LZ_CLUSTER * tid; c < ncn; c += LZ_CLUSTER * LZ_THREADS) {
+      double v[LZ_CLUSTER], s = 0.0;
+#pragma unroll
+      for (int i = 0; i < LZ_CLUSTER; ++i) v[i] = __ldcg(a.part1 + (int64_t)(cl * LZ_CLUSTER + i) * a.ldp + c);
+#pragma unroll
+      for (int i = 0; i < LZ_CLUSTER; ++i) s += v[i];
+      a.part2[(int64_t)c * ncl + cl] = s;
+    }
+    if (!lz_grid_sync(a, arrivals, &s_ok)) return false;
+    for (int c0 = 4 * warp; c0 < ncn; c0 += 8 * LZ_WARPS) {
+      // two column groups at a time, five loads each in flight
+      const int l8 = lane & 7;
+      double s[2];
+      double x[2][5];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = c0 + u * 4 * LZ_WARPS + (lane >> 3);
+        s[u] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+          x[u][i] = (c < ncn && l8 + 8 * i < ncl) ? __ldcg(a.part2 + (int64_t)c * ncl + l8 + 8 * i) : 0.0;
+        for (int q = l8 + 40; c < ncn && q < ncl; q += 8) s[u] += __ldcg(a.part2 + (int64_t)c * ncl + q);
+      }
+      const bool two = c0 + 4 * LZ_WARPS < ncn;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (u && !two) break;
+        s[u] += ((x[u][0] + x[u][1]) + (x[u][2] + x[u][3])) + x[u][4];
+        for (int o = 4; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+        const int c = c0 + u * 4 * LZ_WARPS + (lane >> 3);
+        if (l8 == 0 && c < ncn) hs[c] = s[u];
+      }
+    }
+    __syncthreads();
+    return true;
+  };
+  // w -= V[:, 0:nc) hs on the block's rows, then ||w||^2 over all blocks:
+  // s_beta its root, s_scale the root's reciprocal, s_again whether the test
+  // asks for a second pass, s_broke whether the step broke down. A warp's
+  // task is 16 rows x 2 halves of one of P column ranges, about a task per
+  // warp.
+  auto subtract = [&](double* w, int nc) -> bool {
+    const int RG = max(1, (R + 15) / 16), P = (LZ_WARPS + RG - 1) / RG;
+    const int row16 = lane & 15, half = lane >> 4;
+    double q = 0.0;
+    for (int task = warp; task < RG * P; task += LZ_WARPS) {
+      const int rg = task % RG, pp = 2 * (task / RG) + half, r = rg * 16 + row16;
+      const int c0 = nc * pp / (2 * P), c1 = nc * (pp + 1) / (2 * P);
+      double s = 0.0, s2 = 0.0;
+      if (r < R) {
+        int c = c0;
+        for (; c + 1 < min(c1, a.cs); c += 2) {
+          s += sV[(size_t)c * a.rs + r] * hs[c];
+          s2 += sV[(size_t)(c + 1) * a.rs + r] * hs[c + 1];
+        }
+        for (; c < c1; ++c) s += colp(c)[r] * hs[c];
+      }
+      s += s2;
+      s += __shfl_xor_sync(0xffffffffu, s, 16);
+      if (P == 1) {
+        if (half == 0 && r < R) {
+          const double wi = w[r] - s;
+          w[r] = wi;
+          q += wi * wi;
+        }
+      } else if (half == 0) {
+        ps[task * 16 + row16] = s;  // [part][row group][16]
+      }
+    }
+    if (P > 1) {
+      __syncthreads();
+      for (int r = tid; r < R; r += LZ_THREADS) {
+        double s = 0.0, s2 = 0.0;
+        int p = 0;
+        for (; p + 1 < P; p += 2) {
+          s += ps[p * RG * 16 + r];
+          s2 += ps[(p + 1) * RG * 16 + r];
+        }
+        if (p < P) s += ps[p * RG * 16 + r];
+        const double wi = w[r] - (s + s2);
+        w[r] = wi;
+        q += wi * wi;
+      }
+    }
+    for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if (lane == 0) red[warp] = q;
+    __syncthreads();
+    if (warp == 0) {
+      double t = lane < LZ_WARPS ? red[lane] : 0.0;
+      for (int o = LZ_WARPS / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) a.npart[b] = t;
+    }
+    if (!lz_grid_sync(a, arrivals, &s_ok)) return false;
+    if (warp == 0) {
+      double t = 0.0;
+      for (int i = lane; i < G; i += 32) t += __ldcg(a.npart + i);
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) {
+        t = fmax(t, 0.0);
+        const double rs = rsqrt(t), lim = a.brk_tol * fmax(fabs(s_alpha), 1.0);
+        s_scale = rs;
+        s_beta = t > 0.0 ? t * rs : 0.0;
+        s_again = !(t > 0.514089 * s_before);  // 0.717^2
+        s_broke = t <= lim * lim;              // beta_j <= lim
+      }
+    }
+    __syncthreads();
+    return true;
+  };
+
+  double scale = 1.0, bprev = 0.0, aprev = 0.0;
+  for (int j = a.j0; j < a.m; ++j) {
+    const int nc = a.nlock + j + 1;
+    const double* x = (j == a.j0) ? a.V + (int64_t)(nc - 1) * a.ld : a.wbuf + (int64_t)((j + 1) & 1) * a.n;
+    double* w = a.wbuf + (int64_t)(j & 1) * a.n + r0;
+    __syncthreads();  // (the basis columns in shared memory are in place)
+    // 1. the product, eight lanes per row, four elements each in flight;
+    // other blocks' x comes from L2 (whose random sectors bound this pass: the
+    // operator's slice kept in shared memory in a conflict-free layout was no
+    // faster)
+    const double* vprev = colp(max(nc - 2, 0));
+    const double* vj = colp(nc - 1);
+    for (int r = warp * 4 + (lane >> 3); r < ((R + 3) & ~3); r += LZ_WARPS * 4) {
+      double s0 = 0.0, s1 = 0.0;
+      if (r < R) {
+        const int64_t e1 = a.rp[r0 + r + 1];
+        int64_t e = a.rp[r0 + r] + (lane & 7);
+        for (; e + 24 < e1; e += 32) {
+          const int c0 = a.col[e], c1 = a.col[e + 8], c2 = a.col[e + 16], c3 = a.col[e + 24];
+          const double w0 = a.w[e], w1 = a.w[e + 8], w2 = a.w[e + 16], w3 = a.w[e + 24];
+          const double x0 = __ldcg(x + c0), x1 = __ldcg(x + c1), x2 = __ldcg(x + c2), x3 = __ldcg(x + c3);
+          s0 += w0 * x0;
+          s1 += w1 * x1;
+          s0 += w2 * x2;
+          s1 += w3 * x3;
+        }
+        for (; e < e1; e += 8) s0 += a.w[e] * __ldcg(x + a.col[e]);
+      }
+      double s = s0 + s1;
+      for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((lane & 7) == 0 && r < R) {
+        s *= scale;
+        if (j > a.j0) s -= bprev * vprev[r] + aprev * vj[r];
+        w[r] = s;
+      }
+    }
+    __syncthreads();
+    // 2. and 3.
+    if (!dots(w, nc, true)) return;
+    if (tid == 0) {
+      s_alpha = aprev + hs[nc - 1];
+      s_before = hs[nc];
+    }
+    __syncthreads();
+    if (!subtract(w, nc)) return;
+    if (s_again) {  // (the same in every block)
+      if (!dots(w, nc, false)) return;
+      if (tid == 0) s_alpha += hs[nc - 1];
+      __syncthreads();
+      if (!subtract(w, nc)) return;
+    }
+    const bool broke = s_broke != 0;
+    scale = broke ? 0.0 : s_scale;
+    bprev = broke ? 0.0 : s_beta;
+    aprev = broke ? 0.0 : s_alpha;
+    if (b == 0 && tid == 0) {
+      a.alpha[j] = s_alpha;
+      a.beta[j] = s_beta;
+      a.brk[j] = s_broke;
+    }
+    // v_(j+1) (zeros after a breakdown; those steps are redone)
+    for (int r = tid; r < R; r += LZ_THREADS) {
+      const double v = broke ? 0.0 : w[r] * scale;
+      a.V[(int64_t)nc * a.ld + r0 + r] = v;
+      if (nc < a.cs) sV[(size_t)nc * a.rs + r] = v;
+    }
+  }
+}
 __global__ void k_scale_copy(const double* __restrict__ w, double a, int n, double* __restrict__ out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = w[i] * a;
@@ -625,11 +943,17 @@ struct LanczosOut {
   int matvecs = 0;
 };
 
+// by_kernels: the steps as graph-launched kernels, one per pass, instead of
+// the one-launch cycle (k_lz_cycle, twice as fast). For the resident serving
+// model, whose landmark graph mostly falls apart into components: which
+// vectors of the repeated eigenvalue's space a sequence returns is decided by
+// its rounding, and a model rebuilt from the same landmarks has to give the
+// embedding that coordinates served before were taken in.
 // With nlock > 0 the sequence runs on the operator deflated by the nlock
 // orthonormal columns dLock [nlock][n]: every new basis vector is
 // orthogonalised against them as well as against the Lanczos basis.
 static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, int maxiter, double* dX /*n*nev*/,
-                   LanczosOut& out, const double* dLock = nullptr, int nlock = 0,
+                   LanczosOut& out, bool by_kernels = false, const double* dLock = nullptr, int nlock = 0,
                    uint64_t seed = 0x9E3779B97F4A7C15ull) {
   cudaStream_t s = ctx->stream;
   const int n = op.n;
@@ -643,20 +967,82 @@ static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, 
   MDS_TRY(part.alloc(ctx, sizeof(double) * (size_t)nparts * (nlock + m + 1)));
   MDS_TRY(Yd.alloc(ctx, sizeof(double) * (size_t)m * m));
   MDS_TRY(tmp.alloc(ctx, sizeof(double) * (size_t)n * m));
-  DevBuf h1(ctx), h2(ctx), ab(ctx), brk(ctx), npart(ctx), npart1(ctx), flag2(ctx);
-  MDS_TRY(npart.alloc(ctx, sizeof(double) * (size_t)((n + 255) / 256)));
-  MDS_TRY(npart1.alloc(ctx, sizeof(double) * (size_t)((n + 255) / 256)));
-  MDS_TRY(flag2.alloc(ctx, sizeof(int)));
+  DevBuf ab(ctx), brk(ctx), wbuf(ctx), part1(ctx), part2(ctx), npart(ctx), sync(ctx);
+  DevBuf h1(ctx), h2(ctx), npart1(ctx), flag2(ctx);  // (steps by kernels)
   // step graphs by first step of the cycle; destroyed on every return path
   struct Graphs : std::map<int, cudaGraphExec_t> {
     ~Graphs() {
       for (auto& g : *this) cudaGraphExecDestroy(g.second);
     }
   } graphs;
-  MDS_TRY(h1.alloc(ctx, sizeof(double) * (nlock + m + 1)));
-  MDS_TRY(h2.alloc(ctx, sizeof(double) * (nlock + m + 1)));
   MDS_TRY(ab.alloc(ctx, sizeof(double) * 2 * m));
   MDS_TRY(brk.alloc(ctx, sizeof(int) * m));
+  // the cycle kernel's launch: blocks of at least LZ_MINROWS rows, as many
+  // as fit the device at once, in clusters
+  LzArgs lz{};
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  int lz_blocks = 0;
+  if (by_kernels) {
+    MDS_TRY(npart.alloc(ctx, sizeof(double) * (size_t)((n + 255) / 256)));
+    MDS_TRY(npart1.alloc(ctx, sizeof(double) * (size_t)((n + 255) / 256)));
+    MDS_TRY(flag2.alloc(ctx, sizeof(int)));
+    MDS_TRY(h1.alloc(ctx, sizeof(double) * (nlock + m + 1)));
+    MDS_TRY(h2.alloc(ctx, sizeof(double) * (nlock + m + 1)));
+  } else {
+    static bool attr_done = false;
+    static size_t attr_limit = 0;
+    MDS_TRY(mds_allow_dyn_smem(ctx, k_lz_cycle, &attr_done, &attr_limit));
+    const int ncols = nlock + m;
+    const size_t fixed = lz_fixed_smem(ncols);
+    if (fixed > attr_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "ncv=%d too large", m);
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = LZ_CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cfg.blockDim = dim3(LZ_THREADS);
+    cfg.gridDim = dim3(LZ_CLUSTER);
+    cfg.dynamicSmemBytes = attr_limit;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    MDS_CUDA(ctx, cudaOccupancyMaxActiveClusters(&fit, k_lz_cycle, &cfg));
+    if (fit < 1) return mds_fail(ctx, MDS_ERR_CUDA, "the Lanczos kernel does not fit the device");
+    const int want = (n + LZ_MINROWS * LZ_CLUSTER - 1) / (LZ_MINROWS * LZ_CLUSTER);
+    lz_blocks = LZ_CLUSTER * std::max(1, std::min(fit, want));
+    const int R = (n + lz_blocks - 1) / lz_blocks;
+    lz.rs = (R + 7) / 16 * 16 + 8;  // the smallest stride >= R of 8 modulo 16: four columns' rows on distinct banks
+    lz.cs = (int)std::min<size_t>(ncols, (attr_limit - fixed) / (sizeof(double) * lz.rs));
+    cfg.dynamicSmemBytes = fixed + sizeof(double) * (size_t)lz.cs * lz.rs;
+    cfg.gridDim = dim3(lz_blocks);
+    cfg.numAttrs = 2;
+    lz.ldp = ncols + 1;
+    MDS_TRY(wbuf.alloc(ctx, sizeof(double) * 2 * (size_t)n));
+    MDS_TRY(part1.alloc(ctx, sizeof(double) * (size_t)lz_blocks * lz.ldp));
+    MDS_TRY(part2.alloc(ctx, sizeof(double) * (size_t)(lz_blocks / LZ_CLUSTER) * lz.ldp));
+    MDS_TRY(npart.alloc(ctx, sizeof(double) * lz_blocks));
+    MDS_TRY(sync.alloc(ctx, 2 * sizeof(int)));  // barrier arrivals, error
+    lz.rp = op.rp.as<int64_t>();
+    lz.col = op.col.as<int>();
+    lz.w = op.w.as<double>();
+    lz.n = n;
+    lz.V = V.as<double>();
+    lz.ld = ld;
+    lz.nlock = nlock;
+    lz.m = m;
+    lz.brk_tol = std::numeric_limits<double>::epsilon() * 10.0;
+    lz.wbuf = wbuf.as<double>();
+    lz.part1 = part1.as<double>();
+    lz.part2 = part2.as<double>();
+    lz.npart = npart.as<double>();
+    lz.alpha = ab.as<double>();
+    lz.beta = ab.as<double>() + m;
+    lz.brk = brk.as<int>();
+    lz.bar = sync.as<unsigned>();
+    lz.err = sync.as<int>() + 1;
+  }
   double* Vl = V.as<double>();           // locked columns, then the Lanczos basis
   double* Vp = Vl + (int64_t)nlock * ld;  // Lanczos basis v_0..v_m
   if (nlock)
@@ -718,7 +1104,7 @@ static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, 
   int k = 0;
   std::vector<double> theta_k, s_k;  // kept Ritz values and couplings
   std::vector<double> alpha(m, 0.0), beta(m, 0.0);
-  std::vector<double> hh, hh2, T, Z, th;
+  std::vector<double> hh, T, Z, th;
   int restart = 0;
   for (;; ++restart) {
     // Lanczos steps k..m-1 run with no host round trip: the projections,
@@ -727,52 +1113,62 @@ static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, 
     // (invariant subspace, beta_j ~ 0) found then restarts the steps after
     // it from a fresh direction orthogonal to the basis.
     for (int j0 = k; j0 < m;) {
-      // The steps j0..m-1 are one CUDA graph, captured the first time a cycle
-      // starts at j0 (every pointer and size is fixed within this call) and
-      // replayed afterwards: one launch instead of 9 per step.
-      auto git = graphs.find(j0);
-      if (git == graphs.end()) {
-        MDS_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-        for (int j = j0; j < m; ++j) {
-          const int nc = nlock + j + 1;  // full reorthogonalisation (twice)
-          k_spmv<<<spmv_blocks(op.n), 256, 0, s>>>(op.rp.as<int64_t>(), op.col.as<int>(), op.w.as<double>(),
-                                                   Vp + (int64_t)j * ld, op.n, w);
-          // first pass, with ||w||^2 before it (h1[nc]) and the new w's
-          // partial sums (npart1); the second pass only where ARPACK's test
-          // asks for it (k_gemv_t_part)
-          k_gemv_t_part<<<nparts, 256, 0, s>>>(Vl, ld, n, nc, w, part.as<double>(), 1, nullptr, 0, nullptr, nullptr);
-          k_reduce_part<<<(nc + 4) / 4, 128, 0, s>>>(part.as<double>(), nparts, nc + 1, h1.as<double>(), nullptr);
-          k_gemv_sub<<<(n + 255) / 256, 256, sizeof(double) * nc, s>>>(Vl, ld, n, nc, h1.as<double>(), w,
-                                                                        npart1.as<double>(), nullptr, nullptr);
-          k_gemv_t_part<<<nparts, 256, 0, s>>>(Vl, ld, n, nc, w, part.as<double>(), 0, npart1.as<double>(),
-                                               (n + 255) / 256, h1.as<double>() + nc, flag2.as<int>());
-          k_reduce_part<<<(nc + 3) / 4, 128, 0, s>>>(part.as<double>(), nparts, nc, h2.as<double>(), flag2.as<int>());
-          k_gemv_sub<<<(n + 255) / 256, 256, sizeof(double) * nc, s>>>(Vl, ld, n, nc, h2.as<double>(), w,
-                                                                       npart.as<double>(), flag2.as<int>(),
-                                                                       npart1.as<double>());
-          k_lz_finish_scale<<<(n + 255) / 256, 256, 0, s>>>(h1.as<double>(), h2.as<double>(), npart.as<double>(),
-                                                             (n + 255) / 256, nlock + j, j, eps * 10.0,
-                                                             ab.as<double>(), ab.as<double>() + m, brk.as<int>(), w,
-                                                             n, Vp + (int64_t)(j + 1) * ld);
+      if (by_kernels) {
+        // The steps j0..m-1 are one CUDA graph, captured the first time a cycle
+        // starts at j0 (every pointer and size is fixed within this call) and
+        // replayed afterwards: one launch instead of 9 per step.
+        auto git = graphs.find(j0);
+        if (git == graphs.end()) {
+          MDS_CUDA(ctx, cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+          for (int j = j0; j < m; ++j) {
+            const int nc = nlock + j + 1;  // full reorthogonalisation (twice)
+            k_spmv<<<spmv_blocks(op.n), 256, 0, s>>>(op.rp.as<int64_t>(), op.col.as<int>(), op.w.as<double>(),
+                                                     Vp + (int64_t)j * ld, op.n, w);
+            // first pass, with ||w||^2 before it (h1[nc]) and the new w's
+            // partial sums (npart1); the second pass only where ARPACK's test
+            // asks for it (k_gemv_t_part)
+            k_gemv_t_part<<<nparts, 256, 0, s>>>(Vl, ld, n, nc, w, part.as<double>(), 1, nullptr, 0, nullptr, nullptr);
+            k_reduce_part<<<(nc + 4) / 4, 128, 0, s>>>(part.as<double>(), nparts, nc + 1, h1.as<double>(), nullptr);
+            k_gemv_sub<<<(n + 255) / 256, 256, sizeof(double) * nc, s>>>(Vl, ld, n, nc, h1.as<double>(), w,
+                                                                          npart1.as<double>(), nullptr, nullptr);
+            k_gemv_t_part<<<nparts, 256, 0, s>>>(Vl, ld, n, nc, w, part.as<double>(), 0, npart1.as<double>(),
+                                                 (n + 255) / 256, h1.as<double>() + nc, flag2.as<int>());
+            k_reduce_part<<<(nc + 3) / 4, 128, 0, s>>>(part.as<double>(), nparts, nc, h2.as<double>(), flag2.as<int>());
+            k_gemv_sub<<<(n + 255) / 256, 256, sizeof(double) * nc, s>>>(Vl, ld, n, nc, h2.as<double>(), w,
+                                                                         npart.as<double>(), flag2.as<int>(),
+                                                                         npart1.as<double>());
+            k_lz_finish_scale<<<(n + 255) / 256, 256, 0, s>>>(h1.as<double>(), h2.as<double>(), npart.as<double>(),
+                                                               (n + 255) / 256, nlock + j, j, eps * 10.0,
+                                                               ab.as<double>(), ab.as<double>() + m, brk.as<int>(), w,
+                                                               n, Vp + (int64_t)(j + 1) * ld);
+          }
+          cudaGraph_t g = nullptr;
+          cudaError_t ce = cudaStreamEndCapture(s, &g);
+          if (ce != cudaSuccess) return mds_fail(ctx, MDS_ERR_CUDA, "Lanczos step capture: %s", cudaGetErrorString(ce));
+          cudaGraphExec_t ge = nullptr;
+          ce = cudaGraphInstantiate(&ge, g, 0);
+          cudaGraphDestroy(g);
+          if (ce != cudaSuccess) return mds_fail(ctx, MDS_ERR_CUDA, "Lanczos step graph: %s", cudaGetErrorString(ce));
+          git = graphs.emplace(j0, ge).first;
         }
-        cudaGraph_t g = nullptr;
-        cudaError_t ce = cudaStreamEndCapture(s, &g);
-        if (ce != cudaSuccess) return mds_fail(ctx, MDS_ERR_CUDA, "Lanczos step capture: %s", cudaGetErrorString(ce));
-        cudaGraphExec_t ge = nullptr;
-        ce = cudaGraphInstantiate(&ge, g, 0);
-        cudaGraphDestroy(g);
-        if (ce != cudaSuccess) return mds_fail(ctx, MDS_ERR_CUDA, "Lanczos step graph: %s", cudaGetErrorString(ce));
-        git = graphs.emplace(j0, ge).first;
+        MDS_CUDA(ctx, cudaGraphLaunch(git->second, s));
+        ctx->stats.launches += 8 * (m - j0);
+        MDS_CUDA(ctx, cudaGetLastError());
+      } else {
+        MDS_CUDA(ctx, cudaMemsetAsync(sync.p, 0, 2 * sizeof(int), s));
+        lz.j0 = j0;
+        MDS_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_lz_cycle, lz));
+        ctx->stats.launches++;
       }
-      MDS_CUDA(ctx, cudaGraphLaunch(git->second, s));
       out.matvecs += m - j0;
-      ctx->stats.launches += 8 * (m - j0);
-      MDS_CUDA(ctx, cudaGetLastError());
       std::vector<double> hab(2 * m);
       std::vector<int> hbrk(m);
       MDS_CUDA(ctx, cudaMemcpyAsync(hab.data(), ab.p, sizeof(double) * 2 * m, cudaMemcpyDeviceToHost, s));
       MDS_CUDA(ctx, cudaMemcpyAsync(hbrk.data(), brk.p, sizeof(int) * m, cudaMemcpyDeviceToHost, s));
+      int herr = 0;
+      if (lz.err) MDS_CUDA(ctx, cudaMemcpyAsync(&herr, lz.err, sizeof(int), cudaMemcpyDeviceToHost, s));
       MDS_CUDA(ctx, cudaStreamSynchronize(s));
+      if (herr) return mds_fail(ctx, MDS_ERR_TIMEOUT, "Lanczos steps: a bounded wait between blocks timed out");
       int jb = -1;
       for (int j = j0; j < m; ++j) {
         alpha[j] = hab[j];
@@ -877,8 +1273,8 @@ static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, 
 // (dropping the smallest) and the check repeats.
 // Eigenvalues within 1e-10 of the nev-th are interchangeable with it.
 static int lanczos_complete(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, int maxiter, double* dX,
-                            LanczosOut& out) {
-  MDS_TRY(lanczos(ctx, op, nev, ncv, tol, maxiter, dX, out));
+                            LanczosOut& out, bool by_kernels = false) {
+  MDS_TRY(lanczos(ctx, op, nev, ncv, tol, maxiter, dX, out, by_kernels));
   const int n = op.n;
   // The check runs until the deflated top Ritz value converges (to 1e-8, at
   // most 30 restarts of 40 vectors): crowded eigenvalues just below a missed
@@ -896,7 +1292,7 @@ static int lanczos_complete(mds_ctx* ctx, const SymOp& op, int nev, int ncv, dou
   for (int pass = 0; pass < nev; ++pass) {
     const uint64_t seed = 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull * (uint64_t)(pass + 1);
     LanczosOut o2;
-    MDS_TRY(lanczos(ctx, op, 1, ncv2, 1e-8, 30, y.as<double>(), o2, dX, nev, seed));
+    MDS_TRY(lanczos(ctx, op, 1, ncv2, 1e-8, 30, y.as<double>(), o2, by_kernels, dX, nev, seed));
     out.matvecs += o2.matvecs;
     const double th = o2.evals[0], lo = out.evals[nev - 1];
     if (!(th > lo + 1e-10 * std::max(1.0, std::fabs(lo)))) break;
@@ -909,7 +1305,7 @@ static int lanczos_complete(mds_ctx* ctx, const SymOp& op, int nev, int ncv, dou
       copy = std::fabs(th - out.evals[x]) <= 1e-9 * std::max(1.0, std::fabs(out.evals[x]));
     if (!copy) break;
     o2 = LanczosOut();  // converge the missed pair to the requested tolerance
-    MDS_TRY(lanczos(ctx, op, 1, ncv2, tol, maxiter, y.as<double>(), o2, dX, nev, seed));
+    MDS_TRY(lanczos(ctx, op, 1, ncv2, tol, maxiter, y.as<double>(), o2, by_kernels, dX, nev, seed));
     out.matvecs += o2.matvecs;
     int p = nev - 1;
     while (p > 0 && out.evals[p - 1] < o2.evals[0]) --p;
@@ -1067,16 +1463,19 @@ static int decomp_impl(mds_ctx* ctx, int n, const int32_t* pcol, const int32_t* 
   if (resid) {
     DevBuf Az(ctx), part(ctx);
     MDS_TRY(Az.alloc(ctx, sizeof(double) * n));
-    MDS_TRY(part.alloc(ctx, sizeof(double) * 256));
+    MDS_TRY(part.alloc(ctx, sizeof(double) * 256 * (size_t)nev));
     for (int x = 0; x < nev; ++x) {
       spmv(ctx, op, pX + (int64_t)x * n, Az.as<double>());
       ctx->stats.launches++;
-      k_resid_part<<<256, 256, 0, s>>>(Az.as<double>(), pX + (int64_t)x * n, lo.evals[x], n, part.as<double>());
-      std::vector<double> hpart(256);
-      MDS_CUDA(ctx, cudaMemcpyAsync(hpart.data(), part.p, sizeof(double) * 256, cudaMemcpyDeviceToHost, s));
-      MDS_CUDA(ctx, cudaStreamSynchronize(s));
+      k_resid_part<<<256, 256, 0, s>>>(Az.as<double>(), pX + (int64_t)x * n, lo.evals[x], n,
+                                       part.as<double>() + 256 * (size_t)x);
+    }
+    std::vector<double> hpart(256 * (size_t)nev);
+    MDS_CUDA(ctx, cudaMemcpyAsync(hpart.data(), part.p, sizeof(double) * hpart.size(), cudaMemcpyDeviceToHost, s));
+    MDS_CUDA(ctx, cudaStreamSynchronize(s));
+    for (int x = 0; x < nev; ++x) {
       double ss = 0;
-      for (double v : hpart) ss += v;
+      for (int i = 0; i < 256; ++i) ss += hpart[256 * (size_t)x + i];
       resid[x] = std::sqrt(ss) / std::fabs(lo.evals[x]);
     }
   }
@@ -1159,7 +1558,7 @@ int decomp_resident(mds_ctx* ctx, int n, const int* dpcol, const int* dirow, con
   SymOp op;
   MDS_TRY(build_symop(ctx, n, dpcol, dirow, ddist, sigma, op));
   LanczosOut lo;
-  MDS_TRY(lanczos_complete(ctx, op, nev, ncv, tol, maxiter, dZ, lo));
+  MDS_TRY(lanczos_complete(ctx, op, nev, ncv, tol, maxiter, dZ, lo, true));
   MDS_CUDA(ctx, cudaMemcpyAsync(ddinv, op.dinv.p, sizeof(double) * n, cudaMemcpyDeviceToDevice, ctx->stream));
   MDS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   evals = lo.evals;
