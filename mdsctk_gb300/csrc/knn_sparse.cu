@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "knn_common.cuh"
+#include "overlap_tc.cuh"
 
 #define SP_THREADS 256
 #define SP_CHUNK 1024
@@ -147,21 +148,29 @@ static size_t sparse_knn_smem(int k, int mode) {
 // shared memory by cp.async; the squared distances are exact integers, so
 // each row's k+1 smallest (value, index) keys are kept directly (reference
 // tiles are visited in index order, so a later tie never displaces an earlier
-// one) and no recheck is needed.
+// one) and no recheck is needed. Where the byte rows of the tensor-core
+// product (overlap_tc.cu) fit and its tiles fill the device, that takes the
+// call instead (see mds_knn_data_sparse).
 // ---------------------------------------------------------------------------
 #define BN_TM 32
 #define BN_TN 64
 #define BN_KW 32  // words per K-chunk
 #define BN_WS 36  // words per staged row (bank spread, 16-byte rows)
 
-// CSR rows -> bit sets [n][W] (W words of 32 bits, zero padded)
-__global__ void k_bitset(const int64_t* __restrict__ off, const int* __restrict__ idx, int W,
-                         unsigned* __restrict__ bits) {
+// CSR rows -> bit sets [n][W] (W words of 32 bits, zero padded), with the
+// check that they are binary: *bad (zeroed by the caller) is set when a value
+// is not 1.0 or a row's indices do not ascend strictly within [0, 32 W).
+__global__ void k_bitset(const int64_t* __restrict__ off, const int* __restrict__ idx, const double* __restrict__ val,
+                         int W, unsigned* __restrict__ bits, int* __restrict__ bad) {
   const int r = blockIdx.x;
   unsigned* b = bits + (int64_t)r * W;
-  for (int64_t e = off[r] + threadIdx.x; e < off[r + 1]; e += blockDim.x) {
+  const int64_t e0 = off[r];
+  for (int64_t e = e0 + threadIdx.x; e < off[r + 1]; e += blockDim.x) {
     const int i = idx[e];
-    atomicOr(b + (i >> 5), 1u << (i & 31));
+    if (val[e] != 1.0 || i < 0 || (i >> 5) >= W || (e > e0 && i <= idx[e - 1]))
+      *bad = 1;
+    else
+      atomicOr(b + (i >> 5), 1u << (i & 31));
   }
 }
 
@@ -292,13 +301,15 @@ static size_t bin_knn_smem(int k) {
          sizeof(uint64_t) * BN_TM * next_pow2(k + 1 + BN_TN) + 16;
 }
 
-// every value exactly 1.0 and every row's indices strictly ascending and >= 0
-static bool binary_rows(const int64_t* off, const int32_t* idx, const double* val, int n, int* dmax) {
+// Whether the rows may be binary (a look at the first values; the kernels
+// check every entry), and the largest index if their indices ascend: the
+// last one of some row. (Checking every entry on the host took 74 ms for 37 M
+// contacts, most of the call.)
+static bool maybe_binary(const int64_t* off, const int32_t* idx, const double* val, int n, int* dmax) {
+  for (int64_t e = 0; e < std::min<int64_t>(off[n], 64); ++e)
+    if (val[e] != 1.0) return false;
   for (int r = 0; r < n; ++r)
-    for (int64_t e = off[r]; e < off[r + 1]; ++e) {
-      if (val[e] != 1.0 || idx[e] < 0 || (e > off[r] && idx[e] <= idx[e - 1])) return false;
-      *dmax = std::max(*dmax, idx[e]);
-    }
+    if (off[r + 1] > off[r]) *dmax = std::max(*dmax, idx[off[r + 1] - 1]);
   return true;
 }
 
@@ -315,66 +326,113 @@ __device__ __forceinline__ bool contact_exact(const float* a, const float* b, do
   }
   return __dmul_rn(__dsqrt_rn(d), 10.0) < eps;
 }
-__device__ __forceinline__ bool contact_of(const float* a, const float* b, double eps, float eps_lo, float eps_hi) {
+// lo2 and hi2: the squares (nm^2) of eps / 10 less and plus 1e-5 of itself (-1
+// for eps <= 0, which no distance is below); the FP32 square is within 1e-6
+__device__ __forceinline__ bool contact_of(const float* a, const float* b, double eps, float lo2, float hi2) {
   const float t0 = a[0] - b[0], t1 = a[1] - b[1], t2 = a[2] - b[2];
-  const float d = sqrtf(fmaf(t0, t0, fmaf(t1, t1, t2 * t2))) * 10.0f;  // within ~1e-6 relative
-  if (d < eps_lo) return true;
-  if (d > eps_hi) return false;
+  const float d2 = fmaf(t0, t0, fmaf(t1, t1, t2 * t2));
+  if (d2 < lo2) return true;
+  if (d2 > hi2) return false;
   return contact_exact(a, b, eps);
 }
 
-// mode 0: count each frame's contacts into counts[f]; mode 1: write them in
-// ascending grid order at idx[offsets[f] ...]. One block per frame.
+// Each frame's contacts as a bit mask over the grid (mask [nframes][words],
+// or null: only counted), counts[f] their number. One block per frame, its two
+// groups' coordinates in shared memory; a warp tests 32 grid positions at a
+// time, whose ballot is a mask word, and carries its position (i, j) along
+// instead of dividing. Issue-bound: 185 M pairs of 8,000 frames in 275 us
+// (a 64-bit division and two gathers per pair, for the count and again for the
+// indices: 630 us each).
+#define CP_STAGE 2048  // group atoms kept in shared memory (else read from global memory)
 __global__ void __launch_bounds__(SP_THREADS)
-k_contact(const float* __restrict__ xyz, int natoms, const int* __restrict__ g1, int n1, const int* __restrict__ g2,
-          int n2, double eps, int mode, int64_t* __restrict__ counts, const int64_t* __restrict__ offsets,
-          int* __restrict__ idx) {
+k_contact_mask(const float* __restrict__ xyz, int natoms, const int* __restrict__ g1, int n1,
+               const int* __restrict__ g2, int n2, double eps, int words, unsigned* __restrict__ mask,
+               int64_t* __restrict__ counts) {
+  __shared__ float sx[3 * CP_STAGE];
   __shared__ int wsum[SP_THREADS / 32];
-  __shared__ int64_t s_base;
-  const int f = blockIdx.x;
+  const int f = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* x = xyz + (int64_t)f * natoms * 3;
-  const float eps_lo = (float)(eps * (1.0 - 1e-5)), eps_hi = (float)(eps * (1.0 + 1e-5));
-  const int64_t total = (int64_t)n1 * n2;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_base = (mode == 1) ? offsets[f] : 0;
-  int64_t mine = 0;
-  __syncthreads();
-  for (int64_t p0 = 0; p0 < total; p0 += blockDim.x) {
-    const int64_t p = p0 + threadIdx.x;
-    bool hit = false;
-    if (p < total) {
-      const int i = (int)(p / n2), j = (int)(p % n2);
-      const float* a = x + 3 * (int64_t)g1[i];
-      const float* b = x + 3 * (int64_t)g2[j];
-      const float av[3] = {a[0], a[1], a[2]}, bv[3] = {b[0], b[1], b[2]};
-      hit = contact_of(av, bv, eps, eps_lo, eps_hi);
+  const bool staged = n1 + n2 <= CP_STAGE;
+  if (staged) {
+    for (int t = threadIdx.x; t < n1 + n2; t += blockDim.x) {
+      const float* a = x + 3 * (int64_t)(t < n1 ? g1[t] : g2[t - n1]);
+      sx[t] = a[0];
+      sx[CP_STAGE + t] = a[1];
+      sx[2 * CP_STAGE + t] = a[2];
     }
-    if (mode == 0) {
-      mine += hit ? 1 : 0;
-      continue;
-    }
-    // ordered compaction of this chunk: warp ballots, then warp offsets
-    const unsigned bal = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) wsum[warp] = __popc(bal);
-    __syncthreads();
-    int before = 0, chunk = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      before += (w < warp) ? wsum[w] : 0;
-      chunk += wsum[w];
-    }
-    if (hit) idx[s_base + before + __popc(bal & ((1u << lane) - 1u))] = (int)p;
-    __syncthreads();
-    if (threadIdx.x == 0) s_base += chunk;
     __syncthreads();
   }
-  if (mode == 0) {
-    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if (lane == 0) wsum[warp] = (int)mine;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int64_t t = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += wsum[w];
-      counts[f] = t;
+  const double lo = 0.1 * eps * (1.0 - 1e-5), hi = 0.1 * eps * (1.0 + 1e-5);
+  const float lo2 = eps <= 0.0 ? -1.0f : (float)(lo * lo), hi2 = eps <= 0.0 ? -1.0f : (float)(hi * hi);
+  const unsigned total = (unsigned)n1 * (unsigned)n2;  // < 2^31
+  const unsigned step = blockDim.x, di = step / (unsigned)n2, dj = step % (unsigned)n2;
+  unsigned p = threadIdx.x, i = p / (unsigned)n2, j = p % (unsigned)n2;
+  int mine = 0;
+  for (unsigned w = warp; w < (unsigned)words; w += step / 32) {
+    bool hit = false;
+    if (p < total) {
+      float av[3], bv[3];
+      if (staged) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          av[c] = sx[c * CP_STAGE + i];
+          bv[c] = sx[c * CP_STAGE + n1 + j];
+        }
+      } else {
+        const float* a = x + 3 * (int64_t)g1[i];
+        const float* b = x + 3 * (int64_t)g2[j];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          av[c] = a[c];
+          bv[c] = b[c];
+        }
+      }
+      hit = contact_of(av, bv, eps, lo2, hi2);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+    mine += __popc(bal);
+    if (mask && lane == 0) mask[(int64_t)f * words + w] = bal;
+    p += step;
+    i += di;
+    j += dj;
+    if (j >= (unsigned)n2) {
+      j -= (unsigned)n2;
+      ++i;
+    }
+  }
+  if (lane == 0) wsum[warp] = mine;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int64_t t = 0;
+    for (int w = 0; w < SP_THREADS / 32; ++w) t += wsum[w];
+    counts[f] = t;
+  }
+}
+
+// The mask's grid positions in ascending order at idx[offsets[f] ...]. One
+// block per frame; a warp takes a contiguous piece of the words, lane l bit l
+// of each, so the writes of a word are one run.
+__global__ void __launch_bounds__(SP_THREADS)
+k_contact_list(const unsigned* __restrict__ mask, int words, const int64_t* __restrict__ offsets,
+               int* __restrict__ idx) {
+  constexpr int NW = SP_THREADS / 32;
+  __shared__ int wsum[NW];
+  const int f = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned* m = mask + (int64_t)f * words;
+  const int per = (words + NW - 1) / NW, w0 = min(words, warp * per), w1 = min(words, w0 + per);
+  int c = 0;
+  for (int w = w0 + lane; w < w1; w += 32) c += __popc(m[w]);
+  c = __reduce_add_sync(0xffffffffu, c);
+  if (lane == 0) wsum[warp] = c;
+  __syncthreads();
+  int64_t at = offsets[f];
+  for (int w = 0; w < warp; ++w) at += wsum[w];
+  for (int b = w0; b < w1; b += 32) {
+    const unsigned mine = (b + lane < w1) ? m[b + lane] : 0u;
+    for (int t = 0; t < 32 && b + t < w1; ++t) {
+      const unsigned word = __shfl_sync(0xffffffffu, mine, t);
+      if ((word >> lane) & 1u) idx[at + __popc(word & ((1u << lane) - 1u))] = 32 * (b + t) + lane;
+      at += __popc(word);
     }
   }
 }
@@ -447,53 +505,101 @@ extern "C" int mds_knn_data_sparse(mds_ctx* ctx, const int64_t* ref_off, const i
   }
   MDS_TRY(dd.alloc(ctx, sizeof(double) * width * n_fit));
   MDS_TRY(di.alloc(ctx, sizeof(int) * width * n_fit));
-  // binary vectors: bit sets and popcount tiles (exact, no walk per pair)
+  // binary vectors: the overlaps of 0/1 rows (exact, no walk per pair)
   int dmax = -1;
-  const bool binary = !full && binary_rows(ref_off, ref_idx, ref_val, n_ref, &dmax) &&
-                      (same || binary_rows(fit_off, fit_idx, fit_val, n_fit, &dmax)) && dmax < (1 << 24) - 1;
+  const bool binary = !full && maybe_binary(ref_off, ref_idx, ref_val, n_ref, &dmax) &&
+                      (same || maybe_binary(fit_off, fit_idx, fit_val, n_fit, &dmax)) && dmax < (1 << 24) - 1;
   const int W = mds_round_up(std::max(dmax + 1, 1), 32 * BN_KW) / 32;
   if (binary && (size_t)W * 4 * ((size_t)n_ref + (same ? 0 : n_fit)) <= ((size_t)8 << 30)) {
-    DevBuf br(ctx), bf(ctx), cr(ctx), cf(ctx);
-    MDS_TRY(br.alloc(ctx, sizeof(unsigned) * (size_t)W * n_ref));
-    MDS_TRY(cr.alloc(ctx, sizeof(int) * n_ref));
-    MDS_CUDA(ctx, cudaMemsetAsync(br.p, 0, sizeof(unsigned) * (size_t)W * n_ref, s));
-    std::vector<int> hc(std::max(n_ref, n_fit));
-    for (int r = 0; r < n_ref; ++r) hc[r] = (int)(ref_off[r + 1] - ref_off[r]);
-    MDS_CUDA(ctx, cudaMemcpyAsync(cr.p, hc.data(), sizeof(int) * n_ref, cudaMemcpyHostToDevice, s));
-    MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    k_bitset<<<n_ref, 128, 0, s>>>(dro.as<int64_t>(), dri.as<int>(), W, br.as<unsigned>());
-    const unsigned* pbf = br.as<unsigned>();
-    const int* pcf = cr.as<int>();
-    if (!same) {
-      MDS_TRY(bf.alloc(ctx, sizeof(unsigned) * (size_t)W * n_fit));
-      MDS_TRY(cf.alloc(ctx, sizeof(int) * n_fit));
-      MDS_CUDA(ctx, cudaMemsetAsync(bf.p, 0, sizeof(unsigned) * (size_t)W * n_fit, s));
-      MDS_CUDA(ctx, cudaStreamSynchronize(s));  // hc is reused
-      for (int r = 0; r < n_fit; ++r) hc[r] = (int)(fit_off[r + 1] - fit_off[r]);
-      MDS_CUDA(ctx, cudaMemcpyAsync(cf.p, hc.data(), sizeof(int) * n_fit, cudaMemcpyHostToDevice, s));
-      k_bitset<<<n_fit, 128, 0, s>>>(pfo, pfi, W, bf.as<unsigned>());
-      pbf = bf.as<unsigned>();
-      pcf = cf.as<int>();
-    }
-    MDS_CUDA(ctx, cudaGetLastError());
     const size_t bsm = bin_knn_smem(k);
     static bool bin_done = false;
     static size_t bin_limit = 0;
     MDS_TRY(mds_allow_dyn_smem(ctx, k_bin_knn, &bin_done, &bin_limit));
-    if (bsm > bin_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "k=%d too large", k);
-    ctx->stats.launches = same ? 2 : 3;
-    k_bin_knn<<<(n_fit + BN_TM - 1) / BN_TM, SP_THREADS, bsm, s>>>(pbf, pcf, n_fit, br.as<unsigned>(), cr.as<int>(),
-                                                                    n_ref, W, k, dd.as<double>(), di.as<int>());
-    MDS_CUDA(ctx, cudaGetLastError());
-    MDS_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
-    MDS_CUDA(ctx, cudaMemcpyAsync(out_d, dd.p, sizeof(double) * width * n_fit, cudaMemcpyDeviceToHost, s));
-    MDS_CUDA(ctx, cudaMemcpyAsync(out_i, di.p, sizeof(int) * width * n_fit, cudaMemcpyDeviceToHost, s));
-    MDS_CUDA(ctx, cudaStreamSynchronize(s));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
-    ctx->stats.screen_ms = ms;
-    ctx->stats.passes = 1;
-    return MDS_OK;
+    DevBuf br(ctx), bf(ctx), cr(ctx), cf(ctx), bad(ctx);
+    MDS_TRY(bad.alloc(ctx, sizeof(int)));
+    MDS_CUDA(ctx, cudaMemsetAsync(bad.p, 0, sizeof(int), s));
+    MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
+    ctx->stats.launches = 0;
+    // The tensor-core product needs eight times the bit sets' memory and three
+    // launches a panel. It takes every set whose tiles of 128 x 256 pairs reach
+    // half the SMs: 2,100 rows of 23,104 bits 0.24 ms (2,048 rows by popcount:
+    // 2.9 ms), of 2,000 bits 0.09 ms (1.4 ms). Popcount tiles (two launches,
+    // which is what small sets are counted on to take) below that, 1.0 ms at
+    // 1,400 rows of 2,000 bits, and where the byte rows do not fit.
+    const int64_t K = overlap_width(dmax + 1);
+    const size_t bytes = (size_t)K * ((size_t)n_ref + (same ? 0 : n_fit));
+    bool tc = overlap_tiles(n_fit, n_ref) >= ctx->num_sms / 2 && bytes <= ((size_t)16 << 30);
+    int hbad = 0;
+    auto read_bad = [&]() -> int {
+      MDS_CUDA(ctx, cudaMemcpyAsync(&hbad, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+      MDS_CUDA(ctx, cudaStreamSynchronize(s));
+      return MDS_OK;
+    };
+    auto by_product = [&]() -> int {
+      MDS_TRY(br.alloc(ctx, (size_t)K * n_ref));
+      if (!same) MDS_TRY(bf.alloc(ctx, (size_t)K * n_fit));
+      MDS_TRY(cr.alloc(ctx, sizeof(int) * overlap_count_pad(n_ref)));
+      MDS_TRY(launch_rows_e4m3(ctx, dro.as<int64_t>(), dri.as<int>(), drv.as<double>(), n_ref, K,
+                               br.as<unsigned char>(), cr.as<int>(), bad.as<int>()));
+      if (!same) {
+        MDS_TRY(cf.alloc(ctx, sizeof(int) * n_fit));
+        MDS_TRY(launch_rows_e4m3(ctx, pfo, pfi, pfv, n_fit, K, bf.as<unsigned char>(), cf.as<int>(), bad.as<int>()));
+      }
+      MDS_TRY(read_bad());
+      if (hbad || bsm > bin_limit) return MDS_OK;
+      return overlap_knn(ctx, same ? br.as<unsigned char>() : bf.as<unsigned char>(),
+                         same ? cr.as<int>() : cf.as<int>(), n_fit, br.as<unsigned char>(), cr.as<int>(), n_ref, K, k,
+                         dd.as<double>(), di.as<int>());
+    };
+    auto by_popcount = [&]() -> int {
+      std::vector<int> hc;
+      auto bitset = [&](const int64_t* hoff, const int64_t* off, const int* idx, const double* val, int n, DevBuf& bits,
+                        DevBuf& cnt) -> int {
+        MDS_TRY(bits.alloc(ctx, sizeof(unsigned) * (size_t)W * n));
+        MDS_TRY(cnt.alloc(ctx, sizeof(int) * n));
+        MDS_CUDA(ctx, cudaMemsetAsync(bits.p, 0, sizeof(unsigned) * (size_t)W * n, s));
+        hc.resize(n);
+        for (int r = 0; r < n; ++r) hc[r] = (int)(hoff[r + 1] - hoff[r]);
+        MDS_CUDA(ctx, cudaMemcpyAsync(cnt.p, hc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
+        MDS_CUDA(ctx, cudaStreamSynchronize(s));  // hc is reused
+        ctx->stats.launches++;
+        k_bitset<<<n, 128, 0, s>>>(off, idx, val, W, bits.as<unsigned>(), bad.as<int>());
+        MDS_CUDA(ctx, cudaGetLastError());
+        return MDS_OK;
+      };
+      MDS_TRY(bitset(ref_off, dro.as<int64_t>(), dri.as<int>(), drv.as<double>(), n_ref, br, cr));
+      if (!same) MDS_TRY(bitset(fit_off, pfo, pfi, pfv, n_fit, bf, cf));
+      MDS_TRY(read_bad());
+      if (hbad || bsm > bin_limit) return MDS_OK;
+      ctx->stats.launches++;
+      k_bin_knn<<<(n_fit + BN_TM - 1) / BN_TM, SP_THREADS, bsm, s>>>(
+          same ? br.as<unsigned>() : bf.as<unsigned>(), same ? cr.as<int>() : cf.as<int>(), n_fit, br.as<unsigned>(),
+          cr.as<int>(), n_ref, W, k, dd.as<double>(), di.as<int>());
+      MDS_CUDA(ctx, cudaGetLastError());
+      return MDS_OK;
+    };
+    int rc = tc ? by_product() : MDS_OK;
+    if (tc && rc == MDS_ERR_NOMEM) {  // (a small HBM budget)
+      br.release();
+      bf.release();
+      mds_trim_cache(ctx, 0);
+      tc = false;
+      rc = MDS_OK;
+    }
+    MDS_TRY(rc);
+    if (!tc) MDS_TRY(by_popcount());
+    if (!hbad) {
+      if (bsm > bin_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "k=%d too large", k);
+      MDS_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
+      MDS_CUDA(ctx, cudaMemcpyAsync(out_d, dd.p, sizeof(double) * width * n_fit, cudaMemcpyDeviceToHost, s));
+      MDS_CUDA(ctx, cudaMemcpyAsync(out_i, di.p, sizeof(int) * width * n_fit, cudaMemcpyDeviceToHost, s));
+      MDS_CUDA(ctx, cudaStreamSynchronize(s));
+      float ms = 0;
+      cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
+      ctx->stats.screen_ms = ms;
+      ctx->stats.passes = 1;
+      return MDS_OK;
+    }
   }
   const size_t smem = sparse_knn_smem(k, mode);
   static bool attr_done = false;
@@ -541,8 +647,16 @@ extern "C" int mds_contact_profile(mds_ctx* ctx, const float* xyz, int nframes, 
   MDS_CUDA(ctx, cudaMemcpyAsync(dx.p, xyz, xbytes, cudaMemcpyHostToDevice, s));
   MDS_CUDA(ctx, cudaMemcpyAsync(dg1.p, g1, sizeof(int) * n1, cudaMemcpyHostToDevice, s));
   MDS_CUDA(ctx, cudaMemcpyAsync(dg2.p, g2, sizeof(int) * n2, cudaMemcpyHostToDevice, s));
-  k_contact<<<nframes, SP_THREADS, 0, s>>>(dx.as<float>(), natoms, dg1.as<int>(), n1, dg2.as<int>(), n2, eps, 0,
-                                           dcnt.as<int64_t>(), nullptr, nullptr);
+  const int words = (int)(((int64_t)n1 * n2 + 31) / 32);
+  // the masks of all frames where they take at most a gigabyte (else they are
+  // made for as many frames at a time as fit, once the offsets are known)
+  DevBuf mask(ctx);
+  int at_once = idx ? (int)std::min<int64_t>(nframes, std::max<int64_t>(1, ((int64_t)1 << 28) / words)) : 0;
+  while (at_once > 1 && mask.alloc(ctx, sizeof(unsigned) * (size_t)words * at_once) != MDS_OK) at_once /= 2;
+  if (at_once == 1) MDS_TRY(mask.alloc(ctx, sizeof(unsigned) * (size_t)words));
+  const bool all = at_once == nframes;
+  k_contact_mask<<<nframes, SP_THREADS, 0, s>>>(dx.as<float>(), natoms, dg1.as<int>(), n1, dg2.as<int>(), n2, eps,
+                                                words, all ? mask.as<unsigned>() : nullptr, dcnt.as<int64_t>());
   MDS_CUDA(ctx, cudaGetLastError());
   std::vector<int64_t> cnt(nframes);
   MDS_CUDA(ctx, cudaMemcpyAsync(cnt.data(), dcnt.p, sizeof(int64_t) * nframes, cudaMemcpyDeviceToHost, s));
@@ -557,9 +671,15 @@ extern "C" int mds_contact_profile(mds_ctx* ctx, const float* xyz, int nframes, 
   MDS_TRY(doff.alloc(ctx, sizeof(int64_t) * (nframes + 1)));
   MDS_TRY(didx.alloc(ctx, sizeof(int) * total));
   MDS_CUDA(ctx, cudaMemcpyAsync(doff.p, offsets, sizeof(int64_t) * (nframes + 1), cudaMemcpyHostToDevice, s));
-  k_contact<<<nframes, SP_THREADS, 0, s>>>(dx.as<float>(), natoms, dg1.as<int>(), n1, dg2.as<int>(), n2, eps, 1,
-                                           nullptr, doff.as<int64_t>(), didx.as<int>());
-  MDS_CUDA(ctx, cudaGetLastError());
+  for (int f0 = 0; f0 < nframes; f0 += at_once) {
+    const int nf = std::min(at_once, nframes - f0);
+    if (!all)
+      k_contact_mask<<<nf, SP_THREADS, 0, s>>>(dx.as<float>() + (size_t)f0 * 3 * natoms, natoms, dg1.as<int>(), n1,
+                                               dg2.as<int>(), n2, eps, words, mask.as<unsigned>(),
+                                               dcnt.as<int64_t>() + f0);
+    k_contact_list<<<nf, SP_THREADS, 0, s>>>(mask.as<unsigned>(), words, doff.as<int64_t>() + f0, didx.as<int>());
+    MDS_CUDA(ctx, cudaGetLastError());
+  }
   MDS_CUDA(ctx, cudaMemcpyAsync(idx, didx.p, sizeof(int) * total, cudaMemcpyDeviceToHost, s));
   MDS_CUDA(ctx, cudaStreamSynchronize(s));
   return MDS_OK;
