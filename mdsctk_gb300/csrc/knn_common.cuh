@@ -130,12 +130,12 @@ int build_template(mds_ctx* ctx, const float* dY0, int Ap, int natoms, bool nofi
 // Optional parts of the FP32 screen (k_screen_fp32, knn_rms.cu): tile
 // skipping with the tensor-core screen's row-tile pivots (pivlb [nR][nfit]
 // lower bounds of RMSD to the pivots, prad [2 nC] radii of the 80-frame
-// column tiles, rowlo [nR][nC]), shared row thresholds, thresholds from the
+// column tiles, tlo [nR][nC] bounds of the tiles' pairs), shared row thresholds, thresholds from the
 // (k+1)-th bound, outward column order, and the dense pivot pass.
 struct Fp32ScreenExtra {
   const float* pivlb = nullptr;
   const float* prad = nullptr;
-  const float* rowlo = nullptr;
+  const float* tlo = nullptr;
   int nR = 0, nC = 0, nfit = 0;
   float* rowthr = nullptr;
   const float* nmax = nullptr;
@@ -211,7 +211,7 @@ int vec_unsort(mds_ctx* ctx, const float* src, const int* perm, int n, float* ds
 struct TcSkip {
   const float* pivlb = nullptr;
   const float* prad = nullptr;
-  const float* rowlo = nullptr;  // [nrowtiles][ncoltiles] row-tile bounds, or null
+  const float* tlo = nullptr;    // [nrowtiles][ncoltiles] bounds of the tiles' pairs, or null
   int piv2 = 0;                  // pivots are the row tiles' (two per column tile)
   const int* far_perm = nullptr; // order of the non-diagonal items, or null
 };
@@ -235,11 +235,11 @@ int tc_skip_pivots(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Ar, const fl
 int tc_pivots_begin(mds_ctx* ctx, const KnnRmsPlan& pl, TcPivots& pv, bool rowpiv);
 int tc_pivots_operand(mds_ctx* ctx, const KnnRmsPlan& pl, TcPivots& pv);
 int tc_pivots_radii(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Ar, TcPivots& pv, int f0, int f1);
-int tc_skip_rowlo(mds_ctx* ctx, const TcPivots& pv, const float* lb, int n, float* rowlo);
+int tc_skip_tlo(mds_ctx* ctx, const TcPivots& pv, const float* lb, int n, float* tlo);
 // Order of the non-diagonal work items of a self screen with nseg segments,
 // estimated heaviest first (work: 3 * 1024 + row tiles * (nseg - 1) ints;
 // perm: row tiles * (nseg - 1) ints).
-int tc_far_order(mds_ctx* ctx, const TcPivots& pv, const float* lb, const float* rowlo, int n, int nseg,
+int tc_far_order(mds_ctx* ctx, const TcPivots& pv, const float* lb, const float* tlo, int n, int nseg,
                  int* work, int* perm);
 int tc_skip_bounds(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, const float* recf, int nfit,
                    const TcPivots& pv, float* lb, int* derr = nullptr, int f0 = 0, int f1 = 0);

@@ -383,7 +383,7 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
   // tensor-core screen's row-tile pivots (the middle frame of every 40-frame
   // tile) and 80-frame column tiles. RMSD is a metric, so for row i and any
   // frame j of 80-frame tile T, RMSD(i, j) >= max over the pivots p of T's
-  // two row tiles of lb(i, p) - r_T(p), and >= rowlo[R(i)][T]. A 64-frame
+  // two row tiles of lb(i, p) - r_T(p), and >= tlo[R(i)][T]. A 64-frame
   // tile of this screen overlaps one or two 80-frame tiles; the smaller of
   // their bounds holds for all its frames. The tile is skipped when every
   // row has that bound L > 0 with L^2 above its threshold.
@@ -478,7 +478,7 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
           float L = INF;
           for (int T = Ta; T <= Tb; ++T) {
             const int pa = 2 * T;
-            float LT = __ldg(ex.rowlo + (int64_t)R * ex.nC + T);
+            float LT = __ldg(ex.tlo + (int64_t)R * ex.nC + T);
             LT = fmaxf(LT, __ldg(ex.pivlb + (int64_t)pa * ex.nfit + g) - __ldg(ex.prad + pa));
             if (pa + 1 < ex.nR) LT = fmaxf(LT, __ldg(ex.pivlb + (int64_t)(pa + 1) * ex.nfit + g) - __ldg(ex.prad + pa + 1));
             L = fminf(L, LT);
@@ -1382,7 +1382,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   DevBuf ntiles(ctx);             // tiles the tensor-core screen computed
   unsigned long long ht = 0;      // (read back after the recheck)
   long long dense_pairs = 0;
-  DevBuf f_lb(ctx), f_rowlo(ctx);
+  DevBuf f_lb(ctx), f_tlo(ctx);
   TcPivots f_pv;
   if (pl.prec == MDS_PREC_FP32) {
     // shared row thresholds and the (k+1)-th rule; for a set screened
@@ -1414,11 +1414,11 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       pp.nref = f_pv.nP;
       MDS_TRY(launch_screen_fp32(ctx, pp, Afp, f_pv.A.as<float>(), Rfp, f_pv.R.as<float>(), nfit, nullptr, 32,
                                  choose_nseg_fp32(nfit, ctx->num_sms, f_pv.nP), nullptr, nullptr, &dx));
-      MDS_TRY(f_rowlo.alloc(ctx, sizeof(float) * (size_t)f_pv.nP * f_pv.nC));
-      MDS_TRY(tc_skip_rowlo(ctx, f_pv, f_lb.as<float>(), nfit, f_rowlo.as<float>()));
+      MDS_TRY(f_tlo.alloc(ctx, sizeof(float) * (size_t)f_pv.nP * f_pv.nC));
+      MDS_TRY(tc_skip_tlo(ctx, f_pv, f_lb.as<float>(), nfit, f_tlo.as<float>()));
       ex.pivlb = f_lb.as<float>();
       ex.prad = f_pv.rad.as<float>();
-      ex.rowlo = f_rowlo.as<float>();
+      ex.tlo = f_tlo.as<float>();
       ex.nR = f_pv.nP;
       ex.nC = f_pv.nC;
       ex.nfit = nfit;
@@ -1432,7 +1432,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     // (a set screened against itself uses row-tile pivots)
     TcSkip sk;
     TcPivots upv;
-    DevBuf ulb(ctx), rowlo(ctx), farw(ctx), farp(ctx);
+    DevBuf ulb(ctx), tlo(ctx), farw(ctx), farp(ctx);
     TcPivots& pv = staged ? spv : upv;  // (staged: pivots, radii and bounds made with the chunks)
     DevBuf& lb = staged ? slb : ulb;
     const bool skipping = !pl.screen_keys && !pl.noskip && (nref + 79) / 80 >= 4;
@@ -1445,15 +1445,15 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       sk.pivlb = lb.as<float>();
       sk.prad = pv.rad.as<float>();
       if (same) {
-        MDS_TRY(rowlo.alloc(ctx, sizeof(float) * (size_t)pv.nP * pv.nC));
-        MDS_TRY(tc_skip_rowlo(ctx, pv, lb.as<float>(), nfit, rowlo.as<float>()));
-        sk.rowlo = rowlo.as<float>();
+        MDS_TRY(tlo.alloc(ctx, sizeof(float) * (size_t)pv.nP * pv.nC));
+        MDS_TRY(tc_skip_tlo(ctx, pv, lb.as<float>(), nfit, tlo.as<float>()));
+        sk.tlo = tlo.as<float>();
         sk.piv2 = 1;
         if (nseg > 1) {
           const size_t nfar = (size_t)pv.nP * (nseg - 1);
           MDS_TRY(farw.alloc(ctx, sizeof(int) * (3 * 1024 + nfar)));
           MDS_TRY(farp.alloc(ctx, sizeof(int) * nfar));
-          MDS_TRY(tc_far_order(ctx, pv, lb.as<float>(), rowlo.as<float>(), nfit, nseg, farw.as<int>(),
+          MDS_TRY(tc_far_order(ctx, pv, lb.as<float>(), tlo.as<float>(), nfit, nseg, farw.as<int>(),
                                farp.as<int>()));
           sk.far_perm = farp.as<int>();
         }

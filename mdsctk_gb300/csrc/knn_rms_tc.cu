@@ -175,6 +175,7 @@ int tc_prepare(mds_ctx* ctx, const KnnRmsPlan& pl, const float* dev, int n, TcOp
 // ---------------------------------------------------------------------------
 #define TC_TQ 8  // depth of the task ring (producer -> MMA thread and epilogue warps)
 struct TcShared {
+  float colrec[TC_FR_N * MDS_REC];  // records of the current column tile (first: read 16 bytes at a time)
   uint64_t full[TC_STAGES], empty[TC_STAGES], tfull[2], tempty[2], done;
   uint64_t tq_full[TC_TQ], tq_empty[TC_TQ];
   int2 task[TC_TQ];  // (item, column tile); tile -1 ends an item, item -1 the stream
@@ -183,8 +184,7 @@ struct TcShared {
   int abortf;
   int cnt[TC_FR_M];
   float thr[TC_FR_M];
-  float colrec[TC_FR_N * MDS_REC];  // records of the current column tile
-  float rowrec[TC_FR_M * MDS_REC];  // records of the current row tile
+  float rowE[TC_FR_M];              // |a|^2 of the current row tile's frames
   float gthr[TC_FR_M];              // rows' global thresholds, refreshed per tile
 };
 
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const float* __restrict__ recf, const float* __restrict__ recr, int nfit, int Nr, int Ap,
             int nofit, float guard, float ginv, uint32_t idesc, int Kp, int nseg, int nitems, int rt0, int diag,
-            const float* __restrict__ pivlb, const float* __restrict__ prad, const float* __restrict__ rowlo,
+            const float* __restrict__ pivlb, const float* __restrict__ prad, const float* __restrict__ tlo,
             int piv2, const int* __restrict__ far_perm,
             float* __restrict__ dense, float* __restrict__ rowthr, const float* __restrict__ nmax, int k1,
             unsigned long long* __restrict__ ntiles,
@@ -271,8 +271,10 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // tile T holds row tiles 2T and 2T+1, and prad[2T], prad[2T+1] bound the
   // distances of its frames to their pivots, so L is the larger of the two
   // pivots' bounds. Row tile R also has RMSD(i, p_R) <= r_R for its frames i,
-  // so RMSD(i, j) >= RMSD(j, p_R) - r_R >= rowlo[R][T] = min over j in T of
-  // the lower bound of RMSD(j, p_R), minus r_R. L is the largest of these.
+  // so RMSD(i, j) >= RMSD(j, p_R) - r_R >= min over j in T of the lower bound
+  // of RMSD(j, p_R), minus r_R. L is the largest of these. tlo[R][T]: one bound
+  // for all pairs of the tile, the larger of that and of the columns' pivots'
+  // bounds at their smallest row (k_tile_lo).
   //
   // Row thresholds across segments (rowthr != null): each compaction lowers
   // rowthr[row] to its segment's K'-th bound (atomicMin). Every segment then
@@ -374,61 +376,83 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       rt += rt0;
       const int t0 = (int)((int64_t)ncoltiles * seg / nseg), t1 = (int)((int64_t)ncoltiles * (seg + 1) / nseg);
       const int td = diag ? min(max((rt * TC_FR_M + TC_FR_M / 2) / TC_FR_N, t0), t1 - 1) : t0;
-      uint32_t skipbits = 0;  // bit b: tile tbase + b of the current batch of 8 is skipped
-      int tbase = 0, test_at = 0;
       for (int ti = 0; ti < t1 - t0 && ok; ++ti) {
-        const int tile = tile_order(ti, t0, t1, td);
-        if (pivlb && ti == test_at) {
-          // skip test of the next 8 tiles at once (4 lanes per tile, 10 rows
-          // per lane: one round of loads instead of one per tile), against
-          // the rows' thresholds now, which only tighten later. While some
-          // row has no threshold yet (an item's first tiles), the test is
-          // repeated at every tile, so tiles are skipped as soon as the first
-          // thresholds arrive.
+        if (pivlb) {
+          // Skip test, again after every tile handed out (thresholds only
+          // tighten; it runs under that tile's MMAs). Coarse first: 32 tiles
+          // at once, one lane each, the tile's bound tlo against the largest
+          // threshold of the rows. Then up to 8 of the tiles left at once, 4
+          // lanes each and 10 rows per lane, every row against its own
+          // threshold. (The row test alone, for every tile, kept the MMA
+          // thread waiting 34,000 of 55,000 cycles per computed tile at
+          // 100,000 x 304, where 34 tiles are tested for one computed.)
           // Before the epilogue has loaded this item's list thresholds
           // (S->thr still holds the previous item's rows), the shared row
           // thresholds alone are used: each is itself a valid threshold.
-          skipbits = 0;
-          tbase = ti;
-          test_at = ti + 1;
+          const int window = min(32, t1 - t0 - ti);
           int live = (lane == 0) ? (*(volatile int*)&S->thr_item == item) : 0;
           live = __shfl_sync(0xffffffffu, live, 0);
+          unsigned left = window == 32 ? 0xffffffffu : (1u << window) - 1u;  // tiles of the window not skipped
+          unsigned skip = 0;
           if (live || rowthr) {
             __threadfence_block();
-            const int tj = ti + (lane >> 2), r0 = (lane & 3) * 10;
-            bool can = tj < t1 - t0, open = false;
-            if (can) {
-              const int tb = tile_order(tj, t0, t1, td);
-              const int pa = piv2 ? 2 * tb : tb;
-              const bool pb = piv2 && 2 * tb + 1 < (nfit + TC_FR_M - 1) / TC_FR_M;
-              const float rada = __ldg(prad + pa), radb = pb ? __ldg(prad + pa + 1) : 0.0f;
-              const float Lrow = rowlo ? __ldg(rowlo + (int64_t)rt * ncoltiles + tb) : 0.0f;
+            auto row_thr = [&](int r) {
+              float thr = live ? *(volatile float*)&S->thr[r] : INFINITY;
+              if (rowthr) thr = fminf(thr, __ldcg(rowthr + rt * TC_FR_M + r));
+              return thr;
+            };
+            float mx = 0.0f;
+            for (int r = lane; r < TC_FR_M; r += 32)
+              if (rt * TC_FR_M + r < nfit) mx = fmaxf(mx, row_thr(r));
+            mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+            if (mx < 1e30f) {
+              if (tlo) {
+                float L = 0.0f;
+                if (lane < window) L = __ldg(tlo + (int64_t)rt * ncoltiles + tile_order(ti + lane, t0, t1, td));
+                skip = __ballot_sync(0xffffffffu, lane < window && L > 0.0f && L * L > mx);
+              }
+              const unsigned rest = left & ~skip;
+              const int nth = __popc(rest) > (lane >> 2) ? (int)__fns(rest, 0, (lane >> 2) + 1) : -1;
+              const int r0 = (lane & 3) * 10;
+              bool can = nth >= 0;
+              if (can) {
+                const int tb = tile_order(ti + nth, t0, t1, td);
+                const int pa = piv2 ? 2 * tb : tb;
+                const bool pb = piv2 && 2 * tb + 1 < (nfit + TC_FR_M - 1) / TC_FR_M;
+                const float rada = __ldg(prad + pa), radb = pb ? __ldg(prad + pa + 1) : 0.0f;
+                const float Lt = tlo ? __ldg(tlo + (int64_t)rt * ncoltiles + tb) : 0.0f;
 #pragma unroll
-              for (int x = 0; x < 10; ++x) {
-                const int gi = rt * TC_FR_M + r0 + x;
-                if (gi < nfit) {
-                  float thr = live ? *(volatile float*)&S->thr[r0 + x] : INFINITY;
-                  if (rowthr) thr = fminf(thr, __ldcg(rowthr + gi));
-                  open |= !(thr < 1e30f);
-                  float L = fmaxf(__ldg(pivlb + (int64_t)pa * nfit + gi) - rada, Lrow);
-                  if (pb) L = fmaxf(L, __ldg(pivlb + (int64_t)(pa + 1) * nfit + gi) - radb);
-                  if (!(L > 0.0f && L * L > thr)) can = false;
+                for (int x = 0; x < 10; ++x) {
+                  const int gi = rt * TC_FR_M + r0 + x;
+                  if (gi < nfit) {
+                    const float thr = row_thr(r0 + x);
+                    float L = fmaxf(__ldg(pivlb + (int64_t)pa * nfit + gi) - rada, Lt);
+                    if (pb) L = fmaxf(L, __ldg(pivlb + (int64_t)(pa + 1) * nfit + gi) - radb);
+                    if (!(L > 0.0f && L * L > thr)) can = false;
+                  }
                 }
               }
+              const unsigned bal = __ballot_sync(0xffffffffu, can);
+              for (int g = 0; g < 8; ++g) {
+                const int n = __shfl_sync(0xffffffffu, nth, 4 * g);
+                if (n >= 0 && ((bal >> (4 * g)) & 0xFu) == 0xFu) skip |= 1u << n;
+              }
             }
-            const unsigned bal = __ballot_sync(0xffffffffu, can);
-            if (!__any_sync(0xffffffffu, open)) test_at = ti + 8;
             int still = 1;
             if (live) {  // the list thresholds read belong to this item: not moved on meanwhile
               still = (lane == 0) ? (*(volatile int*)&S->thr_item == item) : 0;
               still = __shfl_sync(0xffffffffu, still, 0);
             }
-            if (still)
-              for (int b = 0; b < 8; ++b)
-                if (((bal >> (4 * b)) & 0xFu) == 0xFu) skipbits |= 1u << b;
+            if (!still) skip = 0;
           }
+          left &= ~skip;
+          if (!left) {
+            ti += window - 1;
+            continue;
+          }
+          ti += __ffs(left) - 1;
         }
-        if ((skipbits >> (ti - tbase)) & 1u) continue;
+        const int tile = tile_order(ti, t0, t1, td);
         if (!(ok = push(item, tile))) break;
         if (lane == 0) {
           for (int kb = 0; kb < nkb; ++kb) {
@@ -509,13 +533,14 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ------------------------------------------------------------ epilogue
     const int ew = warp - 2;
     const int q = warp & 3;          // TMEM lane quarter of this warp
-    const int h = ew >> 2;           // column quarter: chunks [ci0, ci1) of the 10
-    const int ci0 = (h * 10) / 4, ci1 = ((h + 1) * 10) / 4;
+    const int h = ew >> 2;           // column quarter
     const int f = lane / 3, c = lane % 3;
     const int rloc = q * 10 + f;     // row within the 40-frame tile (f < 10)
     uint64_t* scratch = scratch_all + ew * TC_SCR;
     const float INF = __int_as_float(0x7f800000);
-    const float* rrec = S->rowrec + min(rloc, TC_FR_M - 1) * MDS_REC;  // lanes 30, 31 (f = 10) are padding
+    // this lane's row record, in registers for the item (ten rows' records in
+    // shared memory are 16 words apart: five-way bank conflicts per read)
+    float rrec[MDS_REC];
     uint32_t acc = 0;
     bool ok = true;
     int cur = -1, rt = 0, seg = 0, grow = 0, ntile = 0;
@@ -545,9 +570,19 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         grow = rt * TC_FR_M + rloc;
         rowok = (f < 10) && grow < nfit;
         ntile = 0;
-        for (int e = ew * 32 + lane; e < TC_FR_M * MDS_REC; e += TC_EPI_WARPS * 32) {
-          const int r = rt * TC_FR_M + e / MDS_REC;
-          S->rowrec[e] = (r < nfit) ? __ldg(recf + (int64_t)r * MDS_REC + e % MDS_REC) : 0.f;
+        if (ew == 0)
+          for (int r = lane; r < TC_FR_M; r += 32) {
+            const int gi = rt * TC_FR_M + r;
+            S->rowE[r] = (gi < nfit) ? __ldg(recf + (int64_t)gi * MDS_REC + 15) : 0.f;
+          }
+        {
+          const float4* rp = reinterpret_cast<const float4*>(recf + (int64_t)min(grow, nfit - 1) * MDS_REC);
+#pragma unroll
+          for (int v4 = 0; v4 < 4; ++v4) {
+            if (v4 == 2) continue;  // (entries 8..11 are the column side's)
+            const float4 t = __ldg(rp + v4);
+            rrec[4 * v4] = t.x; rrec[4 * v4 + 1] = t.y; rrec[4 * v4 + 2] = t.z; rrec[4 * v4 + 3] = t.w;
+          }
         }
         if (lane < 3 && h + 4 * lane < 10) {
           const int fr = h + 4 * lane;
@@ -625,68 +660,90 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       }
       const uint32_t tq = tbase + ((uint32_t)(q * 32) << 16) + b * 256;
       uint64_t* rowbuf = dense ? nullptr : candbuf + ((int64_t)grow * nseg + seg) * TC_CAPG;
-#pragma unroll 1
-      for (int ci = ci0; ci < ci1; ++ci) {
-        float vx[8], vy[8], vz[8];
-        tmem_ld8(tq + 8 * ci, vx);
-        tmem_ld8(tq + TC_FR_N + 8 * ci, vy);
-        tmem_ld8(tq + 2 * TC_FR_N + 8 * ci, vz);
-        tmem_wait_ld();
+      // three columns [c0 + g0, + 3) of the loaded ones: x, y, z of 3 column
+      // frames per lane row; ncol: columns that are the warp's own
+      auto pairs3 = [&](const float* vx, const float* vy, const float* vz, int g0, int ncol, int c0) {
+        // v[g][d]: row (f, c) of the Gram of pair (f, column frame g0+g)
+        float v[3][3];
 #pragma unroll
-        for (int g0 = 0; g0 < 8; g0 += 3) {
-          // v[g][d]: row (f, c) of the Gram of pair (f, column frame g0+g)
-          float v[3][3];
+        for (int g = 0; g < 3; ++g) {
+          const bool in = g0 + g < ncol;
+          v[g][0] = in ? vx[in ? g0 + g : 0] : 0.f;
+          v[g][1] = in ? vy[in ? g0 + g : 0] : 0.f;
+          v[g][2] = in ? vz[in ? g0 + g : 0] : 0.f;
+        }
+        // 3-lane transpose: lane (f, m=c) gathers rows 0..2 of block m
+        float R[3][3];
 #pragma unroll
-          for (int g = 0; g < 3; ++g) {
-            v[g][0] = (g0 + g < 8) ? vx[(g0 + g) & 7] : 0.f;
-            v[g][1] = (g0 + g < 8) ? vy[(g0 + g) & 7] : 0.f;
-            v[g][2] = (g0 + g < 8) ? vz[(g0 + g) & 7] : 0.f;
-          }
-          // 3-lane transpose: lane (f, m=c) gathers rows 0..2 of block m
-          float R[3][3];
+        for (int d = 0; d < 3; ++d) R[0][d] = sel3(c, v[0][d], v[1][d], v[2][d]);
 #pragma unroll
-          for (int d = 0; d < 3; ++d) R[0][d] = sel3(c, v[0][d], v[1][d], v[2][d]);
-#pragma unroll
-          for (int s = 1; s < 3; ++s) {
-            const int src = 3 * f + (c + s) % 3;
-            const int gi = (c + 3 - s) % 3;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              float send = sel3(gi, v[0][d], v[1][d], v[2][d]);
-              R[s][d] = __shfl_sync(0xffffffffu, send, src & 31);
-            }
-          }
-          // row (c + s) % 3 of block m is R[s]
-          float G[9];
+        for (int s = 1; s < 3; ++s) {
+          const int src = 3 * f + (c + s) % 3;
+          const int gi = (c + 3 - s) % 3;
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
-            G[0 + d] = sel3(c, R[0][d], R[2][d], R[1][d]) * ginv;
-            G[3 + d] = sel3(c, R[1][d], R[0][d], R[2][d]) * ginv;
-            G[6 + d] = sel3(c, R[2][d], R[1][d], R[0][d]) * ginv;
+            float send = sel3(gi, v[0][d], v[1][d], v[2][d]);
+            R[s][d] = __shfl_sync(0xffffffffu, send, src & 31);
           }
-          const int gl = 8 * ci + g0 + c;
-          const int j = tile * TC_FR_N + gl;
-          if (rowok && (g0 + c < 8) && j < Nr) {
-            const float* cr = S->colrec + gl * MDS_REC;
-            if (dense) {
-              // (pivot bounds: no refinement, a loose bound only weakens a skip)
-              const float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]),
-                                                  __builtin_huge_valf(), false);
-              dense[(int64_t)j * nfit + grow] = sqrtf(fmaxf(sv, 0.0f));
-            } else {
-              const float thr = fminf(*(volatile float*)&S->thr[rloc], S->gthr[rloc]);
-              float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]), thr);
-              sv = fmaxf(sv, 0.0f);
-              if (sv < thr) {
-                int pos = atomicAdd(&S->cnt[rloc], 1);
-                if (pos < TC_CAPG)
-                  rowbuf[pos] = mds_pack_key(sv, j);
-                else
-                  atomicMax(err, 4);  // cannot happen with K' + 160 <= capacity
-              }
+        }
+        // row (c + s) % 3 of block m is R[s]
+        float G[9];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          G[0 + d] = sel3(c, R[0][d], R[2][d], R[1][d]) * ginv;
+          G[3 + d] = sel3(c, R[1][d], R[0][d], R[2][d]) * ginv;
+          G[6 + d] = sel3(c, R[2][d], R[1][d], R[0][d]) * ginv;
+        }
+        const int gl = c0 + g0 + c;
+        const int j = tile * TC_FR_N + gl;
+        if (rowok && (g0 + c < ncol) && j < Nr) {
+          float cr[MDS_REC];
+          const float4* cp = reinterpret_cast<const float4*>(S->colrec + gl * MDS_REC);
+#pragma unroll
+          for (int v4 = 1; v4 < 4; ++v4) {
+            const float4 t = cp[v4];
+            cr[4 * v4] = t.x; cr[4 * v4 + 1] = t.y; cr[4 * v4 + 2] = t.z; cr[4 * v4 + 3] = t.w;
+          }
+          if (dense) {
+            // (pivot bounds: no refinement, a loose bound only weakens a skip)
+            const float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]),
+                                                __builtin_huge_valf(), false);
+            dense[(int64_t)j * nfit + grow] = sqrtf(fmaxf(sv, 0.0f));
+          } else {
+            const float thr = fminf(*(volatile float*)&S->thr[rloc], S->gthr[rloc]);
+            float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]), thr);
+            sv = fmaxf(sv, 0.0f);
+            if (sv < thr) {
+              int pos = atomicAdd(&S->cnt[rloc], 1);
+              if (pos < TC_CAPG)
+                rowbuf[pos] = mds_pack_key(sv, j);
+              else
+                atomicMax(err, 4);  // cannot happen with K' + 160 <= capacity
             }
           }
         }
+      };
+      // the warp's 20 columns, twelve and then eight at a time: seven groups of
+      // three (in chunks of 8 columns, two or three a warp, the slowest warps
+      // had nine)
+      {
+        const int c0 = h * (TC_FR_N / 4);
+        float vx[12], vy[12], vz[12];
+        tmem_ld8(tq + c0, vx);
+        tmem_ld4(tq + c0 + 8, vx + 8);
+        tmem_ld8(tq + TC_FR_N + c0, vy);
+        tmem_ld4(tq + TC_FR_N + c0 + 8, vy + 8);
+        tmem_ld8(tq + 2 * TC_FR_N + c0, vz);
+        tmem_ld4(tq + 2 * TC_FR_N + c0 + 8, vz + 8);
+        tmem_wait_ld();
+#pragma unroll
+        for (int g0 = 0; g0 < 12; g0 += 3) pairs3(vx, vy, vz, g0, 12, c0);
+        tmem_ld8(tq + c0 + 12, vx);
+        tmem_ld8(tq + TC_FR_N + c0 + 12, vy);
+        tmem_ld8(tq + 2 * TC_FR_N + c0 + 12, vz);
+        tmem_wait_ld();
+#pragma unroll
+        for (int g0 = 0; g0 < 8; g0 += 3) pairs3(vx, vy, vz, g0, 8, c0 + 12);
       }
       tc_fence_before();
       __syncwarp();
@@ -714,7 +771,7 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         float tk1 = INF;
         float t = warp_select_keep2(src, n, TC_CAPG, 0, need ? Kp : 0, reinterpret_cast<int*>(scratch), lane,
                                     nmax ? k1 : 0, &tk1);
-        if (nmax) t = fminf(t, tk1 + 2.0f * guard * (S->rowrec[r * MDS_REC + 15] + __ldg(nmax)));
+        if (nmax) t = fminf(t, tk1 + 2.0f * guard * (S->rowE[r] + __ldg(nmax)));
         if (lane == 0) {
           if (need) S->cnt[r] = Kp;
           S->thr[r] = t;
@@ -828,7 +885,7 @@ int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, 
   k_screen_tc<<<grid, TC_THREADS, smem, ctx->stream>>>(mA, mB, recf, recr, nfit, pl.nref, pl.Ap, pl.nofit,
                                                        pl.guard_tc, 1.0f / (s * s), idesc, Kp, nseg, nitems, rt0,
                                                        &fit == &ref ? 1 : 0, skip ? skip->pivlb : nullptr,
-                                                       skip ? skip->prad : nullptr, skip ? skip->rowlo : nullptr,
+                                                       skip ? skip->prad : nullptr, skip ? skip->tlo : nullptr,
                                                        skip ? skip->piv2 : 0, skip ? skip->far_perm : nullptr,
                                                        dense, rowthr, nmax, pl.k + 1, ntiles, cand, cand_n, e,
                                                        stall);
@@ -924,18 +981,46 @@ __global__ void k_tile_radius_rc(const float* __restrict__ A, int N, int Ap, con
   }
 }
 
-// rowlo[R][T] = min over the frames j of column tile T of lb(j, row pivot R)
-// (row R of the dense pass) minus the row tile's radius: one warp per (R, T).
-__global__ void k_row_lo(const float* __restrict__ lb, int N, int nC, int nR, const float* __restrict__ rrad,
-                         float* __restrict__ rowlo) {
-  const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= nR * nC) return;
-  const int R = w / nC, T = w % nC;
-  const float* row = lb + (int64_t)R * N;
+// hmin[p][r] = min over the frames i of row tile r of lb[p][i], the bounds of
+// RMSD(i, pivot p). A block takes TL_TILES row tiles of one pivot: their bounds
+// read in one piece, the minima by warp 0. Memory-bound: nP x N floats once (1
+// GB at 100,000 frames; a warp per 80 frames, lanes partly idle, took 600 us,
+// this 215.)
+#define TL_TILES 32
+__global__ void __launch_bounds__(256) k_half_min(const float* __restrict__ lb, int N, int nR,
+                                                  float* __restrict__ hmin) {
+  __shared__ float v[TL_TILES * (TC_FR_M + 1)];
+  const int p = blockIdx.y, r0 = blockIdx.x * TL_TILES;
+  const int f0 = r0 * TC_FR_M, n = min(TL_TILES * TC_FR_M, N - f0);
+  const float* src = lb + (int64_t)p * N + f0;
+#pragma unroll
+  for (int i = 0; i < TL_TILES * TC_FR_M / 256; ++i) {
+    const int e = threadIdx.x + 256 * i;
+    if (e < n) v[e / TC_FR_M * (TC_FR_M + 1) + e % TC_FR_M] = __ldg(src + e);
+  }
+  __syncthreads();
+  const int r = r0 + threadIdx.x;
+  if (threadIdx.x >= TL_TILES || r >= nR) return;
   float m = INFINITY;
-  for (int j = T * TC_FR_N + lane; j < min(N, (T + 1) * TC_FR_N); j += 32) m = fminf(m, __ldg(row + j));
-  for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) rowlo[w] = m - __ldg(rrad + R);
+  for (int x = 0; x < min(TC_FR_M, N - r * TC_FR_M); ++x) m = fminf(m, v[threadIdx.x * (TC_FR_M + 1) + x]);
+  hmin[(int64_t)p * nR + r] = m;
+}
+
+// tlo[R][T], a lower bound of RMSD of every pair of row tile R and column tile
+// T (row tiles 2T, 2T+1), by the triangle inequality: through R's pivot, min
+// over T's frames of their bounds to it minus R's radius; through T's two
+// pivots, min over R's frames of their bounds to each minus T's radius around
+// it; the largest of the three.
+__global__ void k_tile_lo(const float* __restrict__ hmin, int nR, int nC, const float* __restrict__ rrad,
+                          const float* __restrict__ prad, float* __restrict__ tlo) {
+  const int T = blockIdx.x * 32 + (threadIdx.x & 31), R = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (T >= nC || R >= nR) return;
+  const int a = 2 * T, b = min(2 * T + 1, nR - 1);
+  const float* hr = hmin + (int64_t)R * nR;
+  float L = fminf(__ldg(hr + a), __ldg(hr + b)) - __ldg(rrad + R);
+  L = fmaxf(L, __ldg(hmin + (int64_t)a * nR + R) - __ldg(prad + a));
+  if (b > a) L = fmaxf(L, __ldg(hmin + (int64_t)b * nR + R) - __ldg(prad + b));
+  tlo[(int64_t)R * nC + T] = L;
 }
 
 // *out = max over frames of rec[15] = |a|^2 (out zeroed beforehand;
@@ -1049,17 +1134,15 @@ int tc_skip_bounds(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, co
                           nullptr, lb, nullptr, nullptr, nullptr, rt0, nrt);
 }
 
-// The row-tile bounds of a set screened against itself (pivots with rowpiv,
-// lb [nR][n] from tc_skip_bounds): rowlo [nR][nC].
 // Order of the non-diagonal items (row tile R, other segment s'), heaviest
 // estimate first. Estimate: with t_R = twice the smallest bound from pivot R
 // to another pivot (a scale of R's neighbour distances), the number of
-// column tiles T of the segment with rowlo[R][T] < t_R. est[k] and a
+// column tiles T of the segment with tlo[R][T] < t_R. est[k] and a
 // histogram first (one warp per row tile), then a descending exclusive scan
 // of the histogram, then a scatter (order within one estimate unspecified:
 // the results do not depend on the order of the items).
 #define TC_EST_BUCKETS 1024
-__global__ void k_far_est(const float* __restrict__ lb, const float* __restrict__ rowlo, int N, int nR, int nC,
+__global__ void k_far_est(const float* __restrict__ lb, const float* __restrict__ tlo, int N, int nR, int nC,
                           int nseg, int* __restrict__ est, int* __restrict__ hist) {
   const int R = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (R >= nR) return;
@@ -1074,7 +1157,7 @@ __global__ void k_far_est(const float* __restrict__ lb, const float* __restrict_
     const int seg = sp < sd ? sp : sp + 1;
     const int t0 = (int)((int64_t)nC * seg / nseg), t1 = (int)((int64_t)nC * (seg + 1) / nseg);
     int c = 0;
-    for (int T = t0 + lane; T < t1; T += 32) c += (__ldg(rowlo + (int64_t)R * nC + T) < t) ? 1 : 0;
+    for (int T = t0 + lane; T < t1; T += 32) c += (__ldg(tlo + (int64_t)R * nC + T) < t) ? 1 : 0;
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     c = min(c, TC_EST_BUCKETS - 1);
     if (lane == 0) {
@@ -1108,7 +1191,7 @@ __global__ void k_far_scatter(const int* __restrict__ est, int nfar, const int* 
   perm[off[e] + atomicAdd(cnt + e, 1)] = k;
 }
 
-int tc_far_order(mds_ctx* ctx, const TcPivots& pv, const float* lb, const float* rowlo, int n, int nseg,
+int tc_far_order(mds_ctx* ctx, const TcPivots& pv, const float* lb, const float* tlo, int n, int nseg,
                  int* work, int* perm) {
   // work: 3 * TC_EST_BUCKETS + nR * (nseg - 1) ints
   if (!pv.rowpiv || nseg < 2) return mds_fail(ctx, MDS_ERR_INTERNAL, "far order needs row pivots and segments");
@@ -1120,19 +1203,23 @@ int tc_far_order(mds_ctx* ctx, const TcPivots& pv, const float* lb, const float*
   cudaStream_t s = ctx->stream;
   MDS_CUDA(ctx, cudaMemsetAsync(work, 0, sizeof(int) * 3 * TC_EST_BUCKETS, s));
   ctx->stats.launches += 3;
-  k_far_est<<<(nR + 7) / 8, 256, 0, s>>>(lb, rowlo, n, nR, pv.nC, nseg, est, hist);
+  k_far_est<<<(nR + 7) / 8, 256, 0, s>>>(lb, tlo, n, nR, pv.nC, nseg, est, hist);
   k_far_scan<<<1, TC_EST_BUCKETS, 0, s>>>(hist, off);
   k_far_scatter<<<(nfar + 255) / 256, 256, 0, s>>>(est, nfar, off, cnt, perm);
   MDS_CUDA(ctx, cudaGetLastError());
   return MDS_OK;
 }
 
-int tc_skip_rowlo(mds_ctx* ctx, const TcPivots& pv, const float* lb, int n, float* rowlo) {
+int tc_skip_tlo(mds_ctx* ctx, const TcPivots& pv, const float* lb, int n, float* tlo) {
   if (!pv.rowpiv) return mds_fail(ctx, MDS_ERR_INTERNAL, "row-tile pivots were not built");
-  const int nR = pv.nP;
-  const int warps = nR * pv.nC;
-  ctx->stats.launches++;
-  k_row_lo<<<(warps + 7) / 8, 256, 0, ctx->stream>>>(lb, n, pv.nC, nR, pv.rrad.as<float>(), rowlo);
+  const int nR = pv.nP, nC = pv.nC;
+  if (nR > 65535) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "%d row tiles", nR);
+  DevBuf hmin(ctx);
+  MDS_TRY(hmin.alloc(ctx, sizeof(float) * (size_t)nR * nR));
+  ctx->stats.launches += 2;
+  k_half_min<<<dim3((nR + TL_TILES - 1) / TL_TILES, nR), 256, 0, ctx->stream>>>(lb, n, nR, hmin.as<float>());
+  k_tile_lo<<<dim3((nC + 31) / 32, (nR + 7) / 8), 256, 0, ctx->stream>>>(hmin.as<float>(), nR, nC,
+                                                                       pv.rrad.as<float>(), pv.rad.as<float>(), tlo);
   MDS_CUDA(ctx, cudaGetLastError());
   return MDS_OK;
 }
