@@ -211,6 +211,7 @@ int vec_unsort(mds_ctx* ctx, const float* src, const int* perm, int n, float* ds
 struct TcSkip {
   const float* pivlb = nullptr;
   const float* prad = nullptr;
+  const float* rrad = nullptr;   // the row tiles' own radii (piv2)
   const float* tlo = nullptr;    // [nrowtiles][ncoltiles] bounds of the tiles' pairs, or null
   int piv2 = 0;                  // pivots are the row tiles' (two per column tile)
   const int* far_perm = nullptr; // order of the non-diagonal items, or null

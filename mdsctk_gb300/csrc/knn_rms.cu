@@ -1449,6 +1449,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
         MDS_TRY(tc_skip_tlo(ctx, pv, lb.as<float>(), nfit, tlo.as<float>()));
         sk.tlo = tlo.as<float>();
         sk.piv2 = 1;
+        sk.rrad = pv.rrad.as<float>();
         if (nseg > 1) {
           const size_t nfar = (size_t)pv.nP * (nseg - 1);
           MDS_TRY(farw.alloc(ctx, sizeof(int) * (3 * 1024 + nfar)));

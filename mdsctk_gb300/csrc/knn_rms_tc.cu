@@ -248,8 +248,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const float* __restrict__ recf, const float* __restrict__ recr, int nfit, int Nr, int Ap,
             int nofit, float guard, float ginv, uint32_t idesc, int Kp, int nseg, int nitems, int rt0, int diag,
-            const float* __restrict__ pivlb, const float* __restrict__ prad, const float* __restrict__ tlo,
-            int piv2, const int* __restrict__ far_perm,
+            const float* __restrict__ pivlb, const float* __restrict__ prad, const float* __restrict__ rrad,
+            const float* __restrict__ tlo, int piv2, const int* __restrict__ far_perm,
             float* __restrict__ dense, float* __restrict__ rowthr, const float* __restrict__ nmax, int k1,
             unsigned long long* __restrict__ ntiles,
             uint64_t* __restrict__ candbuf, int* __restrict__ cand_n, int* __restrict__ err, int stall) {
@@ -274,7 +274,12 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // so RMSD(i, j) >= RMSD(j, p_R) - r_R >= min over j in T of the lower bound
   // of RMSD(j, p_R), minus r_R. L is the largest of these. tlo[R][T]: one bound
   // for all pairs of the tile, the larger of that and of the columns' pivots'
-  // bounds at their smallest row (k_tile_lo).
+  // bounds at their smallest row (k_tile_lo). L is also at least the smaller
+  // of the two halves' own bounds, pivlb[2T][i] - rrad[2T] for the frames of
+  // row tile 2T and likewise 2T+1: a half's radius is smaller than its
+  // distance to the other half's pivot. (Row tiles across two basins, whose
+  // own radius is useless, were computed against every tile of both basins
+  // without it: 90,000 tiles at 100,000 x 304, with it 51,000.)
   //
   // Row thresholds across segments (rowthr != null): each compaction lowers
   // rowthr[row] to its segment's K'-th bound (atomicMin). Every segment then
@@ -420,14 +425,17 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const int pa = piv2 ? 2 * tb : tb;
                 const bool pb = piv2 && 2 * tb + 1 < (nfit + TC_FR_M - 1) / TC_FR_M;
                 const float rada = __ldg(prad + pa), radb = pb ? __ldg(prad + pa + 1) : 0.0f;
+                const float ra = piv2 ? __ldg(rrad + pa) : rada, rb = pb ? __ldg(rrad + pa + 1) : 0.0f;
                 const float Lt = tlo ? __ldg(tlo + (int64_t)rt * ncoltiles + tb) : 0.0f;
 #pragma unroll
                 for (int x = 0; x < 10; ++x) {
                   const int gi = rt * TC_FR_M + r0 + x;
                   if (gi < nfit) {
                     const float thr = row_thr(r0 + x);
-                    float L = fmaxf(__ldg(pivlb + (int64_t)pa * nfit + gi) - rada, Lt);
-                    if (pb) L = fmaxf(L, __ldg(pivlb + (int64_t)(pa + 1) * nfit + gi) - radb);
+                    const float la = __ldg(pivlb + (int64_t)pa * nfit + gi);
+                    const float lb = pb ? __ldg(pivlb + (int64_t)(pa + 1) * nfit + gi) : 0.0f;
+                    float L = fmaxf(la - rada, Lt);
+                    if (pb) L = fmaxf(L, fmaxf(lb - radb, fminf(la - ra, lb - rb)));
                     if (!(L > 0.0f && L * L > thr)) can = false;
                   }
                 }
@@ -885,7 +893,8 @@ int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, 
   k_screen_tc<<<grid, TC_THREADS, smem, ctx->stream>>>(mA, mB, recf, recr, nfit, pl.nref, pl.Ap, pl.nofit,
                                                        pl.guard_tc, 1.0f / (s * s), idesc, Kp, nseg, nitems, rt0,
                                                        &fit == &ref ? 1 : 0, skip ? skip->pivlb : nullptr,
-                                                       skip ? skip->prad : nullptr, skip ? skip->tlo : nullptr,
+                                                       skip ? skip->prad : nullptr, skip ? skip->rrad : nullptr,
+                                                       skip ? skip->tlo : nullptr,
                                                        skip ? skip->piv2 : 0, skip ? skip->far_perm : nullptr,
                                                        dense, rowthr, nmax, pl.k + 1, ntiles, cand, cand_n, e,
                                                        stall);
@@ -1010,7 +1019,8 @@ __global__ void __launch_bounds__(256) k_half_min(const float* __restrict__ lb, 
 // T (row tiles 2T, 2T+1), by the triangle inequality: through R's pivot, min
 // over T's frames of their bounds to it minus R's radius; through T's two
 // pivots, min over R's frames of their bounds to each minus T's radius around
-// it; the largest of the three.
+// it, or the smaller of the two halves' with each half's own radius; the
+// largest of these.
 __global__ void k_tile_lo(const float* __restrict__ hmin, int nR, int nC, const float* __restrict__ rrad,
                           const float* __restrict__ prad, float* __restrict__ tlo) {
   const int T = blockIdx.x * 32 + (threadIdx.x & 31), R = blockIdx.y * 8 + (threadIdx.x >> 5);
@@ -1018,8 +1028,10 @@ __global__ void k_tile_lo(const float* __restrict__ hmin, int nR, int nC, const 
   const int a = 2 * T, b = min(2 * T + 1, nR - 1);
   const float* hr = hmin + (int64_t)R * nR;
   float L = fminf(__ldg(hr + a), __ldg(hr + b)) - __ldg(rrad + R);
-  L = fmaxf(L, __ldg(hmin + (int64_t)a * nR + R) - __ldg(prad + a));
-  if (b > a) L = fmaxf(L, __ldg(hmin + (int64_t)b * nR + R) - __ldg(prad + b));
+  const float ha = __ldg(hmin + (int64_t)a * nR + R), hb = __ldg(hmin + (int64_t)b * nR + R);
+  L = fmaxf(L, ha - __ldg(prad + a));
+  if (b > a) L = fmaxf(L, hb - __ldg(prad + b));
+  L = fmaxf(L, fminf(ha - __ldg(rrad + a), hb - __ldg(rrad + b)));
   tlo[(int64_t)R * nC + T] = L;
 }
 
