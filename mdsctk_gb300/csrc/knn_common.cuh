@@ -114,8 +114,9 @@ int launch_center(mds_ctx* ctx, const float* draw, int n, int natoms, int Ap, co
                   const float* dswn, float tm, float* Y, double* E);
 // Centring + superposition of n raw frames (three kernels, no scratch
 // buffer): deviations and records only (knn_rms.cu).
-// Uhl (optional): the frames' U = sum a mu^T as double-float pairs [n][18],
-// which the recheck needs for the reference frames.
+// Uhl (optional): the frames' U = sum a mu^T as double-float pairs
+// [n][MDS_USTRIDE] (18 used), which the recheck needs for the reference frames.
+#define MDS_USTRIDE 20  // (rows of whole 16-byte pieces)
 int launch_prep(mds_ctx* ctx, const float* draw, int n, int natoms, int Ap, const float* dmass, const float* dswn,
                 float tm, const float* dmu, const double* dM0, int nofit, float* A, float* R, float* Uhl = nullptr,
                 int* bad = nullptr, int fbase = 0);
@@ -161,11 +162,20 @@ struct RecheckAudit {
   float guard = 0.f;
   unsigned long long* counters = nullptr;
 };
+// Scratch of the staged recheck of up to `nrows` rows (panel 0: none, the
+// block kernel takes every row). It has to outlive the launches, and their
+// replays when they were captured.
+struct RecheckScratch {
+  DevBuf rc, meta, cidx, cbound, sums, big, nbig;
+  int panel = 0;  // rows at a time
+};
+int recheck_scratch(mds_ctx* ctx, int nrows, RecheckScratch& rs);
+size_t recheck_scratch_bytes(int nrows);
 int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const float* Ar, const float* mu,
                    const float* Ur, int nrows, const int* rowlist, int mode, const uint64_t* cand,
                    const int* cand_n, int nseg, int segstride, int Kp, int k, double* out_d, int* out_i,
                    int* flagged, int* nflag, const float* rowthr = nullptr, const RecheckAudit* audit = nullptr,
-                   int cand_by_row = 0);
+                   int cand_by_row = 0, RecheckScratch* rs = nullptr);
 
 int choose_nseg_fp32(int nfit, int num_sms, int nref);
 
@@ -185,6 +195,9 @@ int tc_choose_nseg(mds_ctx* ctx, const KnnRmsPlan& pl, int nfit);
 // 2-D tensor map of a split hi|lo operand: rows x (2 * half) 16-bit values,
 // boxes of 32 x boxrows, 64-byte swizzle (knn_rms_tc.cu).
 int encode_map(mds_ctx* ctx, CUtensorMap* map, const void* ptr, int rows, int half, int boxrows, unsigned prec);
+// 2-D tensor map of a float array rows x cols, boxes of boxcols x boxrows, no
+// swizzle (knn_rms_tc.cu).
+int encode_map_f32(mds_ctx* ctx, CUtensorMap* map, const void* ptr, int64_t rows, int cols, int boxcols, int boxrows);
 
 // tensor-core screen of knn_data (knn_data_tc.cu)
 int tcv_max_kprime();

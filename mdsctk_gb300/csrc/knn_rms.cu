@@ -29,10 +29,57 @@
 
 #include "knn_common.cuh"
 #include "qcp.cuh"
+#include "tc_ptx.cuh"
+#include "warp_sort.cuh"
 
 // ---------------------------------------------------------------------------
 // 1. centring
 // ---------------------------------------------------------------------------
+// Sums of N values over the warp by halving: at each step two values share one
+// exchange, a lane keeping the one for its half, so N values cost about N + 3
+// adds and exchanges instead of 5 N. The sums are those of the xor-shuffle
+// tree, bit for bit (an FP32 add commutes). Value i ends in lane tree_lane(i).
+__host__ __device__ constexpr int tree_lane(int i) {
+  return ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2);
+}
+__device__ __forceinline__ int tree_value(int lane) {  // (lanes of odd number hold none)
+  return (lane & 1) ? 32 : ((lane >> 4) & 1) | (((lane >> 3) & 1) << 1) | (lane & 4) | (((lane >> 1) & 1) << 3);
+}
+template <int N, int O = 16>
+__device__ __forceinline__ float warp_tree(const float (&v)[N], int lane) {
+  constexpr int M = (N + 1) / 2;
+  float r[M];
+  const bool up = (lane & O) != 0;
+#pragma unroll
+  for (int p = 0; p < N / 2; ++p)
+    r[p] = (up ? v[2 * p + 1] : v[2 * p]) + __shfl_xor_sync(0xffffffffu, up ? v[2 * p] : v[2 * p + 1], O);
+  if (N & 1) r[M - 1] = v[N - 1] + __shfl_xor_sync(0xffffffffu, v[N - 1], O);
+  if constexpr (O == 1)
+    return r[0];
+  else
+    return warp_tree<M, O / 2>(r, lane);
+}
+
+// The same over groups of 8 lanes (steps 4, 2, 1): value i ends in the lane
+// whose bits 4, 2, 1 are i's bits 0, 1, 2, as element i >> 3 of out.
+template <int N>
+__device__ __forceinline__ void group8_tree(const float (&v)[N], float (&out)[(N + 7) / 8], int lane) {
+  constexpr int A = (N + 1) / 2, B = (A + 1) / 2, C = (N + 7) / 8;
+  float a[A], b[B];
+  auto step = [&](const float* x, int n, float* y, int o) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int p = 0; p < n / 2; ++p)
+      y[p] = (up ? x[2 * p + 1] : x[2 * p]) + __shfl_xor_sync(0xffffffffu, up ? x[2 * p] : x[2 * p + 1], o);
+    if (n & 1) y[n / 2] = x[n - 1] + __shfl_xor_sync(0xffffffffu, x[n - 1], o);
+  };
+  step(v, N, a, 4);
+  step(a, A, b, 2);
+  step(b, B, out, 1);
+  static_assert((B + 1) / 2 == C, "three halvings");
+}
+__device__ __forceinline__ int group8_value(int gl) { return ((gl >> 2) & 1) | (gl & 2) | ((gl & 1) << 2); }
+
 // Block sum of N float partials: FP32 shuffle tree inside each warp (FP64
 // issues at a small fraction of the FP32 rate on this GPU), then the warps'
 // sums added in FP64 in warp order. red holds (blockDim/32) * N doubles.
@@ -40,17 +87,11 @@
 // only FP64 work) and every thread reads the N sums back.
 template <int N>
 __device__ __forceinline__ void block_sum_vecf(const float (&p)[N], double (&out)[N], double* red) {
-  float v[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    v[i] = p[i];
-    for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-  }
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const float v = warp_tree(p, l);
+  const int iv = tree_value(l);
   __syncthreads();
-  if (l == 0)
-#pragma unroll
-    for (int i = 0; i < N; ++i) red[w * N + i] = (double)v[i];
+  if (iv < N) red[w * N + iv] = (double)v;
   __syncthreads();
   if (threadIdx.x < N) {
     double s = 0;
@@ -70,17 +111,11 @@ __device__ __forceinline__ void block_sum_vecf(const float (&p)[N], double (&out
 // this GPU. red holds (blockDim/32 + 1) * N floats.
 template <int N>
 __device__ __forceinline__ void block_sum_vec32(const float (&p)[N], float (&out)[N], float* red) {
-  float v[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    v[i] = p[i];
-    for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-  }
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const float v = warp_tree(p, l);
+  const int iv = tree_value(l);
   __syncthreads();
-  if (l == 0)
-#pragma unroll
-    for (int i = 0; i < N; ++i) red[w * N + i] = v[i];
+  if (iv < N) red[w * N + iv] = v;
   __syncthreads();
   if (threadIdx.x < N) {
     float s = 0.f;
@@ -108,6 +143,36 @@ __device__ __forceinline__ void df_add_prod(float& hi, float& lo, float a, float
   const float p = __fmul_rn(a, b);
   df_add(hi, lo, p, fmaf(a, b, -p));
 }
+// warp_tree for double-float pairs. Their sum does not commute in the low
+// part: each step adds the upper half's pair to the lower half's, as lane 0's
+// own xor-shuffle tree does, so the value's lane (tree_lane) has lane 0's
+// result bit for bit.
+template <int N, int O = 16>
+__device__ __forceinline__ void warp_tree_df(const float (&h)[N], const float (&l)[N], int lane, float& oh,
+                                             float& ol) {
+  constexpr int M = (N + 1) / 2;
+  float rh[M], rl[M];
+  const bool up = (lane & O) != 0;
+#pragma unroll
+  for (int p = 0; p < N / 2; ++p) {
+    const float gh = __shfl_xor_sync(0xffffffffu, up ? h[2 * p] : h[2 * p + 1], O);
+    const float gl = __shfl_xor_sync(0xffffffffu, up ? l[2 * p] : l[2 * p + 1], O);
+    rh[p] = up ? gh : h[2 * p];
+    rl[p] = up ? gl : l[2 * p];
+    df_add(rh[p], rl[p], up ? h[2 * p + 1] : gh, up ? l[2 * p + 1] : gl);
+  }
+  if (N & 1) {
+    rh[M - 1] = h[N - 1];
+    rl[M - 1] = l[N - 1];
+    df_add(rh[M - 1], rl[M - 1], __shfl_xor_sync(0xffffffffu, h[N - 1], O), __shfl_xor_sync(0xffffffffu, l[N - 1], O));
+  }
+  if constexpr (O == 1) {
+    oh = rh[0];
+    ol = rl[0];
+  } else {
+    warp_tree_df<M, O / 2>(rh, rl, lane, oh, ol);
+  }
+}
 // The 9 sums U[3c+d] = sum_atoms a_c mu_d of a frame as double-float pairs,
 // over the block: out[2i] = hi, out[2i+1] = lo of U[i] (thread 0; red holds
 // (blockDim/32) * 18 floats). Their differences between two frames,
@@ -115,19 +180,14 @@ __device__ __forceinline__ void df_add_prod(float& hi, float& lo, float a, float
 // are kept to about 2^-48 relative.
 __device__ __forceinline__ void block_sum_df9(float (&h)[9], float (&l)[9], float* red, float* out) {
   const int w = threadIdx.x >> 5, ln = threadIdx.x & 31, nw = blockDim.x >> 5;
-#pragma unroll
-  for (int i = 0; i < 9; ++i)
-    for (int o = 16; o > 0; o >>= 1) {
-      const float bh = __shfl_xor_sync(0xffffffffu, h[i], o), bl = __shfl_xor_sync(0xffffffffu, l[i], o);
-      df_add(h[i], l[i], bh, bl);
-    }
+  float vh, vl;
+  warp_tree_df(h, l, ln, vh, vl);
+  const int iv = tree_value(ln);
   __syncthreads();
-  if (ln == 0)
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-      red[w * 18 + 2 * i] = h[i];
-      red[w * 18 + 2 * i + 1] = l[i];
-    }
+  if (iv < 9) {
+    red[w * 18 + 2 * iv] = vh;
+    red[w * 18 + 2 * iv + 1] = vl;
+  }
   __syncthreads();
   if (threadIdx.x < 9) {
     const int i = threadIdx.x;
@@ -319,7 +379,7 @@ __global__ void __launch_bounds__(128) k_prep_out(const float* __restrict__ raw,
       for (int c = 0; c < 3; ++c) o[c * Ap + a] = 0.0f;
     }
   }
-  if (uhl) block_sum_df9(uh, ul, redu, uhl + (int64_t)f * 18);  // uniform branch: all threads or none
+  if (uhl) block_sum_df9(uh, ul, redu, uhl + (int64_t)f * MDS_USTRIDE);  // uniform branch: all threads or none
   const float eup[10] = {ea, u[0], u[1], u[2], u[3], u[4], u[5], u[6], u[7], u[8]};
   float eu[10];
   block_sum_vec32<10>(eup, eu, red);  // every thread has read the record row before this barrier
@@ -644,8 +704,14 @@ int launch_screen_fp32(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, cons
 // RMSD^2 of a pair from its sums w = (D, Q[9]) (see recheck_chunk), the fit
 // row's C6 and U (ui, double-float pairs) and the reference frame's U (uj).
 __device__ __forceinline__ float pair_rmsd2(const float* w, const float* C6, const float* ui,
-                                           const float* __restrict__ uj, bool nofit) {
+                                           const float* __restrict__ ujp, bool nofit) {
   if (nofit) return w[0];
+  float uj[MDS_USTRIDE];
+#pragma unroll
+  for (int i = 0; i < MDS_USTRIDE / 4; ++i) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(ujp) + i);
+    uj[4 * i] = t.x; uj[4 * i + 1] = t.y; uj[4 * i + 2] = t.z; uj[4 * i + 3] = t.w;
+  }
   // P[3r+s] = sum x~_r d_s = Q[3r+s] + sum mu_r d_s, and
   // sum mu_r d_s = U_i[3s+r] - U_j[3s+r] from the frames' double-float U
   float P[9];
@@ -655,7 +721,7 @@ __device__ __forceinline__ float pair_rmsd2(const float* w, const float* C6, con
     for (int ss = 0; ss < 3; ++ss) {
       const int iu = 3 * ss + rr;
       float dh = ui[2 * iu], dl = ui[2 * iu + 1];
-      df_add(dh, dl, -__ldg(uj + 2 * iu), -__ldg(uj + 2 * iu + 1));
+      df_add(dh, dl, -uj[2 * iu], -uj[2 * iu + 1]);
       P[3 * rr + ss] = w[1 + 3 * rr + ss] + (dh + dl);
     }
   return shifted_rmsd2_f32(w[0], C6[0] - P[0], C6[1] - P[4], C6[2] - P[8], 2.0f * C6[3] - (P[1] + P[3]),
@@ -735,7 +801,7 @@ __device__ void recheck_chunk(const float* __restrict__ sa, const float* __restr
   __syncthreads();
   // the eigenvalue solves, one pair per thread
   for (int c = threadIdx.x; c < nc; c += blockDim.x)
-    sd[c] = sqrtf(fmaxf(pair_rmsd2(ssum + c * 10, C6, ui, Ur + (int64_t)cj[c] * 18, nofit), 0.0f));
+    sd[c] = sqrtf(fmaxf(pair_rmsd2(ssum + c * 10, C6, ui, Ur + (int64_t)cj[c] * MDS_USTRIDE, nofit), 0.0f));
   __syncthreads();
 }
 
@@ -825,10 +891,11 @@ __device__ int merge_row_cands(const uint64_t* __restrict__ cand, const int* __r
   return max(within, min(total, k1));
 }
 
-// One block per fit row (rows[b] or b). mode 0: merge nseg candidate lists of
-// K' keys, recheck, select k+1. mode 1: every reference is a candidate
-// (exact row). mode 2 (full matrix): write every exact distance in reference
-// order. Output: out_d/out_i rows of width `width` at row index grow.
+// One block per fit row (rows[b] or b; with nrows_dev the first *nrows_dev
+// rows, in turn over the blocks). mode 0: merge nseg candidate lists of K'
+// keys, recheck, select k+1. mode 1: every reference is a candidate (exact
+// row). Output: out_d/out_i rows of width k at row index grow. For mode 0 this
+// takes the rows that the staged recheck (3b. below) leaves.
 __global__ void __launch_bounds__(RC_THREADS, 4)
 k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const float* __restrict__ mu,
           const float* __restrict__ Ur, int nrows,
@@ -836,7 +903,8 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
           const uint64_t* __restrict__ cand, const int* __restrict__ cand_n, int nseg, int segstride, int Kp, int k,
           double* __restrict__ out_d, int* __restrict__ out_i, int* __restrict__ flagged, int* __restrict__ nflag,
           const float* __restrict__ rowthr, const float* __restrict__ recf, const float* __restrict__ recr,
-          float guard, unsigned long long* __restrict__ audit, int cand_by_row) {
+          float guard, unsigned long long* __restrict__ audit, int cand_by_row,
+          const int* __restrict__ nrows_dev) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* sa = reinterpret_cast<float*>(smem_raw);                 // [3*Ap] a_i
   float* sd = sa + 3 * Ap;                                        // [CHUNK]
@@ -849,29 +917,14 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
   __shared__ float ui[18];                              // the row's U as double-float pairs
   __shared__ float redu[(RC_THREADS / 32) * 18];
 
-  int lr = blockIdx.x;
-  if (lr >= nrows) return;
+  if (nrows_dev) nrows = min(nrows, *nrows_dev);
+  for (int lr = blockIdx.x; lr < nrows; lr += gridDim.x) {
+  __syncthreads();  // (the row before is done with the shared memory)
   int grow = rowlist ? rowlist[lr] : lr;
   const float* af = Af + (int64_t)grow * 3 * Ap;
   for (int e = threadIdx.x; e < 3 * Ap; e += blockDim.x) sa[e] = af[e];
   row_constants(af, mu, Ap, natoms, nofit, C6, ui, s_red, redu);
   const int k1 = k + 1;
-
-  if (mode == 2) {
-    __syncthreads();
-    for (int base = 0; base < Nr; base += RC_CHUNK) {
-      int nc = min(RC_CHUNK, Nr - base);
-      for (int c = threadIdx.x; c < nc; c += blockDim.x) cj[c] = base + c;
-      __syncthreads();
-      recheck_chunk(sa, ui, C6, Ar, Ur, Ap, cj, nc, nofit, sd, ssum);
-      for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-        out_d[(int64_t)grow * Nr + base + c] = (double)sd[c] * 10.0;
-        out_i[(int64_t)grow * Nr + base + c] = base + c;
-      }
-      __syncthreads();
-    }
-    return;
-  }
 
   // Candidate list in keys[0..total): merged and trimmed to K' (mode 0) or
   // implicit 0..Nr-1 (mode 1).
@@ -975,6 +1028,405 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
     out_d[(int64_t)grow * k + x] = (double)mds_key_value(key) * 10.0;
     out_i[(int64_t)grow * k + x] = mds_key_index(key);
   }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 3b. the candidate recheck (mode 0) in stages
+// ---------------------------------------------------------------------------
+// The same values and the same decisions as k_recheck mode 0, without its
+// block-wide phases per row (merging the segment lists, sorting, the solves of
+// a part of the block): at 100,000 x 304, k = 64, those were two thirds of a
+// block's time. In panels of rows whose scratch stays in L2:
+//  0. k_row_const   the row's C6 and U (one block per row; as row_constants).
+//  1. k_rc_cands    a warp per row: the candidates at or below the row's
+//                   threshold, at most RC3_CAP (the smallest bounds when more).
+//  2. k_rc_sums     the ten sums of every candidate pair: a block per row, eight
+//                   lanes per pair as in recheck_chunk.
+//  3. k_rc_finish   a warp per row: the eigenvalue solves (a lane per pair), the
+//                   selection, guard check and audit, the output.
+// Rows with more candidates than that whose next bound does not settle them,
+// with more than RC3_LIST keys, or with fewer than k+1 below the threshold are
+// listed in big[] for k_recheck. 100,000 x 304, k = 64: 5.37 -> RC3_A ms;
+// 20,000 x 1,000, k = 100: 2.41 -> RC3_B ms, outputs bit-identical.
+#define RC3_CAP 128    // candidates per row (256: the rows with more are rechecked in full, 2.63 against 2.37 ms
+                       // at 20,000 x 1,000)
+#define RC3_LIST 512   // keys per row that stage 1 holds
+#define RC3_MAXK1 120  // k + 1 (eight candidates to spare, as the block kernel's first chunk)
+#define RC3_WARPS 8
+
+__global__ void __launch_bounds__(RC_THREADS) k_row_const(const float* __restrict__ Af, const float* __restrict__ mu,
+                                                          int row0, int Ap, int natoms, int nofit,
+                                                          float* __restrict__ rc) {
+  __shared__ double s_red[32 * 6];
+  __shared__ float C6[6], ui[18];
+  __shared__ float redu[(RC_THREADS / 32) * 18];
+  row_constants(Af + (int64_t)(row0 + blockIdx.x) * 3 * Ap, mu, Ap, natoms, nofit, C6, ui, s_red, redu);
+  float* o = rc + (int64_t)blockIdx.x * 24;
+  if (threadIdx.x < 6) o[threadIdx.x] = C6[threadIdx.x];
+  if (threadIdx.x >= 32 && threadIdx.x < 50 && !nofit) o[threadIdx.x - 26] = ui[threadIdx.x - 32];
+}
+
+// meta = (candidates or -1, 1 if further candidates were left out, tau, the
+// smallest bound left out)
+template <int PER>
+__device__ __forceinline__ void rc_sort_write(uint64_t* buf, int m, int Kp, float rthr, int* cidx, float* cbound,
+                                              int4* meta, int lane) {
+  uint64_t v[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) v[i] = (i * 32 + lane < m) ? buf[i * 32 + lane] : MDS_KEY_INF;
+  wsort_u64<PER>(v, lane);
+  const int full = min(m, Kp), nc = min(full, RC3_CAP);
+  const float tau = m >= Kp ? fminf(rthr, mds_key_value(lane_elem<PER>(v, Kp - 1))) : rthr;
+  const float nxt = nc < full ? mds_key_value(lane_elem<PER>(v, nc)) : __int_as_float(0x7f800000);
+#pragma unroll
+  for (int i = 0; i < (PER < RC3_CAP / 32 ? PER : RC3_CAP / 32); ++i) {
+    const int e = i * 32 + lane;
+    if (e < nc) {
+      cidx[e] = mds_key_index(v[i]);
+      cbound[e] = mds_key_value(v[i]);
+    }
+  }
+  if (lane == 0) *meta = make_int4(nc, nc < full ? 1 : 0, __float_as_int(tau), __float_as_int(nxt));
+}
+
+__global__ void __launch_bounds__(RC3_WARPS * 32)
+k_rc_cands(const uint64_t* __restrict__ cand, const int* __restrict__ cand_n, int row0, int rows, int nseg,
+           int segstride, int Kp, int k1, const float* __restrict__ rowthr, int* __restrict__ cidx,
+           float* __restrict__ cbound, int4* __restrict__ meta, int* __restrict__ big, int* __restrict__ nbig) {
+  __shared__ uint64_t s_buf[RC3_WARPS][RC3_LIST];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int rl = blockIdx.x * RC3_WARPS + w;
+  if (rl >= rows) return;
+  const int row = row0 + rl;
+  uint64_t* buf = s_buf[w];
+  const int segn = (lane < nseg) ? min(cand_n[(int64_t)row * nseg + lane], Kp) : 0;
+  const int t = __reduce_add_sync(0xffffffffu, segn);
+  const float rthr = rowthr ? __ldcg(rowthr + row) : __int_as_float(0x7f800000);
+  // the keys at or below the row's threshold (each list ascends, so a list is
+  // left at its first key above it)
+  int m = 0;
+  for (int s = 0; s < nseg; ++s) {
+    const int ns = __shfl_sync(0xffffffffu, segn, s);
+    const uint64_t* src = cand + ((int64_t)row * nseg + s) * segstride;
+    for (int x0 = 0; x0 < ns; x0 += 32) {
+      const int x = x0 + lane;
+      const uint64_t key = (x < ns) ? src[x] : MDS_KEY_INF;
+      const bool keep = x < ns && mds_key_value(key) <= rthr;
+      const unsigned bal = __ballot_sync(0xffffffffu, keep);
+      const int p = m + __popc(bal & ((1u << lane) - 1u));
+      if (keep && p < RC3_LIST) buf[p] = key;
+      m += __popc(bal);
+      if (bal != 0xffffffffu) break;
+    }
+  }
+  __syncwarp();
+  if (m > RC3_LIST || m < min(t, k1)) {
+    if (lane == 0) {
+      meta[rl] = make_int4(-1, 0, 0, 0);
+      big[atomicAdd(nbig, 1)] = row;
+    }
+    return;
+  }
+  int* ci = cidx + (int64_t)rl * RC3_CAP;
+  float* cb = cbound + (int64_t)rl * RC3_CAP;
+  if (m <= RC3_CAP && m < Kp) {  // all of them, in any order
+    for (int x = lane; x < m; x += 32) {
+      ci[x] = mds_key_index(buf[x]);
+      cb[x] = mds_key_value(buf[x]);
+    }
+    if (lane == 0) meta[rl] = make_int4(m, 0, __float_as_int(rthr), 0x7f800000);
+  } else if (m <= 128) {
+    rc_sort_write<4>(buf, m, Kp, rthr, ci, cb, meta + rl, lane);
+  } else if (m <= 256) {
+    rc_sort_write<8>(buf, m, Kp, rthr, ci, cb, meta + rl, lane);
+  } else {
+    rc_sort_write<16>(buf, m, Kp, rthr, ci, cb, meta + rl, lane);
+  }
+}
+
+__global__ void __launch_bounds__(RC_THREADS, 4)
+k_rc_sums(const float* __restrict__ Af, const float* __restrict__ Ar, int row0, int Ap, int nofit,
+          const int* __restrict__ cidx, const int4* __restrict__ meta, float* __restrict__ sums) {
+  extern __shared__ __align__(16) float sa[];  // [3 Ap] a_i
+  const int rl = blockIdx.x;
+  const int nc = meta[rl].x;
+  if (nc <= 0) return;
+  const int Ap4 = Ap >> 2;
+  const float4* af = reinterpret_cast<const float4*>(Af + (int64_t)(row0 + rl) * 3 * Ap);
+  float4* sa4 = reinterpret_cast<float4*>(sa);
+  for (int e = threadIdx.x; e < 3 * Ap4; e += RC_THREADS) sa4[e] = __ldg(af + e);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / RC_GW, gl = lane % RC_GW;
+  __syncthreads();
+  for (int cw = 4 * warp; cw < nc; cw += 4 * (RC_THREADS / 32)) {
+    const int c = cw + grp;
+    const int j = cidx[(int64_t)rl * RC3_CAP + min(c, nc - 1)];
+    const float4* aj4 = reinterpret_cast<const float4*>(Ar + (int64_t)j * 3 * Ap);
+    float2 w[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) w[i] = make_float2(0.0f, 0.0f);
+    for (int q = gl; q < Ap4; q += RC_GW) {
+      const float4 ja = __ldg(aj4 + q), jb = __ldg(aj4 + Ap4 + q), jc = __ldg(aj4 + 2 * Ap4 + q);
+      const float4 ia = sa4[q], ib = sa4[Ap4 + q], ic = sa4[2 * Ap4 + q];
+      pair_acc4(w, ia, ib, ic, ja, jb, jc, nofit != 0);
+    }
+    float v[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) v[i] = w[i].x + w[i].y;
+    float t[2];
+    group8_tree(v, t, lane);
+    if (c < nc) {
+      float* o = sums + ((int64_t)rl * RC3_CAP + c) * 10;
+      const int i = group8_value(gl);
+      o[i] = t[0];
+      if (i < 2) o[8 + i] = t[1];
+    }
+  }
+}
+
+// One row of stage 3 with up to 32 PER candidates. Returns false when the row
+// is not settled (it goes to the block kernel, which rechecks and audits it).
+template <int PER>
+__device__ __forceinline__ bool rc_finish_row(const float* __restrict__ C6, const float* __restrict__ Ur, int nc,
+                                              int4 mt, int nofit, int k, const int* __restrict__ cidx,
+                                              const float* __restrict__ cbound, const float* __restrict__ sums,
+                                              double* __restrict__ od, int* __restrict__ oi,
+                                              const float* __restrict__ recr, float Ei, float guard, bool auditing,
+                                              float& a_coef, int& a_viol, bool& flag, int lane) {
+  uint64_t v[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = i * 32 + lane;
+    v[i] = MDS_KEY_INF;
+    if (e < nc) {
+      const int j = cidx[e];
+      float w[10];
+      const float2* s2 = reinterpret_cast<const float2*>(sums + e * 10);
+#pragma unroll
+      for (int x = 0; x < 5; ++x) {
+        const float2 t = s2[x];
+        w[2 * x] = t.x;
+        w[2 * x + 1] = t.y;
+      }
+      const float sd = sqrtf(fmaxf(pair_rmsd2(w, C6, C6 + 6, Ur + (int64_t)j * MDS_USTRIDE, nofit != 0), 0.0f));
+      v[i] = mds_pack_key(sd, j);
+      if (auditing) {  // (see k_recheck)
+        const float b = cbound[e];
+        if (b > 0.0f) {
+          const float r2 = sd * sd, E = Ei + __ldg(recr + (int64_t)j * MDS_REC + 15);
+          if (E > 0.0f) a_coef = fmaxf(a_coef, (b + guard * E - r2) / E);
+          a_viol += (b > r2 * (1.0f + 3e-5f)) ? 1 : 0;
+        }
+      }
+    }
+  }
+  wsort_u64<PER>(v, lane);
+  const double dk = (double)mds_key_value(lane_elem<PER>(v, k));
+  const double dk2 = dk * dk * (1.0 + 1e-6), tau = (double)__int_as_float(mt.z);
+  if (mt.y && !(dk2 < (double)__int_as_float(mt.w) && dk2 <= tau)) return false;
+  flag = !mt.y && !(dk2 <= tau);
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int e = i * 32 + lane;
+    if (e >= 1 && e <= k) {
+      od[e - 1] = (double)mds_key_value(v[i]) * 10.0;
+      oi[e - 1] = mds_key_index(v[i]);
+    }
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(RC3_WARPS * 32)
+k_rc_finish(const float* __restrict__ rc, const float* __restrict__ Ur, int row0, int rows, int nofit, int k,
+            const int* __restrict__ cidx, const float* __restrict__ cbound, const int4* __restrict__ meta,
+            const float* __restrict__ sums, double* __restrict__ out_d, int* __restrict__ out_i,
+            int* __restrict__ flagged, int* __restrict__ nflag, const float* __restrict__ recf,
+            const float* __restrict__ recr, float guard, unsigned long long* __restrict__ audit,
+            int* __restrict__ big, int* __restrict__ nbig) {
+  __shared__ unsigned s_aud[4];  // pairs, violations, largest error, rows flagged for one
+  if (threadIdx.x < 4) s_aud[threadIdx.x] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, rl = blockIdx.x * RC3_WARPS + (threadIdx.x >> 5);
+  const int4 mt = rl < rows ? meta[rl] : make_int4(-1, 0, 0, 0);
+  const int nc = mt.x;
+  if (nc >= 0) {
+    const int row = row0 + rl;
+    const int64_t at = (int64_t)rl * RC3_CAP;
+    const float Ei = audit ? __ldg(recf + (int64_t)row * MDS_REC + 15) : 0.0f;
+    float a_coef = 0.0f;
+    int a_viol = 0;
+    bool flag = false;
+    const bool done = rc_finish_row<RC3_CAP / 32>(
+        rc + (int64_t)rl * 24, Ur, nc, mt, nofit, k, cidx + at, cbound + at, sums + at * 10, out_d + (int64_t)row * k,
+        out_i + (int64_t)row * k, recr, Ei, guard, audit != nullptr, a_coef, a_viol, flag, lane);
+    if (!done) {
+      if (lane == 0) big[atomicAdd(nbig, 1)] = row;
+    } else {
+      const int viol = __reduce_add_sync(0xffffffffu, a_viol);
+      if (audit) {
+        const unsigned cb = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(a_coef, 0.0f)));
+        if (lane == 0) {
+          atomicAdd(&s_aud[0], (unsigned)nc);
+          if (viol) {
+            atomicAdd(&s_aud[1], (unsigned)viol);
+            atomicAdd(&s_aud[3], 1u);
+          }
+          atomicMax(&s_aud[2], cb);
+        }
+      }
+      if (lane == 0 && (viol > 0 || flag)) flagged[atomicAdd(nflag, 1)] = row;
+    }
+  }
+  __syncthreads();
+  if (audit && threadIdx.x == 0) {
+    if (s_aud[0]) atomicAdd(audit + 0, (unsigned long long)s_aud[0]);
+    if (s_aud[1]) atomicAdd(audit + 1, (unsigned long long)s_aud[1]);
+    if (s_aud[2]) atomicMax(audit + 2, (unsigned long long)s_aud[2]);
+    if (s_aud[3]) atomicAdd(audit + 3, (unsigned long long)s_aud[3]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 3c. every exact distance, in reference order (-s false)
+// ---------------------------------------------------------------------------
+// A block takes FR_R rows x FR_C reference frames at a time, atoms staged in
+// chunks of FR_KC through shared memory (two TMA boxes a chunk, FR_ST stages); a group of 8 lanes sums 2 rows x 2 frames, so each shared-memory load
+// serves two pairs and the FMA pipe, not the L1 pipe, is the bound. Twelve
+// warps of 160 registers. Per pair the sums run over the same atoms in the same
+// lanes and order as in recheck_chunk (bit-identical). 3,001 x 257 atoms: FR_B
+// ms; one row per block, every frame read from L2 for it alone, 2.78 ms. (With
+// each thread issuing its own 16-byte copies 3.6 ms, with a bulk copy per 256
+// contiguous bytes 6.4 ms: the copies' own instructions were the limit.)
+#define FR_R 8
+#define FR_C 24
+#define FR_KC 64  // (Ap is a multiple of it)
+#define FR_ST 4
+#define FR_THREADS 384
+#define FR_FS (3 * FR_KC)  // floats per staged frame (a quarter warp's load is 128 contiguous bytes: no conflicts)
+#define FR_STAGE ((FR_R + FR_C) * FR_FS)
+#define FR_AHEAD 2  // chunks in flight ahead of the one in use (the other stages let the warps drift apart)
+#define FR_SMEM (sizeof(float) * (FR_ST * FR_STAGE + 2 * FR_R * FR_C * 10 + FR_R * 24))
+
+__global__ void __launch_bounds__(FR_THREADS, 1)
+k_full_rows(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUtensorMap tmR,
+            const float* __restrict__ rc, const float* __restrict__ Ur, int nfit, int Nr, int Ap, int nofit, double* __restrict__ out_d,
+            int* __restrict__ out_i, int* __restrict__ err) {
+  extern __shared__ __align__(128) float sm[];
+  __shared__ uint64_t full[FR_ST], empty[FR_ST];
+  __shared__ int s_abort;
+  float* sf = sm;                               // [FR_ST][FR_R + FR_C][FR_FS]
+  float* ssum = sf + FR_ST * FR_STAGE;          // [warp][two tiles of 16 pairs][10]
+  float* src = ssum + 2 * FR_R * FR_C * 10;     // [FR_R][24]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = lane / RC_GW, gl = lane % RC_GW;
+  const int row0 = blockIdx.x * FR_R;
+  const int rp = (warp & 3) * 2, cp = (warp >> 2) * 8 + grp * 2;  // this group's rows and frames in the tile
+  for (int e = threadIdx.x; e < FR_R * 24; e += FR_THREADS)
+    src[e] = rc[(int64_t)min(row0 + e / 24, nfit - 1) * 24 + e % 24];
+  const int nch = Ap / FR_KC, ntile = (Nr + FR_C - 1) / FR_C;
+  const int t0 = (int)((int64_t)ntile * blockIdx.y / gridDim.y), t1 = (int)((int64_t)ntile * (blockIdx.y + 1) / gridDim.y);
+  const int total = (t1 - t0) * nch;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < FR_ST; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], FR_THREADS / 32);
+    }
+    s_abort = 0;
+    mbar_fence_init();
+  }
+  __syncthreads();
+  // chunk n of the block's tiles into its stage: two boxes of FR_KC atoms, the
+  // rows' (frame, coordinate) rows and the reference frames'
+  auto load = [&](int n) {
+    const int tile = t0 + n / nch, kc = n % nch, st = n % FR_ST;
+    mbar_expect_tx(&full[st], FR_STAGE * sizeof(float));
+    tma_load_2d(sf + st * FR_STAGE, &tmF, &full[st], kc * FR_KC, 3 * row0);
+    tma_load_2d(sf + st * FR_STAGE + FR_R * FR_FS, &tmR, &full[st], kc * FR_KC, 3 * tile * FR_C);
+  };
+  int issued = 0;  // (thread 0)
+  if (threadIdx.x == 0)
+    for (; issued < min(FR_AHEAD, total); ++issued) load(issued);
+  int n = 0;
+  bool ok = true;
+  float* wsum = ssum + warp * 320;
+  for (int tile = t0; tile < t1 && ok; ++tile) {
+    float2 w[2][2][10];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 10; ++i) w[a][b][i] = make_float2(0.0f, 0.0f);
+    for (int kc = 0; kc < nch; ++kc, ++n) {
+      const int st = n % FR_ST;
+      // thread 0 keeps FR_AHEAD chunks in flight; the stage a chunk takes was
+      // left by every warp FR_ST - FR_AHEAD chunks ago, mostly
+      if (threadIdx.x == 0 && issued < total) {
+        ok = issued < FR_ST || mbar_wait(&empty[issued % FR_ST], ((issued / FR_ST) & 1) ^ 1, &s_abort);
+        if (ok) load(issued++);
+      }
+      ok = __all_sync(0xffffffffu, ok && mbar_wait(&full[st], (n / FR_ST) & 1, &s_abort));
+      if (!ok) break;
+      const float* xf = sf + st * FR_STAGE + rp * FR_FS;
+      const float* yf = sf + st * FR_STAGE + (FR_R + cp) * FR_FS;
+#pragma unroll
+      for (int q = 0; q < FR_KC / 4 / RC_GW; ++q) {
+        const int at = 4 * (gl + RC_GW * q);
+        float4 x[2][3];
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) x[a][c] = *reinterpret_cast<const float4*>(xf + a * FR_FS + c * FR_KC + at);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          float4 y[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) y[c] = *reinterpret_cast<const float4*>(yf + b * FR_FS + c * FR_KC + at);
+#pragma unroll
+          for (int a = 0; a < 2; ++a)
+            pair_acc4(w[a][b], x[a][0], x[a][1], x[a][2], y[0], y[1], y[2], nofit != 0);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+    }
+    if (!ok) break;
+    // the group's 4 x 10 sums (pair p: row p / 2, frame p % 2); every other
+    // tile, or after the last, a pair per lane for the solves, two tiles of 16
+    // pairs (a tile at a time they took as many issue slots as the sums)
+    float v[40], t[5];
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int i = 0; i < 10; ++i) v[10 * p + i] = w[p >> 1][p & 1][i].x + w[p >> 1][p & 1][i].y;
+    group8_tree(v, t, lane);
+    const int gv = group8_value(gl), half = (tile - t0) & 1;
+#pragma unroll
+    for (int x = 0; x < 5; ++x) wsum[half * 160 + grp * 40 + 8 * x + gv] = t[x];
+    __syncwarp();
+    if (half == 0 && tile + 1 < t1) continue;
+    if (lane < 16 * (half + 1)) {
+      const int tl = tile - half + (lane >> 4), rr = (lane >> 3) & 1, cc = lane & 7;  // frame cc of the warp's eight
+      const int r = rp + rr, row = row0 + r, j = tl * FR_C + (warp >> 2) * 8 + cc;
+      if (row < nfit && j < Nr) {
+        const float* ps = wsum + (lane >> 4) * 160 + (cc >> 1) * 40 + (rr * 2 + (cc & 1)) * 10;
+        const float sd = sqrtf(fmaxf(pair_rmsd2(ps, src + r * 24, src + r * 24 + 6,
+                                                Ur + (int64_t)j * MDS_USTRIDE, nofit != 0), 0.0f));
+        out_d[(int64_t)row * Nr + j] = (double)sd * 10.0;
+        out_i[(int64_t)row * Nr + j] = j;
+      }
+    }
+    __syncwarp();
+  }
+  if (!ok && threadIdx.x == 0) {
+    atomicMax(err, 1);
+    // the copies in flight end, or time out, before the block leaves
+    for (int x = n; x < issued; ++x) {
+      volatile int dummy = 0;
+      mbar_wait(&full[x % FR_ST], (x / FR_ST) & 1, &dummy, 50000000ull);
+    }
+  }
+  if (!ok && lane == 0) s_abort = 1;
+  __syncthreads();
 }
 
 size_t recheck_smem(int Ap, int Kp, int k, int mode) {
@@ -1068,7 +1520,7 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
                    const float* Ur, int nrows, const int* rowlist, int mode,
                    const uint64_t* cand, const int* cand_n, int nseg, int segstride, int Kp, int k,
                    double* out_d, int* out_i, int* flagged, int* nflag, const float* rowthr,
-                   const RecheckAudit* audit, int cand_by_row) {
+                   const RecheckAudit* audit, int cand_by_row, RecheckScratch* rs) {
   size_t smem = recheck_smem(pl.Ap, Kp, k, mode);
   if (mode == 0) {
     // the streaming merge works on the best K' plus one segment's K'
@@ -1084,15 +1536,95 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
   static size_t limit = 0;
   MDS_TRY(mds_allow_dyn_smem(ctx, k_recheck, &attr_set, &limit));
   if (smem > limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "recheck shared memory %zu > %zu", smem, limit);
-  if (nrows > 0) ctx->stats.launches++;
-  if (nrows > 0)
-    k_recheck<<<nrows, RC_THREADS, smem, ctx->stream>>>(Af, Ar, mu, Ur, nrows, rowlist, pl.nref, pl.Ap, pl.natoms,
-                                                        pl.nofit, mode, cand, cand_n, nseg, segstride, Kp, k,
-                                                        out_d, out_i, flagged, nflag, rowthr,
-                                                        audit ? audit->recf : nullptr, audit ? audit->recr : nullptr,
-                                                        audit ? audit->guard : 0.0f,
-                                                        audit ? audit->counters : nullptr, cand_by_row);
+  if (nrows <= 0) return MDS_OK;
+  const float* recf = audit ? audit->recf : nullptr;
+  const float* recr = audit ? audit->recr : nullptr;
+  const float guard = audit ? audit->guard : 0.0f;
+  unsigned long long* counters = audit ? audit->counters : nullptr;
+  cudaStream_t s = ctx->stream;
+  const int* nrows_dev = nullptr;
+  int grid = nrows;
+  if (rs && rs->panel > 0 && mode == 0 && !rowlist && k + 1 <= RC3_MAXK1 && nseg <= 32) {
+    static bool sums_done = false;
+    static size_t sums_limit = 0;
+    MDS_TRY(mds_allow_dyn_smem(ctx, k_rc_sums, &sums_done, &sums_limit));
+    MDS_CUDA(ctx, cudaMemsetAsync(rs->nbig.p, 0, sizeof(int), s));
+    for (int r0 = 0; r0 < nrows; r0 += rs->panel) {
+      const int nr = std::min(rs->panel, nrows - r0), wb = (nr + RC3_WARPS - 1) / RC3_WARPS;
+      ctx->stats.launches += 4;
+      k_row_const<<<nr, RC_THREADS, 0, s>>>(Af, mu, r0, pl.Ap, pl.natoms, pl.nofit, rs->rc.as<float>());
+      k_rc_cands<<<wb, RC3_WARPS * 32, 0, s>>>(cand, cand_n, r0, nr, nseg, segstride, Kp, k + 1, rowthr,
+                                               rs->cidx.as<int>(), rs->cbound.as<float>(), rs->meta.as<int4>(),
+                                               rs->big.as<int>(), rs->nbig.as<int>());
+      k_rc_sums<<<nr, RC_THREADS, sizeof(float) * 3 * pl.Ap, s>>>(
+          Af, Ar, r0, pl.Ap, pl.nofit, rs->cidx.as<int>(), rs->meta.as<int4>(), rs->sums.as<float>());
+      k_rc_finish<<<wb, RC3_WARPS * 32, 0, s>>>(rs->rc.as<float>(), Ur, r0, nr, pl.nofit, k, rs->cidx.as<int>(),
+                                                rs->cbound.as<float>(), rs->meta.as<int4>(), rs->sums.as<float>(),
+                                                out_d, out_i, flagged, nflag, recf, recr, guard, counters,
+                                                rs->big.as<int>(), rs->nbig.as<int>());
+      MDS_CUDA(ctx, cudaGetLastError());
+    }
+    // the rows left, a count only the device knows
+    rowlist = rs->big.as<int>();
+    nrows_dev = rs->nbig.as<int>();
+    cand_by_row = 1;
+    grid = std::min(nrows, 4 * ctx->num_sms);
+  }
+  ctx->stats.launches++;
+  k_recheck<<<grid, RC_THREADS, smem, s>>>(Af, Ar, mu, Ur, nrows, rowlist, pl.nref, pl.Ap, pl.natoms, pl.nofit, mode,
+                                           cand, cand_n, nseg, segstride, Kp, k, out_d, out_i, flagged, nflag, rowthr,
+                                           recf, recr, guard, counters, cand_by_row, nrows_dev);
   MDS_CUDA(ctx, cudaGetLastError());
+  return MDS_OK;
+}
+
+int recheck_scratch(mds_ctx* ctx, int nrows, RecheckScratch& rs) {
+  int panel = std::max(1, std::min(nrows, 16384));  // 100 MB: the pairs' sums stay in L2
+  while (true) {
+    const size_t slots = (size_t)panel * RC3_CAP;
+    if (rs.rc.alloc(ctx, sizeof(float) * 24 * (size_t)panel) == MDS_OK &&
+        rs.meta.alloc(ctx, sizeof(int4) * (size_t)panel) == MDS_OK &&
+        rs.cidx.alloc(ctx, sizeof(int) * slots) == MDS_OK && rs.cbound.alloc(ctx, sizeof(float) * slots) == MDS_OK &&
+        rs.sums.alloc(ctx, sizeof(float) * 10 * slots) == MDS_OK)
+      break;
+    rs.panel = 0;
+    if (panel <= 256) return MDS_OK;  // (a small HBM budget: the block kernel takes every row)
+    panel /= 4;
+  }
+  MDS_TRY(rs.big.alloc(ctx, sizeof(int) * (size_t)std::max(nrows, 1)));
+  MDS_TRY(rs.nbig.alloc(ctx, sizeof(int)));
+  rs.panel = panel;
+  return MDS_OK;
+}
+size_t recheck_scratch_bytes(int nrows) {
+  return (size_t)std::min(nrows, 16384) * (96 + 16 + RC3_CAP * 48) + sizeof(int) * (size_t)nrows + 4096;
+}
+
+// The full matrix of exact distances (rc: the rows' constants, [nfit][24]).
+static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const float* Ar, const float* mu,
+                            const float* Ur, int nfit, double* out_d, int* out_i) {
+  DevBuf rc(ctx), err(ctx);
+  MDS_TRY(rc.alloc(ctx, sizeof(float) * 24 * (size_t)nfit));
+  MDS_TRY(err.alloc(ctx, sizeof(int)));
+  MDS_CUDA(ctx, cudaMemsetAsync(err.p, 0, sizeof(int), ctx->stream));
+  const int nrt = (nfit + FR_R - 1) / FR_R, ntile = (pl.nref + FR_C - 1) / FR_C;
+  // column ranges so that there are about 8 blocks per SM
+  const int ny = std::max(1, std::min(std::min(ntile, 65535), (8 * ctx->num_sms + nrt - 1) / nrt));
+  ctx->stats.launches += 2;
+  k_row_const<<<nfit, RC_THREADS, 0, ctx->stream>>>(Af, mu, 0, pl.Ap, pl.natoms, pl.nofit, rc.as<float>());
+  static bool attr_done = false;
+  static size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_full_rows, &attr_done, &attr_limit));
+  CUtensorMap mF, mR;
+  MDS_TRY(encode_map_f32(ctx, &mF, Af, (int64_t)3 * nfit, pl.Ap, FR_KC, 3 * FR_R));
+  MDS_TRY(encode_map_f32(ctx, &mR, Ar, (int64_t)3 * pl.nref, pl.Ap, FR_KC, 3 * FR_C));
+  k_full_rows<<<dim3(nrt, ny), FR_THREADS, FR_SMEM, ctx->stream>>>(mF, mR, rc.as<float>(), Ur, nfit, pl.nref, pl.Ap,
+                                                                   pl.nofit, out_d, out_i, err.as<int>());
+  MDS_CUDA(ctx, cudaGetLastError());
+  int herr = 0;
+  MDS_CUDA(ctx, cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  MDS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  if (herr) return mds_fail(ctx, MDS_ERR_TIMEOUT, "full matrix: a bounded wait timed out");
   return MDS_OK;
 }
 
@@ -1262,7 +1794,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   MDS_TRY(Ar.alloc(ctx, sizeof(float) * 3 * Ap * (size_t)nref));
   MDS_TRY(Rr.alloc(ctx, sizeof(float) * MDS_REC * (size_t)nref));
   DevBuf Ur(ctx);  // the reference frames' U = sum a mu^T as double-float pairs (recheck)
-  MDS_TRY(Ur.alloc(ctx, sizeof(float) * 18 * (size_t)nref));
+  MDS_TRY(Ur.alloc(ctx, sizeof(float) * MDS_USTRIDE * (size_t)nref));
   // frames with a non-finite coordinate (reference set, fit set): smallest
   // index, checked at the call's first synchronisation after the screen
   DevBuf badf(ctx);
@@ -1276,7 +1808,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       const int f0 = cb[c], nf = cb[c + 1] - cb[c];
       MDS_TRY(launch_prep(ctx, draw + (size_t)f0 * 3 * natoms, nf, natoms, Ap, dmass.as<float>(), dswn.as<float>(),
                           tm, dmu.as<float>(), dM0.as<double>(), pl.nofit, A + (size_t)f0 * 3 * Ap,
-                          R + (size_t)f0 * MDS_REC, U ? U + (size_t)f0 * 18 : nullptr, bad, f0));
+                          R + (size_t)f0 * MDS_REC, U ? U + (size_t)f0 * MDS_USTRIDE : nullptr, bad, f0));
     }
     return MDS_OK;
   };
@@ -1303,7 +1835,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       MDS_TRY(launch_prep(ctx, draw_ref + (size_t)f0 * 3 * natoms, f1 - f0, natoms, Ap, dmass.as<float>(),
                           dswn.as<float>(), tm, dmu.as<float>(), dM0.as<double>(), pl.nofit,
                           Ar.as<float>() + (size_t)f0 * 3 * Ap, Rr.as<float>() + (size_t)f0 * MDS_REC,
-                          pl.nofit ? nullptr : Ur.as<float>() + (size_t)f0 * 18, badf.as<int>(), f0));
+                          pl.nofit ? nullptr : Ur.as<float>() + (size_t)f0 * MDS_USTRIDE, badf.as<int>(), f0));
       MDS_TRY(tc_prepare_range(ctx, pl, Ar.as<float>(), nref, tcr, 1, f0, f1));
       MDS_TRY(tc_prepare_range(ctx, pl, Ar.as<float>(), nref, tcr, 0, f0, f1));
       MDS_TRY(tc_pivots_radii(ctx, pl, Ar.as<float>(), spv, f0, f1));
@@ -1334,8 +1866,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   }
   if (pl.full) {
     MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), nfit, nullptr, 2, nullptr, nullptr, 1, 1,
-                           1, 0, dout_d, dout_i, flagged.as<int>(), nflag.as<int>()));
+    MDS_TRY(launch_full_rows(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), nfit, dout_d, dout_i));
     MDS_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
     int hbad[2] = {0, 0};
     MDS_CUDA(ctx, cudaMemcpyAsync(hbad, badf.p, sizeof(hbad), cudaMemcpyDeviceToHost, s));
@@ -1496,9 +2027,12 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   audit.recr = Rr.as<float>();
   audit.guard = (pl.prec == MDS_PREC_FP32) ? pl.guard_fp32 : pl.guard_tc;
   audit.counters = audit_c.as<unsigned long long>();
+  RecheckScratch rs;
+  MDS_TRY(recheck_scratch(ctx, nfit, rs));
   MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), nfit, nullptr, 0,
                          cand.as<uint64_t>(), cand_n.as<int>(), nseg, segstride, Kp, k, dout_d, dout_i,
-                         flagged.as<int>(), nflag.as<int>(), rowthr.p ? rowthr.as<float>() : nullptr, &audit));
+                         flagged.as<int>(), nflag.as<int>(), rowthr.p ? rowthr.as<float>() : nullptr, &audit, 0,
+                         &rs));
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
   int hflag = 0, hbad[2] = {0, 0}, herr[4 + 2 * MDS_MAX_CHUNKS] = {};
   unsigned long long hc[4] = {0, 0, 0, 0};

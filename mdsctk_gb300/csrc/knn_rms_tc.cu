@@ -810,7 +810,7 @@ typedef CUresult (*PFN_encodeTiled_t)(CUtensorMap*, CUtensorMapDataType, cuuint3
                                       CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                       CUtensorMapFloatOOBfill);
 
-int encode_map(mds_ctx* ctx, CUtensorMap* map, const void* ptr, int rows, int Ap, int boxrows, unsigned prec) {
+static int encode_fn(mds_ctx* ctx, PFN_encodeTiled_t* out) {
   static PFN_encodeTiled_t fn = nullptr;
   if (!fn) {
     void* p = nullptr;
@@ -821,15 +821,33 @@ int encode_map(mds_ctx* ctx, CUtensorMap* map, const void* ptr, int rows, int Ap
       return mds_fail(ctx, MDS_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
     fn = reinterpret_cast<PFN_encodeTiled_t>(p);
   }
-  cuuint64_t gdim[2] = {(cuuint64_t)(2 * Ap), (cuuint64_t)rows};
-  cuuint64_t gstride[1] = {(cuuint64_t)(2 * Ap) * 2};
-  cuuint32_t box[2] = {TC_KB, (cuuint32_t)boxrows};
+  *out = fn;
+  return MDS_OK;
+}
+
+static int encode_2d(mds_ctx* ctx, CUtensorMap* map, CUtensorMapDataType type, int esize, const void* ptr,
+                     int64_t rows, int64_t cols, int boxcols, int boxrows, CUtensorMapSwizzle swizzle) {
+  PFN_encodeTiled_t fn = nullptr;
+  MDS_TRY(encode_fn(ctx, &fn));
+  cuuint64_t gdim[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t gstride[1] = {(cuuint64_t)cols * esize};
+  cuuint32_t box[2] = {(cuuint32_t)boxcols, (cuuint32_t)boxrows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, prec == MDS_PREC_FP16X3 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-                  2, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  CUresult r = fn(map, type, 2, const_cast<void*>(ptr), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return mds_fail(ctx, MDS_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   return MDS_OK;
+}
+
+int encode_map(mds_ctx* ctx, CUtensorMap* map, const void* ptr, int rows, int Ap, int boxrows, unsigned prec) {
+  return encode_2d(ctx, map,
+                   prec == MDS_PREC_FP16X3 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr,
+                   rows, 2 * Ap, TC_KB, boxrows, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+
+int encode_map_f32(mds_ctx* ctx, CUtensorMap* map, const void* ptr, int64_t rows, int cols, int boxcols, int boxrows) {
+  return encode_2d(ctx, map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, ptr, rows, cols, boxcols, boxrows,
+                   CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 int tc_choose_nseg(mds_ctx* ctx, const KnnRmsPlan& pl, int nfit) {

@@ -122,6 +122,7 @@ struct Slot {
   int cap = 0;
   DevBuf raw, A, R, cand, cand_n, out_d, out_i, flagged, nflag, derr, ext, lb, rowthr;
   DevBuf audit;  // the recheck's audit counters of the screen's bounds (4 x u64)
+  RecheckScratch rs;
   TcOperands tcq;
   float* h_raw = nullptr;
   double* h_d = nullptr;
@@ -233,7 +234,7 @@ static int launch_batch(mds_server* S, Slot& sl, int bucket) {
   MDS_TRY(launch_recheck(c, pl, sl.A.as<float>(), S->A.as<float>(), S->dmu.as<float>(), S->U.as<float>(), bucket,
                          nullptr, 0, sl.cand.as<uint64_t>(), sl.cand_n.as<int>(), nseg, segstride, S->Kp, S->k,
                          sl.out_d.as<double>(), sl.out_i.as<int>(), sl.flagged.as<int>(), sl.nflag.as<int>(),
-                         S->prec == MDS_PREC_FP32 ? nullptr : sl.rowthr.as<float>(), &audit));
+                         S->prec == MDS_PREC_FP32 ? nullptr : sl.rowthr.as<float>(), &audit, 0, &sl.rs));
   c->stats.launches++;
   k_serve_ext<<<(bucket + SE_WARPS - 1) / SE_WARPS, SE_WARPS * 32, serve_ext_smem(S->k), c->stream>>>(
       sl.out_d.as<double>(), sl.out_i.as<int>(), bucket, S->k, S->cfg.sigma, S->ddinv.as<double>(),
@@ -451,6 +452,7 @@ static size_t slot_bytes(const mds_server* S, int cap) {
   b += (size_t)cap * S->nseg_max * S->segstride * 8 + (size_t)cap * S->nseg_max * 4;
   b += (size_t)cap * S->k * 12 + (size_t)cap * S->nev * 8 + (size_t)cap * 4;
   b += (size_t)cap * S->pv.nC * 4;                            // pivot bounds
+  b += recheck_scratch_bytes(cap);
   return b + (64u << 20);
 }
 
@@ -525,7 +527,7 @@ static int build_model(mds_server* S, const float* hxyz, const float* hmass) {
   MDS_CUDA(c, cudaMemcpyAsync(S->dM0.p, M0, sizeof(double) * 9, cudaMemcpyHostToDevice, s));
   MDS_TRY(S->A.alloc(c, sizeof(float) * 3 * (size_t)Ap * n));
   MDS_TRY(S->R.alloc(c, sizeof(float) * MDS_REC * (size_t)n));
-  MDS_TRY(S->U.alloc(c, sizeof(float) * 18 * (size_t)n));
+  MDS_TRY(S->U.alloc(c, sizeof(float) * MDS_USTRIDE * (size_t)n));
   MDS_TRY(launch_prep(c, raw.as<float>(), n, natoms, Ap, S->dmass.as<float>(), S->dswn.as<float>(), tm,
                       S->dmu.as<float>(), S->dM0.as<double>(), (S->cfg.flags & MDS_NOFIT) ? 1 : 0, S->A.as<float>(),
                       S->R.as<float>(), (S->cfg.flags & MDS_NOFIT) ? nullptr : S->U.as<float>()));
@@ -592,7 +594,8 @@ extern "C" int mds_server_create(const mds_server_config* cfg, const float* land
               sl.audit.alloc(c, 4 * sizeof(unsigned long long)) == MDS_OK &&
               sl.derr.alloc(c, 4 * sizeof(int)) == MDS_OK && sl.rowthr.alloc(c, sizeof(float) * cap) == MDS_OK &&
               (S->pv.nC == 0 || sl.lb.alloc(c, sizeof(float) * (size_t)S->pv.nC * cap) == MDS_OK) &&
-              sl.ext.alloc(c, sizeof(double) * (size_t)cap * S->nev) == MDS_OK;
+              sl.ext.alloc(c, sizeof(double) * (size_t)cap * S->nev) == MDS_OK &&
+              recheck_scratch(c, cap, sl.rs) == MDS_OK;
     if (!ok) {
       S->last_error = mds_last_error(c);
       return MDS_ERR_NOMEM;
@@ -633,11 +636,14 @@ extern "C" int mds_server_destroy(mds_server* S) {
     sl.raw.release(); sl.A.release(); sl.R.release(); sl.cand.release();
     sl.cand_n.release(); sl.out_d.release(); sl.out_i.release(); sl.flagged.release(); sl.nflag.release();
     sl.derr.release(); sl.ext.release(); sl.tcq.A.release(); sl.tcq.B.release(); sl.lb.release(); sl.rowthr.release();
+    sl.audit.release(); sl.rs.rc.release(); sl.rs.meta.release(); sl.rs.cidx.release(); sl.rs.cbound.release();
+    sl.rs.sums.release(); sl.rs.big.release(); sl.rs.nbig.release();
     mds_destroy(sl.ctx);
   }
   S->dmass.release(); S->dswn.release(); S->dmu.release(); S->dM0.release(); S->Y.release(); S->E.release();
   S->A.release(); S->R.release(); S->U.release(); S->dZ.release(); S->ddinv.release(); S->dZl.release(); S->tc.A.release();
   S->tc.B.release(); S->nmax.release();
+  S->pv.idx.release(); S->pv.rrad.release();
   S->pv.A.release(); S->pv.R.release(); S->pv.rad.release(); S->pv.tc.A.release(); S->pv.tc.B.release();
   mds_destroy(S->main);
   delete S;
