@@ -8,11 +8,13 @@
 //                  for the correlation metric the reference's own sums in its
 //                  order (sum, sum of squares -> mean and scale) and the
 //                  standardized FP32 vector.
-//  2. k_screen_dot all pairs: FP32 dot products on CUDA cores (64 x 64 tile,
-//                  4 x 4 pairs per thread), screen value = lower bound of the
-//                  squared distance (Euclidean: |x|^2 + |y|^2 - 2 x.y, minus a
-//                  rounding guard; correlation: (1 - r)/2 minus a guard),
-//                  fused per-row top-K' in shared memory.
+//  2. k_dot_panel  all pairs: FP32 dot products on CUDA cores, screen value =
+//                  lower bound of the squared distance (Euclidean: |x|^2 +
+//                  |y|^2 - 2 x.y, minus a rounding guard; correlation:
+//                  (1 - r)/2 minus a guard), a panel of rows at a time;
+//     k_panel_select  the K' smallest values of each row.
+//     k_screen_dot is both in one kernel, with the lists in shared memory, for
+//     calls without room for a panel.
 //  3. k_data_recheck merge the column segments, recompute every candidate in
 //                  FP64 with the reference's exact operation order (no fused
 //                  multiply-add, sequential sum), select k+1 by (value, index),
@@ -220,6 +222,242 @@ static size_t screen_dot_smem(int Kp) {
   return sizeof(float) * (2 * DT_TM * DT_FS + 2 * DT_TN * DT_FS + DT_TN) + sizeof(int) * DT_TM +
          sizeof(float) * DT_TM + sizeof(uint64_t) * DT_TM * next_pow2(Kp + DT_TN);
 }
+
+// ---------------------------------------------------------------------------
+// 2b. screen through a panel: the values of all pairs, then the lists
+// ---------------------------------------------------------------------------
+// The same screen values as k_screen_dot (the same order of operations),
+// written to panels of rows in global memory, and the same lists (the K'
+// smallest values of each row) taken from the panel by one warp per row and
+// segment of columns. Apart, the product runs as a matrix product and a row is
+// thinned out a few times; k_screen_dot sorts every row's pool after each 64
+// columns of each of its segments, which is most of its time. Measured, values
+// and lists against k_screen_dot: 5,003 x 20,011 of 50 components 0.37 / 7.2
+// ms; 100,000 x 100,000 of 64 39 / 1,419 ms; 1 x 200,000 0.12 / 2.8 ms; 400 x
+// 400 of 16 0.015 / 0.080 ms: no size was found at which k_screen_dot wins, so
+// it runs only where the panel's memory is missing (and in the entry point
+// that may not allocate).
+#define DP_TM 64       // rows of a tile
+#define DP_T 128       // columns of a tile
+#define DP_THREADS 128 // 8 x 8 pairs per thread
+#define DP_BLOCKS 4    // per SM
+#define DP_TY (DP_THREADS / 16)
+#define DP_PR (DP_TM / DP_TY)  // rows per thread
+#define DP_PANEL_BYTES ((int64_t)1 << 30)
+#define DS_WARPS 8
+
+// S[i][ld] for the rows [row0, row0 + nrows) of the fit set against every
+// reference vector; the columns Nr .. ld - 1 get +inf. `ka` = dim rounded up
+// to 4 (the operands are zero from dim to Dp). Bound by the FP32 pipe and the
+// shared-memory reads that feed it (one 128-bit read per 16 multiply-adds, as
+// many cycles of one as of the other). 5,003 x 20,011 x 50: 0.264 ms (0.145 ms
+// of multiply-adds); 128 x 128 tiles with 256 threads, two blocks per SM, 0.273
+// ms; 16 x 8 pairs per thread 0.294 ms (fewer reads, too few warps).
+__global__ void __launch_bounds__(DP_THREADS, DP_BLOCKS)
+k_dot_panel(const float* __restrict__ Xf, const float* __restrict__ Xr, const float* __restrict__ nf,
+            const float* __restrict__ nr, int row0, int nrows, int Nr, int Dp, int ka, int corr, float guard,
+            int nrt, int64_t ld, float* __restrict__ S) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float* sf = reinterpret_cast<float*>(smem_raw);  // [2][DP_TM * DT_FS]
+  float* sr = sf + 2 * DP_TM * DT_FS;              // [2][DP_T * DT_FS]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;  // ty < DP_TY
+  const int rt = blockIdx.x % nrt, ct = blockIdx.x / nrt;
+  const int nch = (ka + DT_KC - 1) / DT_KC;
+  auto load = [&](int stage, int kc) {
+    float* df = sf + stage * DP_TM * DT_FS;
+    float* dr = sr + stage * DP_T * DT_FS;
+#pragma unroll
+    for (int e = tid; e < DP_T * 8; e += DP_THREADS) {
+      const int v = e >> 3, h = e & 7;
+      const int i = rt * DP_TM + v, j = ct * DP_T + v;
+      if (v < DP_TM)
+        cpa16(df + v * DT_FS + 4 * h, Xf + (int64_t)(i < nrows ? row0 + i : 0) * Dp + kc * DT_KC + 4 * h,
+              i < nrows);
+      cpa16(dr + v * DT_FS + 4 * h, Xr + (int64_t)(j < Nr ? j : 0) * Dp + kc * DT_KC + 4 * h, j < Nr);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+  };
+  float acc[DP_PR][8];
+#pragma unroll
+  for (int p = 0; p < DP_PR; ++p)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[p][q] = 0.f;
+  load(0, 0);
+  for (int kc = 0; kc < nch; ++kc) {
+    if (kc + 1 < nch) {
+      load((kc + 1) & 1, kc + 1);
+      asm volatile("cp.async.wait_group 1;\n" ::);
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::);
+    }
+    __syncthreads();
+    const float* df = sf + (kc & 1) * DP_TM * DT_FS + ty * DT_FS;
+    const float* dr = sr + (kc & 1) * DP_T * DT_FS + tx * DT_FS;
+    const int kn = min(DT_KC, ka - kc * DT_KC);
+#pragma unroll 1
+    for (int a = 0; a < kn; a += 4) {
+      float4 rv[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) rv[q] = *reinterpret_cast<const float4*>(dr + 16 * q * DT_FS + a);
+#pragma unroll
+      for (int p = 0; p < DP_PR; ++p) {
+        const float4 fv = *reinterpret_cast<const float4*>(df + DP_TY * p * DT_FS + a);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(fv.x, rv[q].x, acc[p][q]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(fv.y, rv[q].y, acc[p][q]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(fv.z, rv[q].z, acc[p][q]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(fv.w, rv[q].w, acc[p][q]);
+      }
+    }
+    __syncthreads();
+  }
+  float cn[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int j = ct * DP_T + tx + 16 * q;
+    cn[q] = j < Nr ? nr[j] : 0.f;
+  }
+#pragma unroll
+  for (int p = 0; p < DP_PR; ++p) {
+    const int i = rt * DP_TM + ty + DP_TY * p;
+    if (i >= nrows) continue;
+    const float rn = nf[row0 + i];
+    float* o = S + (int64_t)i * ld;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int j = ct * DP_T + tx + 16 * q;
+      float v = corr ? 0.5f * (1.0f - acc[p][q]) : rn + cn[q] - 2.0f * acc[p][q];
+      v = fmaxf(v - guard * (rn + cn[q]), 0.0f);
+      o[j] = j < Nr ? v : __int_as_float(0x7f800000);
+    }
+  }
+}
+
+static size_t dot_panel_smem() { return sizeof(float) * 2 * (DP_TM + DP_T) * DT_FS; }
+
+// Keeps the smallest of a row's n <= 32 PER keys: all with a value at or below
+// the returned threshold, at least Kp and at most Kp + slack of them (any ties
+// of the Kp-th beyond that are dropped). The threshold is found by bisecting
+// the values' bits (they are non-negative, so the bits order as integers)
+// with the keys in registers: a count is PER compares and one reduction, where
+// a bitonic sort of 256 keys takes 36 steps of PER exchanges each (with pools
+// of 512 keys sorted: 0.466 ms of k_panel_select at 5,003 x 20,011, now 0.105).
+template <int PER>
+__device__ __forceinline__ int ds_compact(uint64_t* pool, int n, int Kp, int slack, int lane, float& thr) {
+  if (n <= Kp) return n;
+  uint64_t v[PER];
+  unsigned lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    v[i] = i * 32 + lane < n ? pool[i * 32 + lane] : MDS_KEY_INF;
+    if (i * 32 + lane < n) {
+      lo = min(lo, (unsigned)(v[i] >> 32));
+      hi = max(hi, (unsigned)(v[i] >> 32));
+    }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  // smallest t in [lo, hi] with count(value <= t) >= Kp, or any t whose count
+  // is within the slack
+  int c = n;
+  while (lo < hi) {
+    const unsigned mid = lo + ((hi - lo) >> 1);
+    int m = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) m += (unsigned)(v[i] >> 32) <= mid;
+    m = __reduce_add_sync(0xffffffffu, m);
+    if (m >= Kp) {
+      hi = mid;
+      c = m;
+      if (m <= Kp + slack) break;
+    } else {
+      lo = mid + 1;
+    }
+  }
+  const unsigned t = hi;
+  const bool ties = c > Kp + slack;  // (then t is the Kp-th value itself)
+  __syncwarp();
+  int o = 0;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const unsigned x = (unsigned)(v[i] >> 32);
+    const bool in = ties ? x < t : x <= t;
+    const unsigned b = __ballot_sync(0xffffffffu, in);
+    if (in) pool[o + __popc(b & ((1u << lane) - 1))] = v[i];
+    o += __popc(b);
+  }
+  if (ties) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const bool in = (unsigned)(v[i] >> 32) == t;
+      const unsigned b = __ballot_sync(0xffffffffu, in);
+      const int at = o + __popc(b & ((1u << lane) - 1));
+      if (in && at < Kp) pool[at] = v[i];
+      o = min(o + __popc(b), Kp);
+    }
+  }
+  thr = __uint_as_float(t);
+  __syncwarp();
+  return o;
+}
+
+// The K' smallest of S[i][c0, c1), one warp per row and segment of columns:
+// 128 columns per step, two steps in flight; values below the threshold (at
+// or above the K'-th smallest so far) go to the row's pool of 32 PER keys.
+// Bound by the ballots of the steps that hold a value below the threshold
+// (0.4 GB read in 0.105 ms at 5,003 x 20,011).
+template <int PER>
+__global__ void __launch_bounds__(DS_WARPS * 32)
+k_panel_select(const float* __restrict__ S, int64_t ld, int row0, int nrows, int nseg, int Kp,
+               uint64_t* __restrict__ cand, int* __restrict__ cand_n) {
+  __shared__ uint64_t pools[DS_WARPS][32 * PER];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t item = (int64_t)blockIdx.x * DS_WARPS + warp;
+  if (item >= (int64_t)nrows * nseg) return;
+  const int i = (int)(item / nseg), seg = (int)(item % nseg);
+  const int steps = (int)(ld / 128);
+  const int s0 = (int)((int64_t)steps * seg / nseg), s1 = (int)((int64_t)steps * (seg + 1) / nseg);
+  const float4* g = reinterpret_cast<const float4*>(S + (int64_t)i * ld) + lane;
+  uint64_t* pool = pools[warp];
+  const float inf = __int_as_float(0x7f800000);
+  float thr = inf;
+  int n = 0;
+  const float4 none = make_float4(inf, inf, inf, inf);
+  float4 nx[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) nx[u] = s0 + u < s1 ? __ldcs(g + (int64_t)(s0 + u) * 32) : none;
+  for (int st = s0; st < s1; st += 2) {
+    float4 cur[2] = {nx[0], nx[1]};
+#pragma unroll
+    for (int u = 0; u < 2; ++u) nx[u] = st + 2 + u < s1 ? __ldcs(g + (int64_t)(st + 2 + u) * 32) : none;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float v[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const unsigned m = __ballot_sync(0xffffffffu, v[c] < thr);
+        if (m == 0) continue;
+        if (v[c] < thr)
+          pool[n + __popc(m & ((1u << lane) - 1))] = mds_pack_key(v[c], (st + u) * 128 + 4 * lane + c);
+        n += __popc(m);
+      }
+      if (n > 32 * PER - 128) {
+        __syncwarp();
+        n = ds_compact<PER>(pool, n, Kp, 8, lane, thr);
+      }
+    }
+  }
+  __syncwarp();
+  n = ds_compact<PER>(pool, n, Kp, 0, lane, thr);
+  const int64_t list = (int64_t)(row0 + i) * nseg + seg;
+  for (int x = lane; x < n; x += 32) cand[list * Kp + x] = pool[x];
+  if (lane == 0) cand_n[list] = n;
+}
+#define DS_SMALL_KP 96  // K' up to which a pool of 256 keys is used, else 512
+static_assert(DS_SMALL_KP + 8 <= 256 - 128 && DT_MAX_KP + 8 <= 512 - 128, "a pool keeps room for a step");
 
 // ---------------------------------------------------------------------------
 // 3. exact recheck in the reference's arithmetic
@@ -758,9 +996,29 @@ int knn_data_run(mds_ctx* ctx, const double* dref, int nref, const double* dfit,
   }
   const float guard = MDS_GUARD_FP32;
   if (tc) nseg = tcv_choose_nseg(ctx, nfit, nref);
-  DevBuf cand(ctx), cand_n(ctx), rows(ctx), rthr(ctx);
-  MDS_TRY(cand.alloc(ctx, sizeof(uint64_t) * (size_t)nfit * nseg * Kp));
-  MDS_TRY(cand_n.alloc(ctx, sizeof(int) * (size_t)nfit * nseg));
+  DevBuf cand(ctx), cand_n(ctx), rows(ctx), rthr(ctx), panel(ctx);
+  auto alloc_lists = [&](int segs) -> int {
+    MDS_TRY(cand.alloc(ctx, sizeof(uint64_t) * (size_t)nfit * segs * Kp));
+    return cand_n.alloc(ctx, sizeof(int) * (size_t)nfit * segs);
+  };
+  // FP32 screen of a large set: values in panels, then lists
+  const int pct = (nref + DP_T - 1) / DP_T;
+  const int64_t ld = (int64_t)pct * DP_T;
+  int prows = 0;  // rows of a panel (0: k_screen_dot)
+  if (!tc && nfit > 0) {
+    // a warp per row and segment: enough warps for every SM, and lists that
+    // the recheck can merge in registers
+    const int seg = std::min({std::max(RW_MAXT / Kp, 1), pct, ctx->num_sms * 32 / nfit + 1});
+    prows = (int)std::min<int64_t>(nfit, std::max<int64_t>(DP_PANEL_BYTES / (ld * 4) / DP_T, 1) * DP_T);
+    if (panel.alloc(ctx, sizeof(float) * (size_t)ld * prows) == MDS_OK && alloc_lists(seg) == MDS_OK) {
+      nseg = seg;
+    } else {  // (a small HBM budget)
+      prows = 0;
+      panel.release();
+      mds_trim_cache(ctx, 0);
+    }
+  }
+  if (prows == 0) MDS_TRY(alloc_lists(nseg));
   size_t smem = screen_dot_smem(Kp);
   st.screen_launches = 1;
   if (tc) {
@@ -769,6 +1027,27 @@ int knn_data_run(mds_ctx* ctx, const double* dref, int nref, const double* dfit,
     MDS_TRY(launch_screen_tcv(ctx, xf, nfp, nfit, Xr.as<float>(), Nrm.as<float>(), nref, Dp, corr, Kp, k, nseg, same,
                               !noskip, cand.as<uint64_t>(), cand_n.as<int>(), rthr.as<float>(), &tiles));
     st.screen_pairs = tiles * 256LL * 128LL;
+  } else if (prows > 0) {
+    const size_t psm = dot_panel_smem();
+    MDS_CUDA(ctx, cudaFuncSetAttribute(k_dot_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+    st.screen_launches = 0;
+    for (int r0 = 0; r0 < nfit; r0 += prows) {
+      const int nr = std::min(prows, nfit - r0), prt = (nr + DP_TM - 1) / DP_TM;
+      st.launches += 2;
+      st.screen_launches++;
+      k_dot_panel<<<(unsigned)((int64_t)prt * pct), DP_THREADS, psm, s>>>(
+          xf, Xr.as<float>(), nfp, Nrm.as<float>(), r0, nr, nref, Dp, mds_round_up(dim, 4), corr, guard, prt, ld,
+          panel.as<float>());
+      const int sgrid = (int)(((int64_t)nr * nseg + DS_WARPS - 1) / DS_WARPS);
+      if (Kp <= DS_SMALL_KP)
+        k_panel_select<8><<<sgrid, DS_WARPS * 32, 0, s>>>(panel.as<float>(), ld, r0, nr, nseg, Kp,
+                                                          cand.as<uint64_t>(), cand_n.as<int>());
+      else
+        k_panel_select<16><<<sgrid, DS_WARPS * 32, 0, s>>>(panel.as<float>(), ld, r0, nr, nseg, Kp,
+                                                           cand.as<uint64_t>(), cand_n.as<int>());
+    }
+    MDS_CUDA(ctx, cudaGetLastError());
+    panel.release();
   } else {
     MDS_CUDA(ctx, cudaFuncSetAttribute(k_screen_dot, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     st.launches++;
