@@ -52,26 +52,6 @@ struct TcOperands {
   int K = 0;       // padded atoms per split part (row length is 2K: hi | lo)
 };
 
-__device__ __forceinline__ void warp_bitonic_sort(uint64_t* a, int n, int P2, int lane) {
-  for (int x = n + lane; x < P2; x += 32) a[x] = MDS_KEY_INF;
-  __syncwarp();
-  for (int k = 2; k <= P2; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = lane; i < P2; i += 32) {
-        int ixj = i ^ j;
-        if (ixj > i) {
-          uint64_t x = a[i], y = a[ixj];
-          bool up = (i & k) == 0;
-          if ((x > y) == up) {
-            a[i] = y;
-            a[ixj] = x;
-          }
-        }
-      }
-      __syncwarp();
-    }
-}
-
 // All threads of the block; P2 a power of two; a[] fully initialised.
 __device__ __forceinline__ void block_bitonic_sort(uint64_t* a, int P2) {
   for (int k = 2; k <= P2; k <<= 1)
@@ -177,7 +157,7 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
                    int* flagged, int* nflag, const float* rowthr = nullptr, const RecheckAudit* audit = nullptr,
                    int cand_by_row = 0, RecheckScratch* rs = nullptr);
 
-int choose_nseg_fp32(int nfit, int num_sms, int nref);
+int choose_nseg_fp32(int nfit, int num_sms, int nref, int Kp, bool same);
 
 // Candidates wanted per row before rounding: k+33, 2(k+1), and with the
 // tensor-core screen 4(k+1) up to 256 (its thresholds follow the (k+1)-th

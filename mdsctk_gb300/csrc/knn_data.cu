@@ -198,7 +198,7 @@ k_screen_dot(const float* __restrict__ Xf, const float* __restrict__ Xr, const f
     for (int r = warp; r < DT_TM; r += DT_THREADS / 32) {
       int n = scnt[r];
       if (n <= Kp) continue;
-      warp_bitonic_sort(pool + r * P2, n, P2, lane);
+      warp_sort_keys(pool + r * P2, n, lane);
       if (lane == 0) {
         scnt[r] = Kp;
         sthr[r] = mds_key_value(pool[r * P2 + Kp - 1]);
@@ -211,7 +211,7 @@ k_screen_dot(const float* __restrict__ Xf, const float* __restrict__ Xr, const f
     int lr = row0 + r;
     if (lr >= nrows) continue;
     int n = min(scnt[r], Kp);
-    warp_bitonic_sort(pool + r * P2, scnt[r], P2, lane);
+    warp_sort_keys(pool + r * P2, scnt[r], lane);
     uint64_t* dst = cand + ((int64_t)lr * nseg + seg) * Kp;
     for (int x = lane; x < n; x += 32) dst[x] = pool[r * P2 + x];
     if (lane == 0) cand_n[(int64_t)lr * nseg + seg] = n;

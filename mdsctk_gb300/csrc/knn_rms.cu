@@ -406,13 +406,20 @@ __global__ void __launch_bounds__(128) k_prep_out(const float* __restrict__ raw,
 // ---------------------------------------------------------------------------
 // 3. FP32 CUDA-core screen: tile of 32 fit x 64 ref frames per step, each
 //    thread owns 2 x 4 pairs (72 accumulators), atoms staged through shared
-//    memory in chunks of 32 with cp.async double buffering.
+//    memory in chunks of 32 with cp.async double buffering. Two blocks share
+//    an SM where K' <= 64 (the row records are in shared memory and the column
+//    records read where they are used, so that 128 registers do): the loads
+//    and the lists of one run under the multiply-adds of the other. Bound by
+//    those, then by the lists of the first tiles. Rows against themselves,
+//    screen alone: 1,000 x 60 atoms, k = 20: 0.116 ms (0.20 with one block and
+//    lists sorted in shared memory); 8,000 x 304, k = 100: 2.9 (4.9).
 // ---------------------------------------------------------------------------
 #define SC_TM 32
 #define SC_TN 64
 #define SC_KC 32
 #define SC_FS 98  // floats per frame per stage: 3*32 + 2 (bank spread)
 #define SC_THREADS 256
+#define SC_STATIC (4 * SC_TM * (MDS_REC + 1) + 1024)  // shared memory besides the dynamic part
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -434,7 +441,7 @@ __device__ __forceinline__ int sc_tile_order(int i, int t0, int t1, int td) {
   return (Rn > L) ? td + m + j : td - m - j;
 }
 
-__global__ void __launch_bounds__(SC_THREADS, 1)
+__global__ void __launch_bounds__(SC_THREADS, 2)
 k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
               const float* __restrict__ recf, const float* __restrict__ recr, int nrows,
               const int* __restrict__ rowlist, int Nr, int Ap, int nofit, float guard, int Kp,
@@ -462,10 +469,10 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* sfit = reinterpret_cast<float*>(smem_raw);                 // [2][32*98]
   float* sref = sfit + 2 * SC_TM * SC_FS;                           // [2][64*98]
-  float* scol = sref + 2 * SC_TN * SC_FS;                           // [64][16]
-  int* scnt = reinterpret_cast<int*>(scol + SC_TN * MDS_REC);       // [32]
+  int* scnt = reinterpret_cast<int*>(sref + 2 * SC_TN * SC_FS);     // [32]
   float* sthr = reinterpret_cast<float*>(scnt + SC_TM);             // [32]
   uint64_t* pool = reinterpret_cast<uint64_t*>(sthr + SC_TM);       // [32][P2]
+  __shared__ __align__(16) float srow[SC_TM * MDS_REC];
   __shared__ float sgthr[SC_TM];  // the rows' shared thresholds, read per tile
   // a row's pool holds its K' best plus one tile of new entries; its stride
   // is the power of two the sort works on
@@ -483,12 +490,11 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
   const bool dense = ex.dense != nullptr;
   const float INF = __int_as_float(0x7f800000);
 
-  int grow[2];
-  float rrec[2][MDS_REC];
-  for (int p = 0; p < 2; ++p) {
-    int lr = row0 + ty + 16 * p;
-    grow[p] = (lr < nrows) ? (rowlist ? rowlist[lr] : lr) : -1;
-    for (int i = 0; i < MDS_REC; ++i) rrec[p][i] = (grow[p] >= 0) ? recf[(int64_t)grow[p] * MDS_REC + i] : 0.f;
+  // the rows' records (first read after the barriers of a tile)
+  for (int e = tid; e < SC_TM * MDS_REC; e += SC_THREADS) {
+    const int lr = row0 + e / MDS_REC;
+    const int g = (lr < nrows) ? (rowlist ? rowlist[lr] : lr) : -1;
+    srow[e] = (g >= 0) ? recf[(int64_t)g * MDS_REC + e % MDS_REC] : 0.f;
   }
   if (tid < SC_TM) {
     scnt[tid] = 0;
@@ -549,12 +555,6 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
       if (__syncthreads_and(can)) continue;
     }
     if (ex.ntiles && !dense && tid == 0) atomicAdd(ex.ntiles, 1ull);
-    // column records of this tile
-    for (int e = tid; e < SC_TN * MDS_REC; e += SC_THREADS) {
-      int fr = e / MDS_REC, i = e % MDS_REC;
-      int j = tile * SC_TN + fr;
-      scol[e] = (j < Nr) ? recr[(int64_t)j * MDS_REC + i] : 0.f;
-    }
     float acc[2][4][9];
 #pragma unroll
     for (int p = 0; p < 2; ++p)
@@ -605,16 +605,22 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
     }
     // epilogue: lower bounds and top-K' insertion (or the dense bounds)
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      if (grow[p] < 0) continue;
-      int lr = ty + 16 * p;
+    for (int q = 0; q < 4; ++q) {
+      const int j = tile * SC_TN + tx + 16 * q;
+      if (j >= Nr) continue;
+      float cr[MDS_REC];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        int j = tile * SC_TN + tx + 16 * q;
-        if (j >= Nr) continue;
-        const float* cr = scol + (tx + 16 * q) * MDS_REC;
+      for (int i = 0; i < MDS_REC / 4; ++i) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(recr + (int64_t)j * MDS_REC) + i);
+        cr[4 * i] = t.x; cr[4 * i + 1] = t.y; cr[4 * i + 2] = t.z; cr[4 * i + 3] = t.w;
+      }
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int lr = ty + 16 * p;
+        if (row0 + lr >= nrows) continue;
+        const float* rr = srow + lr * MDS_REC;
         const float thr = dense ? INF : fminf(sthr[lr], sgthr[lr]);
-        float s = screen_shifted_f32(acc[p][q], rrec[p], cr, nofit != 0, guard * (rrec[p][15] + cr[15]), thr);
+        float s = screen_shifted_f32(acc[p][q], rr, cr, nofit != 0, guard * (rr[15] + cr[15]), thr);
         s = fmaxf(s, 0.0f);
         if (dense) {
           ex.dense[(int64_t)j * nrows + row0 + lr] = sqrtf(s);
@@ -631,7 +637,7 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
       const int n = scnt[r];
       const bool first = ex.nmax && sthr[r] == INF && n >= ex.k1;
       if (n <= Kp && !first) continue;
-      warp_bitonic_sort(pool + r * P2, n, P2, lane);
+      warp_sort_keys(pool + r * P2, n, lane);
       if (lane == 0) {
         float t = (n >= Kp) ? mds_key_value(pool[r * P2 + Kp - 1]) : INF;
         const int lr = row0 + r;
@@ -653,7 +659,7 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
     int lr = row0 + r;
     if (lr >= nrows) continue;
     int n = min(scnt[r], Kp);
-    warp_bitonic_sort(pool + r * P2, scnt[r], P2, lane);
+    warp_sort_keys(pool + r * P2, scnt[r], lane);
     uint64_t* dst = cand + ((int64_t)lr * nseg + seg) * Kp;
     for (int x = lane; x < n; x += 32) dst[x] = pool[r * P2 + x];
     if (lane == 0) cand_n[(int64_t)lr * nseg + seg] = n;
@@ -661,7 +667,7 @@ k_screen_fp32(const float* __restrict__ Af, const float* __restrict__ Ar,
 }
 
 size_t screen_fp32_smem(int Kp) {
-  return sizeof(float) * (2 * SC_TM * SC_FS + 2 * SC_TN * SC_FS + SC_TN * MDS_REC) +
+  return sizeof(float) * (2 * SC_TM * SC_FS + 2 * SC_TN * SC_FS) +
          sizeof(int) * SC_TM + sizeof(float) * SC_TM + sizeof(uint64_t) * SC_TM * next_pow2(Kp + SC_TN);
 }
 
@@ -1661,12 +1667,13 @@ int launch_prep(mds_ctx* ctx, const float* draw, int n, int natoms, int Ap, cons
   return MDS_OK;
 }
 
-int choose_nseg_fp32(int nfit, int num_sms, int nref) {
-  int nrt = (nfit + SC_TM - 1) / SC_TM, nct = (nref + SC_TN - 1) / SC_TN;
+// Segments of nct column tiles for nrt row tiles on `slots` blocks at a time:
+// the fewest (of at most smax) that leave the last wave nearly full.
+static int choose_nseg(int nrt, int slots, int nct, int smax) {
   int best = 1;
   double besteff = 0;
-  for (int s = 1; s <= 8 && s <= nct; ++s) {
-    double waves = (double)nrt * s / num_sms;
+  for (int s = 1; s <= smax && s <= nct; ++s) {
+    double waves = (double)nrt * s / slots;
     double eff = waves / std::ceil(waves);
     if (eff > besteff + 0.02) {
       besteff = eff;
@@ -1677,19 +1684,16 @@ int choose_nseg_fp32(int nfit, int num_sms, int nref) {
   return best;
 }
 
-static int choose_nseg(int nrowtiles, int num_sms, int ncoltiles) {
-  int best = 1;
-  double besteff = 0;
-  for (int s = 1; s <= 8 && s <= ncoltiles; ++s) {
-    double waves = (double)nrowtiles * s / num_sms;
-    double eff = waves / std::ceil(waves);
-    if (eff > besteff + 0.02) {
-      besteff = eff;
-      best = s;
-    }
-    if (eff >= 0.95) break;
-  }
-  return best;
+// Segments of the FP32 screen; two of its blocks share an SM where the lists of
+// K' allow it. The few row tiles of a small fit set take up to SC_SEGS
+// segments (100 fit frames against 12,000 of 304 atoms, K' = 96: 0.39 ms, 1.49
+// with eight); a set against itself takes up to eight, so that a segment's
+// later tiles can still be skipped by thresholds its first tiles set (2,000
+// frames of 60 atoms: 0.18 ms, 0.23 with up to 32).
+#define SC_SEGS 32
+int choose_nseg_fp32(int nfit, int num_sms, int nref, int Kp, bool same) {
+  const int per_sm = 2 * (screen_fp32_smem(Kp) + SC_STATIC) <= 228 * 1024 ? 2 : 1;
+  return choose_nseg((nfit + SC_TM - 1) / SC_TM, per_sm * num_sms, (nref + SC_TN - 1) / SC_TN, same ? 8 : SC_SEGS);
 }
 
 int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float* draw_fit,
@@ -1890,8 +1894,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
 
   // first pass
   int Kp = pl.kprime;
-  int ncoltiles = (nref + 63) / 64;
-  int nseg = choose_nseg((nfit + 31) / 32, ctx->num_sms, ncoltiles);
+  int nseg = choose_nseg_fp32(nfit, ctx->num_sms, nref, Kp, same);
   if (pl.prec != MDS_PREC_FP32) {
     nseg = tc_choose_nseg(ctx, pl, nfit);
     // A set screened against itself skips most tiles and its items differ
@@ -1944,7 +1947,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       KnnRmsPlan pp = pl;
       pp.nref = f_pv.nP;
       MDS_TRY(launch_screen_fp32(ctx, pp, Afp, f_pv.A.as<float>(), Rfp, f_pv.R.as<float>(), nfit, nullptr, 32,
-                                 choose_nseg_fp32(nfit, ctx->num_sms, f_pv.nP), nullptr, nullptr, &dx));
+                                 choose_nseg_fp32(nfit, ctx->num_sms, f_pv.nP, 32, false), nullptr, nullptr, &dx));
       MDS_TRY(f_tlo.alloc(ctx, sizeof(float) * (size_t)f_pv.nP * f_pv.nC));
       MDS_TRY(tc_skip_tlo(ctx, f_pv, f_lb.as<float>(), nfit, f_tlo.as<float>()));
       ex.pivlb = f_lb.as<float>();

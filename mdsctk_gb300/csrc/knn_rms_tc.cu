@@ -40,6 +40,7 @@
 #include "qcp.cuh"
 #include "tc_ptx.cuh"
 #include "tc_select.cuh"
+#include "warp_sort.cuh"
 
 // TC_FR_M / TC_FR_N (frames per row / column tile) come from knn_common.cuh
 #define TC_M 128
@@ -629,17 +630,7 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               warp_select_keep(src, n, Kp, reinterpret_cast<int*>(scratch), lane);
               n = Kp;
             }
-            int P2 = 32;
-            while (P2 < n) P2 <<= 1;
-            if (n <= 1) {
-            } else if (P2 <= TC_SCR) {
-              for (int x = lane; x < n; x += 32) scratch[x] = src[x];
-              __syncwarp();
-              warp_bitonic_sort(scratch, n, P2, lane);
-              for (int x = lane; x < n; x += 32) src[x] = scratch[x];
-            } else {
-              warp_bitonic_sort(src, n, TC_CAPG, lane);  // in place (global; __syncwarp orders it)
-            }
+            if (n > 1) warp_sort_keys(src, n, lane);
             if (lane == 0) cand_n[(int64_t)gr * nseg + seg] = n;
             __syncwarp();
           }

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "knn_common.cuh"
+#include "warp_sort.cuh"
 #include "overlap_tc.cuh"
 
 #define SP_THREADS 256
@@ -153,6 +154,7 @@ static size_t sparse_knn_smem(int k, int mode) {
 // call instead (see mds_knn_data_sparse).
 // ---------------------------------------------------------------------------
 #define BN_TM 32
+// (the pools fit in shared memory for up to WSORT_MAX keys per row)
 #define BN_TN 64
 #define BN_KW 32  // words per K-chunk
 #define BN_WS 36  // words per staged row (bank spread, 16-byte rows)
@@ -275,7 +277,7 @@ k_bin_knn(const unsigned* __restrict__ Bf, const int* __restrict__ cf, int nfit,
     for (int r = warp; r < BN_TM; r += SP_THREADS / 32) {
       const int n = scnt[r];
       if (n <= k1) continue;
-      warp_bitonic_sort(pool + r * P2, n, P2, lane);
+      warp_sort_keys(pool + r * P2, n, lane);
       if (lane == 0) {
         scnt[r] = k1;
         sthr[r] = mds_key_value(pool[r * P2 + k1 - 1]);
@@ -287,7 +289,7 @@ k_bin_knn(const unsigned* __restrict__ Bf, const int* __restrict__ cf, int nfit,
   for (int r = warp; r < BN_TM; r += SP_THREADS / 32) {
     const int row = row0 + r;
     if (row >= nfit) continue;
-    warp_bitonic_sort(pool + r * P2, scnt[r], P2, lane);
+    warp_sort_keys(pool + r * P2, scnt[r], lane);
     for (int x = lane; x < k; x += 32) {
       const uint64_t key = pool[r * P2 + x + 1];
       out_d[(int64_t)row * k + x] = sqrt((double)mds_key_value(key));

@@ -217,7 +217,7 @@ static int launch_batch(mds_server* S, Slot& sl, int bucket) {
                              sl.cand.as<uint64_t>(), sl.cand_n.as<int>(), sl.derr.as<int>(),
                              S->pv.nC > 0 ? &sk : nullptr, nullptr, sl.rowthr.as<float>(), S->nmax.as<float>()));
   } else {
-    nseg = std::min(choose_nseg_fp32(bucket, c->num_sms, S->n), S->nseg_max);
+    nseg = std::min(choose_nseg_fp32(bucket, c->num_sms, S->n, S->Kp, false), S->nseg_max);
     MDS_CUDA(c, cudaMemsetAsync(sl.derr.p, 0, sizeof(int), c->stream));
     MDS_TRY(launch_screen_fp32(c, pl, sl.A.as<float>(), S->A.as<float>(), sl.R.as<float>(), S->R.as<float>(), bucket,
                                nullptr, S->Kp, nseg, sl.cand.as<uint64_t>(), sl.cand_n.as<int>()));
