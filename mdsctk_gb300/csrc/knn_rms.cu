@@ -1696,6 +1696,19 @@ int choose_nseg_fp32(int nfit, int num_sms, int nref, int Kp, bool same) {
   return choose_nseg((nfit + SC_TM - 1) / SC_TM, per_sm * num_sms, (nref + SC_TN - 1) / SC_TN, same ? 8 : SC_SEGS);
 }
 
+// Counters and error words of one call, in one device block: one copy sets
+// them (with the masses) and one copy reads them, where seven fills and reads
+// of a word each cost a short call about 45 us of its 350.
+struct RmsStatus {
+  unsigned long long audit[4];  // the recheck's audit of the screen's bounds
+  unsigned long long ntiles;    // tiles the screen computed
+  int nflag;                    // flagged rows
+  int bad[2];                   // smallest frame with a non-finite coordinate (reference set, fit set)
+  // error words of the tensor-core launches: [0..1] the pivot pass, [2..3]
+  // the screen, then two per staged chunk's pivot pass
+  int tcerr[4 + 2 * MDS_MAX_CHUNKS];
+};
+
 int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float* draw_fit,
                 const float* hmass, double* dout_d, int* dout_i) {
   const int Ap = pl.Ap, natoms = pl.natoms;
@@ -1711,11 +1724,19 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   }
   if (!(M > 0)) return mds_fail(ctx, MDS_ERR_ARG, "total mass must be positive");
   for (int a = 0; a < natoms; ++a) swn[a] = (float)std::sqrt((double)hmass[a] / M);
-  DevBuf dmass, dswn;
-  MDS_TRY(dmass.alloc(ctx, sizeof(float) * natoms));
-  MDS_TRY(dswn.alloc(ctx, sizeof(float) * Ap));
-  MDS_CUDA(ctx, cudaMemcpyAsync(dmass.p, hmass, sizeof(float) * natoms, cudaMemcpyHostToDevice, s));
-  MDS_CUDA(ctx, cudaMemcpyAsync(dswn.p, swn.data(), sizeof(float) * Ap, cudaMemcpyHostToDevice, s));
+  RmsStatus hst{};
+  hst.bad[0] = hst.bad[1] = 0x7f7f7f7f;
+  const size_t st_bytes = (sizeof(RmsStatus) + 63) / 64 * 64;
+  DevBuf setup(ctx);  // status, weights, masses
+  std::vector<unsigned char> hsetup(st_bytes + sizeof(float) * (Ap + natoms));
+  std::memcpy(hsetup.data(), &hst, sizeof(hst));
+  std::memcpy(hsetup.data() + st_bytes, swn.data(), sizeof(float) * Ap);
+  std::memcpy(hsetup.data() + st_bytes + sizeof(float) * Ap, hmass, sizeof(float) * natoms);
+  MDS_TRY(setup.alloc(ctx, hsetup.size()));
+  MDS_CUDA(ctx, cudaMemcpyAsync(setup.p, hsetup.data(), hsetup.size(), cudaMemcpyHostToDevice, s));
+  RmsStatus* dst = setup.as<RmsStatus>();
+  const float* dswn = reinterpret_cast<const float*>(setup.as<unsigned char>() + st_bytes);
+  const float* dmass = dswn + Ap;
 
   const bool same = (draw_fit == nullptr);
   const int nref = pl.nref, nfit = same ? nref : pl.nfit;
@@ -1776,58 +1797,47 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   st.launches++;
   if (pl.href && !staged) MDS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->chunk_ev[0], 0));
   k_center<<<1, 128, 0, s>>>(staged ? praw.as<float>() + (size_t)spv.nP * 3 * natoms : draw_ref, 1, natoms, Ap,
-                             dmass.as<float>(), dswn.as<float>(), tm, Y0.as<float>(), E0.as<double>());
+                             dmass, dswn, tm, Y0.as<float>(), E0.as<double>());
   MDS_CUDA(ctx, cudaGetLastError());
 
   const int k = pl.k;
-  DevBuf flagged(ctx), nflag(ctx);
+  DevBuf flagged(ctx);
   MDS_TRY(flagged.alloc(ctx, sizeof(int) * (size_t)std::max(nfit, 1)));
-  MDS_TRY(nflag.alloc(ctx, sizeof(int)));
 
   // template and superposition
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
   std::vector<double> mu;
   double M0[9];
   MDS_TRY(build_template(ctx, Y0.as<float>(), Ap, natoms, pl.nofit != 0, mu, M0));
-  DevBuf dmu(ctx), dM0(ctx), Ar(ctx), Rr(ctx), Af(ctx), Rf(ctx);
-  std::vector<float> muf(mu.begin(), mu.end());
-  MDS_TRY(dmu.alloc(ctx, sizeof(float) * 3 * Ap));
-  MDS_TRY(dM0.alloc(ctx, sizeof(double) * 9));
-  MDS_CUDA(ctx, cudaMemcpyAsync(dmu.p, muf.data(), sizeof(float) * 3 * Ap, cudaMemcpyHostToDevice, s));
-  MDS_CUDA(ctx, cudaMemcpyAsync(dM0.p, M0, sizeof(double) * 9, cudaMemcpyHostToDevice, s));
+  DevBuf tmpl(ctx), Ar(ctx), Rr(ctx), Af(ctx), Rf(ctx);
+  std::vector<float> htmpl(3 * Ap + 18);  // mu, then M0 (3 Ap floats: a multiple of 8 bytes)
+  std::copy(mu.begin(), mu.end(), htmpl.begin());
+  std::memcpy(htmpl.data() + 3 * Ap, M0, sizeof(double) * 9);
+  MDS_TRY(tmpl.alloc(ctx, sizeof(float) * htmpl.size()));
+  MDS_CUDA(ctx, cudaMemcpyAsync(tmpl.p, htmpl.data(), sizeof(float) * htmpl.size(), cudaMemcpyHostToDevice, s));
+  const float* dmu = tmpl.as<float>();
+  const double* dM0 = reinterpret_cast<const double*>(dmu + 3 * Ap);
   MDS_TRY(Ar.alloc(ctx, sizeof(float) * 3 * Ap * (size_t)nref));
   MDS_TRY(Rr.alloc(ctx, sizeof(float) * MDS_REC * (size_t)nref));
   DevBuf Ur(ctx);  // the reference frames' U = sum a mu^T as double-float pairs (recheck)
   MDS_TRY(Ur.alloc(ctx, sizeof(float) * MDS_USTRIDE * (size_t)nref));
-  // frames with a non-finite coordinate (reference set, fit set): smallest
-  // index, checked at the call's first synchronisation after the screen
-  DevBuf badf(ctx);
-  MDS_TRY(badf.alloc(ctx, 2 * sizeof(int)));
-  MDS_CUDA(ctx, cudaMemsetAsync(badf.p, 0x7f, 2 * sizeof(int), s));
   // superposition, one upload chunk at a time
   auto prep_chunks = [&](const float* draw, bool host, const std::vector<int>& cb, int nc, int ev0, float* A,
                          float* R, float* U, int* bad) -> int {
     for (int c = 0; c < nc; ++c) {
       if (host) MDS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->chunk_ev[ev0 + c], 0));
       const int f0 = cb[c], nf = cb[c + 1] - cb[c];
-      MDS_TRY(launch_prep(ctx, draw + (size_t)f0 * 3 * natoms, nf, natoms, Ap, dmass.as<float>(), dswn.as<float>(),
-                          tm, dmu.as<float>(), dM0.as<double>(), pl.nofit, A + (size_t)f0 * 3 * Ap,
+      MDS_TRY(launch_prep(ctx, draw + (size_t)f0 * 3 * natoms, nf, natoms, Ap, dmass, dswn,
+                          tm, dmu, dM0, pl.nofit, A + (size_t)f0 * 3 * Ap,
                           R + (size_t)f0 * MDS_REC, U ? U + (size_t)f0 * MDS_USTRIDE : nullptr, bad, f0));
     }
     return MDS_OK;
   };
-  // error words of the tensor-core launches, read at the call's
-  // synchronisation after the recheck: [0..1] the pivot pass, [2..3] the
-  // screen, then two per staged chunk's pivot pass
-  DevBuf tcerr(ctx);
-  const int nerr = 4 + 2 * MDS_MAX_CHUNKS;
-  MDS_TRY(tcerr.alloc(ctx, nerr * sizeof(int)));
-  MDS_CUDA(ctx, cudaMemsetAsync(tcerr.p, 0, nerr * sizeof(int), s));
   TcOperands tcr, tcf;
   DevBuf slb(ctx);  // staged: lower bounds from every frame to every pivot [nP][n]
   if (staged) {
-    MDS_TRY(launch_prep(ctx, praw.as<float>(), spv.nP, natoms, Ap, dmass.as<float>(), dswn.as<float>(), tm,
-                        dmu.as<float>(), dM0.as<double>(), pl.nofit, spv.A.as<float>(), spv.R.as<float>(), nullptr,
+    MDS_TRY(launch_prep(ctx, praw.as<float>(), spv.nP, natoms, Ap, dmass, dswn, tm,
+                        dmu, dM0, pl.nofit, spv.A.as<float>(), spv.R.as<float>(), nullptr,
                         nullptr, 0));
     MDS_TRY(tc_pivots_operand(ctx, pl, spv));
     MDS_TRY(tc_alloc(ctx, pl, nref, tcr, 1));
@@ -1836,19 +1846,19 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     for (int c = 0; c < nc_ref; ++c) {
       MDS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->chunk_ev[c], 0));
       const int f0 = cb_ref[c], f1 = cb_ref[c + 1];
-      MDS_TRY(launch_prep(ctx, draw_ref + (size_t)f0 * 3 * natoms, f1 - f0, natoms, Ap, dmass.as<float>(),
-                          dswn.as<float>(), tm, dmu.as<float>(), dM0.as<double>(), pl.nofit,
+      MDS_TRY(launch_prep(ctx, draw_ref + (size_t)f0 * 3 * natoms, f1 - f0, natoms, Ap, dmass,
+                          dswn, tm, dmu, dM0, pl.nofit,
                           Ar.as<float>() + (size_t)f0 * 3 * Ap, Rr.as<float>() + (size_t)f0 * MDS_REC,
-                          pl.nofit ? nullptr : Ur.as<float>() + (size_t)f0 * MDS_USTRIDE, badf.as<int>(), f0));
+                          pl.nofit ? nullptr : Ur.as<float>() + (size_t)f0 * MDS_USTRIDE, dst->bad, f0));
       MDS_TRY(tc_prepare_range(ctx, pl, Ar.as<float>(), nref, tcr, 1, f0, f1));
       MDS_TRY(tc_prepare_range(ctx, pl, Ar.as<float>(), nref, tcr, 0, f0, f1));
       MDS_TRY(tc_pivots_radii(ctx, pl, Ar.as<float>(), spv, f0, f1));
-      MDS_TRY(tc_skip_bounds(ctx, pl, tcr, Rr.as<float>(), nref, spv, slb.as<float>(), tcerr.as<int>() + 4 + 2 * c,
+      MDS_TRY(tc_skip_bounds(ctx, pl, tcr, Rr.as<float>(), nref, spv, slb.as<float>(), dst->tcerr + 4 + 2 * c,
                              f0, f1));
     }
   } else {
     MDS_TRY(prep_chunks(draw_ref, pl.href != nullptr, cb_ref, nc_ref, 0, Ar.as<float>(), Rr.as<float>(),
-                        pl.nofit ? nullptr : Ur.as<float>(), badf.as<int>()));
+                        pl.nofit ? nullptr : Ur.as<float>(), dst->bad));
   }
   const float* Afp = Ar.as<float>();
   const float* Rfp = Rr.as<float>();
@@ -1856,7 +1866,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     MDS_TRY(Af.alloc(ctx, sizeof(float) * 3 * Ap * (size_t)nfit));
     MDS_TRY(Rf.alloc(ctx, sizeof(float) * MDS_REC * (size_t)nfit));
     MDS_TRY(prep_chunks(draw_fit, pl.hfit != nullptr, cb_fit, nc_fit, MDS_MAX_CHUNKS, Af.as<float>(),
-                        Rf.as<float>(), nullptr, badf.as<int>() + 1));
+                        Rf.as<float>(), nullptr, &dst->bad[1]));
     Afp = Af.as<float>();
     Rfp = Rf.as<float>();
   }
@@ -1870,10 +1880,10 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   }
   if (pl.full) {
     MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    MDS_TRY(launch_full_rows(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), nfit, dout_d, dout_i));
+    MDS_TRY(launch_full_rows(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, dout_d, dout_i));
     MDS_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
     int hbad[2] = {0, 0};
-    MDS_CUDA(ctx, cudaMemcpyAsync(hbad, badf.p, sizeof(hbad), cudaMemcpyDeviceToHost, s));
+    MDS_CUDA(ctx, cudaMemcpyAsync(hbad, dst->bad, sizeof(hbad), cudaMemcpyDeviceToHost, s));
     MDS_CUDA(ctx, cudaEventSynchronize(ctx->ev[2]));
     MDS_CUDA(ctx, cudaStreamSynchronize(s));
     float ms = 0;
@@ -1910,11 +1920,8 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   const int segstride = (pl.prec == MDS_PREC_FP32) ? Kp : tc_seg_stride();
   MDS_TRY(cand.alloc(ctx, sizeof(uint64_t) * (size_t)nfit * nseg * segstride));
   MDS_TRY(cand_n.alloc(ctx, sizeof(int) * (size_t)nfit * nseg));
-  MDS_CUDA(ctx, cudaMemsetAsync(nflag.p, 0, sizeof(int), s));
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
   DevBuf rowthr(ctx), nmax(ctx);  // shared row thresholds of the tensor-core screen, max |a_j|^2
-  DevBuf ntiles(ctx);             // tiles the tensor-core screen computed
-  unsigned long long ht = 0;      // (read back after the recheck)
   long long dense_pairs = 0;
   DevBuf f_lb(ctx), f_tlo(ctx);
   TcPivots f_pv;
@@ -1929,12 +1936,10 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       MDS_CUDA(ctx, cudaMemsetAsync(rowthr.p, 0x7f, sizeof(float) * std::max(nfit, 1), s));
       MDS_TRY(nmax.alloc(ctx, sizeof(float)));
       MDS_TRY(tc_rec_nmax(ctx, Rr.as<float>(), nref, nmax.as<float>()));
-      MDS_TRY(ntiles.alloc(ctx, sizeof(unsigned long long)));
-      MDS_CUDA(ctx, cudaMemsetAsync(ntiles.p, 0, sizeof(unsigned long long), s));
       ex.rowthr = rowthr.as<float>();
       ex.nmax = nmax.as<float>();
       ex.k1 = k + 1;
-      ex.ntiles = ntiles.as<unsigned long long>();
+      ex.ntiles = &dst->ntiles;
     }
     ex.diag = same ? 1 : 0;
     const bool skipping = !keys_only && !pl.noskip && same && (nref + TC_FR_N - 1) / TC_FR_N >= 4;
@@ -1974,7 +1979,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       if (!staged) {
         MDS_TRY(tc_skip_pivots(ctx, pl, Ar.as<float>(), Rr.as<float>(), pv, same));
         MDS_TRY(lb.alloc(ctx, sizeof(float) * (size_t)pv.nP * nfit));
-        MDS_TRY(tc_skip_bounds(ctx, pl, same ? tcr : tcf, Rfp, nfit, pv, lb.as<float>(), tcerr.as<int>()));
+        MDS_TRY(tc_skip_bounds(ctx, pl, same ? tcr : tcf, Rfp, nfit, pv, lb.as<float>(), dst->tcerr));
       }
       sk.pivlb = lb.as<float>();
       sk.prad = pv.rad.as<float>();
@@ -1998,13 +2003,11 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     MDS_TRY(rowthr.alloc(ctx, sizeof(float) * std::max(nfit, 1)));
     MDS_TRY(nmax.alloc(ctx, sizeof(float)));
     MDS_TRY(tc_rec_nmax(ctx, Rr.as<float>(), nref, nmax.as<float>()));
-    MDS_TRY(ntiles.alloc(ctx, sizeof(unsigned long long)));
-    MDS_CUDA(ctx, cudaMemsetAsync(ntiles.p, 0, sizeof(unsigned long long), s));
     MDS_TRY(launch_screen_tc(ctx, pl, same ? tcr : tcf, tcr, Rfp, Rr.as<float>(), nfit, Kp, nseg,
-                             cand.as<uint64_t>(), cand_n.as<int>(), pl.screen_keys ? nullptr : tcerr.as<int>() + 2,
+                             cand.as<uint64_t>(), cand_n.as<int>(), pl.screen_keys ? nullptr : dst->tcerr + 2,
                              skipping ? &sk : nullptr, nullptr,
                              rowthr.as<float>(), pl.screen_keys ? nullptr : nmax.as<float>(),
-                             ntiles.as<unsigned long long>()));
+                             &dst->ntiles));
     st.screen_launches = skipping ? 2 : 1;
     // (staged: the pivot pass ran with the chunks, its time in the prep stage)
     dense_pairs = skipping ? (long long)pv.nP * nfit : 0;
@@ -2022,29 +2025,24 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     return MDS_OK;
   }
   // the recheck audits the screen's bounds on the pairs it rechecks
-  DevBuf audit_c(ctx);
-  MDS_TRY(audit_c.alloc(ctx, 4 * sizeof(unsigned long long)));
-  MDS_CUDA(ctx, cudaMemsetAsync(audit_c.p, 0, 4 * sizeof(unsigned long long), s));
   RecheckAudit audit;
   audit.recf = Rfp;
   audit.recr = Rr.as<float>();
   audit.guard = (pl.prec == MDS_PREC_FP32) ? pl.guard_fp32 : pl.guard_tc;
-  audit.counters = audit_c.as<unsigned long long>();
+  audit.counters = dst->audit;
   RecheckScratch rs;
   MDS_TRY(recheck_scratch(ctx, nfit, rs));
-  MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), nfit, nullptr, 0,
+  MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, nullptr, 0,
                          cand.as<uint64_t>(), cand_n.as<int>(), nseg, segstride, Kp, k, dout_d, dout_i,
-                         flagged.as<int>(), nflag.as<int>(), rowthr.p ? rowthr.as<float>() : nullptr, &audit, 0,
+                         flagged.as<int>(), &dst->nflag, rowthr.p ? rowthr.as<float>() : nullptr, &audit, 0,
                          &rs));
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
-  int hflag = 0, hbad[2] = {0, 0}, herr[4 + 2 * MDS_MAX_CHUNKS] = {};
-  unsigned long long hc[4] = {0, 0, 0, 0};
-  MDS_CUDA(ctx, cudaMemcpyAsync(herr, tcerr.p, sizeof(herr), cudaMemcpyDeviceToHost, s));
-  if (ntiles.p) MDS_CUDA(ctx, cudaMemcpyAsync(&ht, ntiles.p, sizeof(ht), cudaMemcpyDeviceToHost, s));
-  MDS_CUDA(ctx, cudaMemcpyAsync(&hflag, nflag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  MDS_CUDA(ctx, cudaMemcpyAsync(hc, audit_c.p, sizeof(hc), cudaMemcpyDeviceToHost, s));
-  MDS_CUDA(ctx, cudaMemcpyAsync(hbad, badf.p, sizeof(hbad), cudaMemcpyDeviceToHost, s));
+  MDS_CUDA(ctx, cudaMemcpyAsync(&hst, dst, sizeof(hst), cudaMemcpyDeviceToHost, s));
   MDS_CUDA(ctx, cudaStreamSynchronize(s));
+  int* herr = hst.tcerr;
+  const int* hbad = hst.bad;
+  const unsigned long long* hc = hst.audit;
+  int hflag = hst.nflag;
   for (int c = 0; c < MDS_MAX_CHUNKS; ++c)
     if (herr[4 + 2 * c] && !herr[0]) herr[0] = herr[4 + 2 * c];
   if (herr[0] || herr[2])
@@ -2076,8 +2074,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   st.kprime = Kp;
   st.rows_flagged = hflag;
   st.passes = 1;
-  // (ht landed with the sync above)
-  st.screen_pairs = (long long)ht * (pl.prec == MDS_PREC_FP32 ? 32 * 64 : TC_FR_M * TC_FR_N) + dense_pairs;
+  st.screen_pairs = (long long)hst.ntiles * (pl.prec == MDS_PREC_FP32 ? 32 * 64 : TC_FR_M * TC_FR_N) + dense_pairs;
 
   // re-screen flagged rows with more candidates (FP32 screen), then exact rows
   while (hflag > 0) {
@@ -2087,13 +2084,13 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     std::sort(hrows.begin(), hrows.end());
     MDS_TRY(rows.alloc(ctx, sizeof(int) * hflag));
     MDS_CUDA(ctx, cudaMemcpyAsync(rows.p, hrows.data(), sizeof(int) * hflag, cudaMemcpyHostToDevice, s));
-    MDS_CUDA(ctx, cudaMemsetAsync(nflag.p, 0, sizeof(int), s));
+    MDS_CUDA(ctx, cudaMemsetAsync(&dst->nflag, 0, sizeof(int), s));
     Kp = std::min(Kp * 4, 448);
     st.passes++;
     if (Kp >= nref || st.passes > 3) {
       // exact rows: every reference is a candidate
-      MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), hflag, rows.as<int>(), 1, nullptr,
-                             nullptr, 1, 1, 1, k, dout_d, dout_i, flagged.as<int>(), nflag.as<int>()));
+      MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), hflag, rows.as<int>(), 1, nullptr,
+                             nullptr, 1, 1, 1, k, dout_d, dout_i, flagged.as<int>(), &dst->nflag));
       MDS_CUDA(ctx, cudaStreamSynchronize(s));
       break;
     }
@@ -2106,10 +2103,10 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
                                nseg2, cand.as<uint64_t>(), cand_n.as<int>()));
     RecheckAudit audit2 = audit;  // the re-screen's bounds carry the FP32 guard
     audit2.guard = pl.guard_fp32;
-    MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu.as<float>(), Ur.as<float>(), hflag, rows.as<int>(), 0,
+    MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), hflag, rows.as<int>(), 0,
                            cand.as<uint64_t>(), cand_n.as<int>(), nseg2, Kp, Kp, k, dout_d, dout_i,
-                           flagged.as<int>(), nflag.as<int>(), nullptr, &audit2));
-    MDS_CUDA(ctx, cudaMemcpyAsync(&hflag, nflag.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+                           flagged.as<int>(), &dst->nflag, nullptr, &audit2));
+    MDS_CUDA(ctx, cudaMemcpyAsync(&hflag, &dst->nflag, sizeof(int), cudaMemcpyDeviceToHost, s));
     MDS_CUDA(ctx, cudaStreamSynchronize(s));
   }
   return MDS_OK;
