@@ -25,8 +25,7 @@ void mds_trim_cache(mds_ctx* ctx, size_t keep) {
   }
 }
 
-int mds_upload_chunked(mds_ctx* ctx, void* dst, const void* src, int n, size_t frame_bytes, int ev0,
-                       std::vector<int>& bounds, int* nchunks, int align) {
+int mds_upload_plan(mds_ctx* ctx, int n, size_t frame_bytes, std::vector<int>& bounds, int* nchunks, int align) {
   if (!ctx->order_ev) {
     for (auto& cs : ctx->copy_stream) MDS_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     for (auto& e : ctx->chunk_ev) MDS_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -44,6 +43,12 @@ int mds_upload_chunked(mds_ctx* ctx, void* dst, const void* src, int n, size_t f
   // the destination may be a cached block last used by work on ctx->stream
   MDS_CUDA(ctx, cudaEventRecord(ctx->order_ev, ctx->stream));
   for (auto cs : ctx->copy_stream) MDS_CUDA(ctx, cudaStreamWaitEvent(cs, ctx->order_ev, 0));
+  *nchunks = c;
+  return MDS_OK;
+}
+
+int mds_upload_chunk(mds_ctx* ctx, void* dst, const void* src, size_t frame_bytes, int ev0,
+                     const std::vector<int>& bounds, int c) {
   // All chunks on one copy stream, so they land in order. The host link
   // carries ~205 GB/s whichever way the copies are issued (one or several
   // streams, or a kernel reading the mapped host memory); with the chunks
@@ -51,13 +56,10 @@ int mds_upload_chunked(mds_ctx* ctx, void* dst, const void* src, int n, size_t f
   // one stream before any of the other's, and the first chunk landed last
   // but one.
   cudaStream_t cs = ctx->copy_stream[0];
-  for (int i = 0; i < c; ++i) {
-    const size_t off = frame_bytes * (size_t)bounds[i], bytes = frame_bytes * (size_t)(bounds[i + 1] - bounds[i]);
-    MDS_CUDA(ctx, cudaMemcpyAsync(static_cast<char*>(dst) + off, static_cast<const char*>(src) + off, bytes,
-                                  cudaMemcpyHostToDevice, cs));
-    MDS_CUDA(ctx, cudaEventRecord(ctx->chunk_ev[ev0 + i], cs));
-  }
-  *nchunks = c;
+  const size_t off = frame_bytes * (size_t)bounds[c], bytes = frame_bytes * (size_t)(bounds[c + 1] - bounds[c]);
+  MDS_CUDA(ctx, cudaMemcpyAsync(static_cast<char*>(dst) + off, static_cast<const char*>(src) + off, bytes,
+                                cudaMemcpyHostToDevice, cs));
+  MDS_CUDA(ctx, cudaEventRecord(ctx->chunk_ev[ev0 + c], cs));
   return MDS_OK;
 }
 

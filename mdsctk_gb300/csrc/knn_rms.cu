@@ -328,7 +328,9 @@ __global__ void __launch_bounds__(128) k_prep_sums(const float* __restrict__ raw
 }
 
 // The rotation of every frame (one thread per frame, FP64 QCP): record
-// entries 3..12 (|y|^2, y mu^T) -> 3..11 (R, row-major).
+// entries 3..12 (|y|^2, y mu^T) -> 3..11 (R, row-major). Bound by the FP64
+// pipe (1.6 multiply-adds per cycle and SM), so a warp is a block of its own:
+// 2,501 frames on all SMs RO_B us, on the 20 that blocks of 128 filled RO_A.
 __global__ void k_prep_rot(int n, const double* __restrict__ M0, float* __restrict__ rec) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= n) return;
@@ -1661,7 +1663,7 @@ int launch_prep(mds_ctx* ctx, const float* draw, int n, int natoms, int Ap, cons
   if (n <= 0) return MDS_OK;
   ctx->stats.launches += nofit ? 2 : 3;
   k_prep_sums<<<n, 128, 0, ctx->stream>>>(draw, n, natoms, Ap, dmass, dswn, tm, dmu, nofit, R, bad, fbase);
-  if (!nofit) k_prep_rot<<<(n + 127) / 128, 128, 0, ctx->stream>>>(n, dM0, R);
+  if (!nofit) k_prep_rot<<<(n + 31) / 32, 32, 0, ctx->stream>>>(n, dM0, R);
   k_prep_out<<<n, 128, 0, ctx->stream>>>(draw, n, natoms, Ap, dswn, dmu, dM0, nofit, A, R, Uhl);
   MDS_CUDA(ctx, cudaGetLastError());
   return MDS_OK;
@@ -1772,9 +1774,15 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   TcPivots spv;
   DevBuf praw(ctx), gidx(ctx);
   if (staged) MDS_TRY(tc_pivots_begin(ctx, pl, spv, true));
-  if (pl.href)
-    MDS_TRY(mds_upload_chunked(ctx, const_cast<float*>(draw_ref), pl.href, nref, frame_bytes, 0, cb_ref, &nc_ref,
-                               staged ? TC_FR_N : 1));
+  auto upload = [&](const float* dst, const float* src, int ev0, const std::vector<int>& cb, int c) -> int {
+    return mds_upload_chunk(ctx, const_cast<float*>(dst), src, frame_bytes, ev0, cb, c);
+  };
+  if (pl.href) {
+    // the first chunk now (the template is made from its first frame), all of
+    // them when staged; else each when the one before is being superposed
+    MDS_TRY(mds_upload_plan(ctx, nref, frame_bytes, cb_ref, &nc_ref, staged ? TC_FR_N : 1));
+    for (int c = 0; c < (staged ? nc_ref : 1); ++c) MDS_TRY(upload(draw_ref, pl.href, 0, cb_ref, c));
+  }
   if (staged) {
     // the pivots' frames, and frame 0 (the template's) after them, gathered
     // from the host frames while the chunks are in flight
@@ -1786,9 +1794,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     k_gather_raw<<<(int)gi.size(), 128, 0, s>>>(hmap, gidx.as<int>(), (int)gi.size(), 3 * natoms, praw.as<float>());
     MDS_CUDA(ctx, cudaGetLastError());
   }
-  if (pl.hfit && !same)
-    MDS_TRY(mds_upload_chunked(ctx, const_cast<float*>(draw_fit), pl.hfit, nfit, frame_bytes, MDS_MAX_CHUNKS,
-                               cb_fit, &nc_fit));
+  if (pl.hfit && !same) MDS_TRY(mds_upload_plan(ctx, nfit, frame_bytes, cb_fit, &nc_fit));
   // the first reference frame, centred, defines the template
   DevBuf Y0(ctx), E0(ctx);
   MDS_TRY(Y0.alloc(ctx, sizeof(float) * 3 * Ap));
@@ -1821,11 +1827,16 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   MDS_TRY(Rr.alloc(ctx, sizeof(float) * MDS_REC * (size_t)nref));
   DevBuf Ur(ctx);  // the reference frames' U = sum a mu^T as double-float pairs (recheck)
   MDS_TRY(Ur.alloc(ctx, sizeof(float) * MDS_USTRIDE * (size_t)nref));
-  // superposition, one upload chunk at a time
-  auto prep_chunks = [&](const float* draw, bool host, const std::vector<int>& cb, int nc, int ev0, float* A,
+  // Superposition, one upload chunk at a time, each chunk uploaded while the
+  // one before it is superposed (2,047 frames of 304 atoms against 20,011 from
+  // pageable memory: UP_B us a call, UP_A with all copies issued first).
+  auto prep_chunks = [&](const float* draw, const float* host, const std::vector<int>& cb, int nc, int ev0, float* A,
                          float* R, float* U, int* bad) -> int {
     for (int c = 0; c < nc; ++c) {
-      if (host) MDS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->chunk_ev[ev0 + c], 0));
+      if (host) {
+        if (c > 0 || ev0 > 0) MDS_TRY(upload(draw, host, ev0, cb, c));
+        MDS_CUDA(ctx, cudaStreamWaitEvent(s, ctx->chunk_ev[ev0 + c], 0));
+      }
       const int f0 = cb[c], nf = cb[c + 1] - cb[c];
       MDS_TRY(launch_prep(ctx, draw + (size_t)f0 * 3 * natoms, nf, natoms, Ap, dmass, dswn,
                           tm, dmu, dM0, pl.nofit, A + (size_t)f0 * 3 * Ap,
@@ -1857,7 +1868,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
                              f0, f1));
     }
   } else {
-    MDS_TRY(prep_chunks(draw_ref, pl.href != nullptr, cb_ref, nc_ref, 0, Ar.as<float>(), Rr.as<float>(),
+    MDS_TRY(prep_chunks(draw_ref, pl.href, cb_ref, nc_ref, 0, Ar.as<float>(), Rr.as<float>(),
                         pl.nofit ? nullptr : Ur.as<float>(), dst->bad));
   }
   const float* Afp = Ar.as<float>();
@@ -1865,7 +1876,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   if (!same) {
     MDS_TRY(Af.alloc(ctx, sizeof(float) * 3 * Ap * (size_t)nfit));
     MDS_TRY(Rf.alloc(ctx, sizeof(float) * MDS_REC * (size_t)nfit));
-    MDS_TRY(prep_chunks(draw_fit, pl.hfit != nullptr, cb_fit, nc_fit, MDS_MAX_CHUNKS, Af.as<float>(),
+    MDS_TRY(prep_chunks(draw_fit, pl.hfit, cb_fit, nc_fit, MDS_MAX_CHUNKS, Af.as<float>(),
                         Rf.as<float>(), nullptr, &dst->bad[1]));
     Afp = Af.as<float>();
     Rfp = Rf.as<float>();

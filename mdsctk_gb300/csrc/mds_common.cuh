@@ -45,16 +45,18 @@ struct mds_ctx {
 // Record an error message on the context and return `code`.
 int mds_fail(mds_ctx* ctx, int code, const char* fmt, ...);
 
-// Upload n frames of `frame_bytes` each from host memory to dst in up to
-// MDS_MAX_CHUNKS chunks, in order on the context's first copy stream and
-// ordered after the work already queued on ctx->stream. Chunk c covers
-// frames [bounds[c], bounds[c+1]) and completes event ctx->chunk_ev[ev0 + c];
-// the consumer waits on that event before reading the chunk. From pageable
-// host memory the copies are correct but do not overlap. Returns the number
-// of chunks through *nchunks. Inner chunk bounds are multiples of `align`
-// frames.
-int mds_upload_chunked(mds_ctx* ctx, void* dst, const void* src, int n, size_t frame_bytes, int ev0,
-                       std::vector<int>& bounds, int* nchunks, int align = 1);
+// Upload of n frames of `frame_bytes` each from host memory in up to
+// MDS_MAX_CHUNKS chunks. The plan splits them: chunk c covers frames
+// [bounds[c], bounds[c+1]), inner bounds are multiples of `align` frames, the
+// number of chunks is returned through *nchunks; the copies are ordered after
+// the work queued on ctx->stream by now. mds_upload_chunk issues the copy of
+// chunk c to dst on the context's first copy stream; it completes event
+// ctx->chunk_ev[ev0 + c], which the consumer waits on before it reads the
+// chunk. A copy from pageable memory holds the calling thread until it is
+// done, so the work on a chunk is launched before the next chunk is issued.
+int mds_upload_plan(mds_ctx* ctx, int n, size_t frame_bytes, std::vector<int>& bounds, int* nchunks, int align = 1);
+int mds_upload_chunk(mds_ctx* ctx, void* dst, const void* src, size_t frame_bytes, int ev0,
+                     const std::vector<int>& bounds, int c);
 
 // Free cached device blocks until at most `keep` bytes remain cached
 // (synchronises the context's stream first).
