@@ -107,6 +107,8 @@ int build_template(mds_ctx* ctx, const float* dY0, int Ap, int natoms, bool nofi
 // skipping data (pivots, radii, row-tile bounds) is laid out on these tiles.
 #define TC_FR_M 40
 #define TC_FR_N 80
+// Column segments of a screen at most: the staged recheck merges as many lists.
+#define TC_MAX_SEGS 32
 
 // Optional parts of the FP32 screen (k_screen_fp32, knn_rms.cu): tile
 // skipping with the tensor-core screen's row-tile pivots (pivlb [nR][nfit]

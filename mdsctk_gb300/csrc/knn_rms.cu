@@ -1687,15 +1687,14 @@ static int choose_nseg(int nrt, int slots, int nct, int smax) {
 }
 
 // Segments of the FP32 screen; two of its blocks share an SM where the lists of
-// K' allow it. The few row tiles of a small fit set take up to SC_SEGS
+// K' allow it. The few row tiles of a small fit set take up to 32
 // segments (100 fit frames against 12,000 of 304 atoms, K' = 96: 0.39 ms, 1.49
 // with eight); a set against itself takes up to eight, so that a segment's
 // later tiles can still be skipped by thresholds its first tiles set (2,000
 // frames of 60 atoms: 0.18 ms, 0.23 with up to 32).
-#define SC_SEGS 32
 int choose_nseg_fp32(int nfit, int num_sms, int nref, int Kp, bool same) {
   const int per_sm = 2 * (screen_fp32_smem(Kp) + SC_STATIC) <= 228 * 1024 ? 2 : 1;
-  return choose_nseg((nfit + SC_TM - 1) / SC_TM, per_sm * num_sms, (nref + SC_TN - 1) / SC_TN, same ? 8 : SC_SEGS);
+  return choose_nseg((nfit + SC_TM - 1) / SC_TM, per_sm * num_sms, (nref + SC_TN - 1) / SC_TN, same ? 8 : TC_MAX_SEGS);
 }
 
 // Counters and error words of one call, in one device block: one copy sets
@@ -1929,6 +1928,8 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   if (pl.screen_keys) nseg = 1;
   DevBuf cand(ctx), cand_n(ctx), rows(ctx);
   const int segstride = (pl.prec == MDS_PREC_FP32) ? Kp : tc_seg_stride();
+  if (nseg > 8 && cand.alloc(ctx, sizeof(uint64_t) * (size_t)nfit * nseg * segstride) != MDS_OK)
+    nseg = 8;  // (a small HBM budget)
   MDS_TRY(cand.alloc(ctx, sizeof(uint64_t) * (size_t)nfit * nseg * segstride));
   MDS_TRY(cand_n.alloc(ctx, sizeof(int) * (size_t)nfit * nseg));
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));

@@ -202,9 +202,11 @@ static int launch_batch(mds_server* S, Slot& sl, int bucket) {
   MDS_CUDA(c, cudaMemsetAsync(sl.audit.p, 0, 4 * sizeof(unsigned long long), c->stream));
   MDS_TRY(launch_prep(c, sl.raw.as<float>(), bucket, S->natoms, S->Ap, S->dmass.as<float>(), S->dswn.as<float>(),
                       S->tm, S->dmu.as<float>(), S->dM0.as<double>(), pl.nofit, sl.A.as<float>(), sl.R.as<float>()));
+  // segments: the lists of a batch smaller than the slot may use its whole buffer
+  const int segs = std::min<int>(TC_MAX_SEGS, (int64_t)sl.cap * S->nseg_max / bucket);
   int nseg;
   if (S->prec != MDS_PREC_FP32) {
-    nseg = std::min(tc_choose_nseg(c, pl, bucket), S->nseg_max);
+    nseg = std::min(tc_choose_nseg(c, pl, bucket), segs);
     MDS_TRY(tc_prepare(c, pl, sl.A.as<float>(), bucket, sl.tcq, 0));
     TcSkip sk;
     if (S->pv.nC > 0) {  // tile skipping: bounds of the batch's frames to the landmark pivots
@@ -217,7 +219,7 @@ static int launch_batch(mds_server* S, Slot& sl, int bucket) {
                              sl.cand.as<uint64_t>(), sl.cand_n.as<int>(), sl.derr.as<int>(),
                              S->pv.nC > 0 ? &sk : nullptr, nullptr, sl.rowthr.as<float>(), S->nmax.as<float>()));
   } else {
-    nseg = std::min(choose_nseg_fp32(bucket, c->num_sms, S->n, S->Kp, false), S->nseg_max);
+    nseg = std::min(choose_nseg_fp32(bucket, c->num_sms, S->n, S->Kp, false), segs);
     MDS_CUDA(c, cudaMemsetAsync(sl.derr.p, 0, sizeof(int), c->stream));
     MDS_TRY(launch_screen_fp32(c, pl, sl.A.as<float>(), S->A.as<float>(), sl.R.as<float>(), S->R.as<float>(), bucket,
                                nullptr, S->Kp, nseg, sl.cand.as<uint64_t>(), sl.cand_n.as<int>()));
