@@ -204,6 +204,7 @@ int vec_unsort(mds_ctx* ctx, const float* src, const int* perm, int n, float* ds
 // bounds of RMSD from every fit frame to the pivot of every column tile
 // (pivlb [ncoltiles][nfit]) and the tiles' radii (prad [ncoltiles]).
 struct TcSkip {
+  const int* home = nullptr;  // nearest column tile per row tile (a separate fit set)
   const float* pivlb = nullptr;
   const float* prad = nullptr;
   const float* rrad = nullptr;   // the row tiles' own radii (piv2)
@@ -245,7 +246,13 @@ int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, 
                      const float* recf, const float* recr, int nfit, int Kp, int nseg, uint64_t* cand,
                      int* cand_n, int* derr = nullptr, const TcSkip* skip = nullptr,
                      float* dense = nullptr, float* rowthr = nullptr, const float* nmax = nullptr,
-                     unsigned long long* ntiles = nullptr, int rt0 = 0, int nrt_items = -1);
+                     unsigned long long* ntiles = nullptr, int rt0 = 0, int nrt_items = -1, bool seeded = false);
+// Thresholds for the rows of a fit set from its bounds lb to the pivots of a
+// reference set (column-tile pivots), into rowthr, and the nearest column tile of
+// each row tile, into home (knn_rms_tc.cu); then launch_screen_tc with seeded =
+// true and TcSkip::home starts from them.
+int tc_seed_rowthr(mds_ctx* ctx, const KnnRmsPlan& pl, const TcPivots& pv, const float* lb, const float* recf, int nfit,
+                   float* rowthr, int* home);
 // Split operands in steps: the buffer for n frames, then the rows of frames
 // [f0, f1) (f0 a multiple of a column tile; f1 too unless it is n).
 int tc_alloc(mds_ctx* ctx, const KnnRmsPlan& pl, int n, TcOperands& op, int layout);

@@ -1983,7 +1983,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     // (a set screened against itself uses row-tile pivots)
     TcSkip sk;
     TcPivots upv;
-    DevBuf ulb(ctx), tlo(ctx), farw(ctx), farp(ctx);
+    DevBuf ulb(ctx), tlo(ctx), farw(ctx), farp(ctx), home(ctx);
     TcPivots& pv = staged ? spv : upv;  // (staged: pivots, radii and bounds made with the chunks)
     DevBuf& lb = staged ? slb : ulb;
     const bool skipping = !pl.screen_keys && !pl.noskip && (nref + 79) / 80 >= 4;
@@ -2015,11 +2015,17 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
     MDS_TRY(rowthr.alloc(ctx, sizeof(float) * std::max(nfit, 1)));
     MDS_TRY(nmax.alloc(ctx, sizeof(float)));
     MDS_TRY(tc_rec_nmax(ctx, Rr.as<float>(), nref, nmax.as<float>()));
+    const bool seeded = skipping && !same;
+    if (seeded) {
+      MDS_TRY(home.alloc(ctx, sizeof(int) * ((nfit + TC_FR_M - 1) / TC_FR_M)));
+      MDS_TRY(tc_seed_rowthr(ctx, pl, pv, lb.as<float>(), Rfp, nfit, rowthr.as<float>(), home.as<int>()));
+      sk.home = home.as<int>();
+    }
     MDS_TRY(launch_screen_tc(ctx, pl, same ? tcr : tcf, tcr, Rfp, Rr.as<float>(), nfit, Kp, nseg,
                              cand.as<uint64_t>(), cand_n.as<int>(), pl.screen_keys ? nullptr : dst->tcerr + 2,
                              skipping ? &sk : nullptr, nullptr,
                              rowthr.as<float>(), pl.screen_keys ? nullptr : nmax.as<float>(),
-                             &dst->ntiles));
+                             &dst->ntiles, 0, -1, seeded));
     st.screen_launches = skipping ? 2 : 1;
     // (staged: the pivot pass ran with the chunks, its time in the prep stage)
     dense_pairs = skipping ? (long long)pv.nP * nfit : 0;

@@ -213,22 +213,26 @@ __device__ __forceinline__ int tile_order(int i, int t0, int t1, int td) {
   return (Rn > L) ? td + m + j : td - m - j;
 }
 
-// Column segment holding the column tile of row tile rt's middle frame.
-__device__ __forceinline__ int diag_seg(int rt, int nseg, int nct) {
-  const int dt = min((rt * TC_FR_M + TC_FR_M / 2) / TC_FR_N, nct - 1);
+// Column tile nearest to row tile rt: home[rt] (k_seed_thr), or the tile of its
+// middle frame for a set screened against itself.
+__device__ __forceinline__ int near_tile(int rt, int nct, const int* home) {
+  return home ? __ldg(home + rt) : min((rt * TC_FR_M + TC_FR_M / 2) / TC_FR_N, nct - 1);
+}
+// Column segment holding column tile dt.
+__device__ __forceinline__ int diag_seg(int dt, int nseg, int nct) {
   int s = 0;
   while (s + 1 < nseg && (int)((int64_t)nct * (s + 1) / nseg) <= dt) ++s;
   return s;
 }
 
-// Work item -> (row tile, column segment). A set screened against itself
-// (diag) first hands out, row tile by row tile, the segment holding the row
-// tile's own frames, and only then the other segments: by the time those
+// Work item -> (row tile, column segment). With a nearest column tile (diag: a
+// set screened against itself, or home) first hands out, row tile by row tile,
+// the segment holding it, and only then the other segments: by the time those
 // start, the near tiles have set the shared row thresholds they skip by.
 // The other segments come in the order far_perm gives (when not null: the
 // estimated heaviest first, so that the longest items do not start last).
 __device__ __forceinline__ void item_split(int item, int nrt, int nseg, int nct, int diag, const int* far_perm,
-                                           int& rt, int& seg) {
+                                           const int* home, int& rt, int& seg) {
   if (!diag || nseg == 1) {
     rt = item / nseg;
     seg = item % nseg;
@@ -236,12 +240,12 @@ __device__ __forceinline__ void item_split(int item, int nrt, int nseg, int nct,
   }
   if (item < nrt) {
     rt = item;
-    seg = diag_seg(rt, nseg, nct);
+    seg = diag_seg(near_tile(rt, nct, home), nseg, nct);
     return;
   }
   const int k = far_perm ? __ldg(far_perm + (item - nrt)) : item - nrt;
   rt = k / (nseg - 1);
-  const int s = k % (nseg - 1), sd = diag_seg(rt, nseg, nct);
+  const int s = k % (nseg - 1), sd = diag_seg(near_tile(rt, nct, home), nseg, nct);
   seg = s < sd ? s : s + 1;
 }
 
@@ -253,7 +257,8 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             const float* __restrict__ tlo, int piv2, const int* __restrict__ far_perm,
             float* __restrict__ dense, float* __restrict__ rowthr, const float* __restrict__ nmax, int k1,
             unsigned long long* __restrict__ ntiles,
-            uint64_t* __restrict__ candbuf, int* __restrict__ cand_n, int* __restrict__ err, int stall) {
+            uint64_t* __restrict__ candbuf, int* __restrict__ cand_n, int* __restrict__ err, int stall, int tight,
+            const int* __restrict__ home) {
   // err[0]: error code; err[1]: next unclaimed work item (zeroed by the host).
   // Work items (row tile, column segment) are claimed dynamically by each
   // CTA's producer, which also decides which column tiles of the item to
@@ -298,8 +303,11 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   // row threshold to min(K'-th bound, t'). The recheck verifies the (k+1)-th
   // exact value against the final shared threshold, as against the K'-th.
   //
+  // rowthr may hold thresholds from the start (k_seed_thr).
+  //
   // Dense mode (dense != null; the pivot pass): every pair's lower bound of
-  // RMSD (sqrt of the screen value) is written to dense[j][i]; no lists.
+  // RMSD (sqrt of the screen value) is written to dense[j][i]; no lists. With
+  // `tight` the bound is within the guard of the exact value.
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   unsigned char* base = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -378,10 +386,10 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         break;
       }
       int rt, seg;
-      item_split(item, nitems / nseg, nseg, ncoltiles, diag, far_perm, rt, seg);
+      item_split(item, nitems / nseg, nseg, ncoltiles, diag, far_perm, home, rt, seg);
       rt += rt0;
       const int t0 = (int)((int64_t)ncoltiles * seg / nseg), t1 = (int)((int64_t)ncoltiles * (seg + 1) / nseg);
-      const int td = diag ? min(max((rt * TC_FR_M + TC_FR_M / 2) / TC_FR_N, t0), t1 - 1) : t0;
+      const int td = diag ? min(max(near_tile(rt, ncoltiles, home), t0), t1 - 1) : t0;
       for (int ti = 0; ti < t1 - t0 && ok; ++ti) {
         if (pivlb) {
           // Skip test, again after every tile handed out (thresholds only
@@ -574,7 +582,7 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       if (task.x != cur) {
         // start of an item: row records and this warp's rows' lists
         cur = task.x;
-        item_split(cur, nitems / nseg, nseg, ncoltiles, diag, far_perm, rt, seg);
+        item_split(cur, nitems / nseg, nseg, ncoltiles, diag, far_perm, home, rt, seg);
         rt += rt0;
         grow = rt * TC_FR_M + rloc;
         rowok = (f < 10) && grow < nfit;
@@ -704,9 +712,9 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             cr[4 * v4] = t.x; cr[4 * v4 + 1] = t.y; cr[4 * v4 + 2] = t.z; cr[4 * v4 + 3] = t.w;
           }
           if (dense) {
-            // (pivot bounds: no refinement, a loose bound only weakens a skip)
+            // (unless tight: no refinement, a loose bound only weakens a skip)
             const float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]),
-                                                __builtin_huge_valf(), false);
+                                                __builtin_huge_valf(), tight != 0);
             dense[(int64_t)j * nfit + grow] = sqrtf(fmaxf(sv, 0.0f));
           } else {
             const float thr = fminf(*(volatile float*)&S->thr[rloc], S->gthr[rloc]);
@@ -867,7 +875,7 @@ int tc_seg_stride() { return TC_CAPG; }
 int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, const TcOperands& ref,
                      const float* recf, const float* recr, int nfit, int Kp, int nseg, uint64_t* cand,
                      int* cand_n, int* derr, const TcSkip* skip, float* dense, float* rowthr, const float* nmax,
-                     unsigned long long* ntiles, int rt0, int nrt_items) {
+                     unsigned long long* ntiles, int rt0, int nrt_items, bool seeded) {
   if (Kp + 2 * TC_FR_N > TC_CAPG)
     return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "tensor-core screen supports K' <= %d (k too large)",
                     TC_CAPG - 2 * TC_FR_N);
@@ -896,7 +904,7 @@ int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, 
     e = err.as<int>();
   }
   MDS_CUDA(ctx, cudaMemsetAsync(e, 0, 2 * sizeof(int), ctx->stream));  // error code, work counter
-  if (rowthr)  // 0x7f7f7f7f = 3.4e38: above every bound
+  if (rowthr && !seeded)  // 0x7f7f7f7f = 3.4e38: above every bound
     MDS_CUDA(ctx, cudaMemsetAsync(rowthr, 0x7f, sizeof(float) * (size_t)nfit, ctx->stream));
   const float s = tc_scale(pl.prec);
   const uint32_t idesc = umma_idesc_f16(TC_M, TC_N, pl.prec == MDS_PREC_FP16X3 ? 0 : 1);
@@ -905,12 +913,12 @@ int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, 
   ctx->stats.launches++;
   k_screen_tc<<<grid, TC_THREADS, smem, ctx->stream>>>(mA, mB, recf, recr, nfit, pl.nref, pl.Ap, pl.nofit,
                                                        pl.guard_tc, 1.0f / (s * s), idesc, Kp, nseg, nitems, rt0,
-                                                       &fit == &ref ? 1 : 0, skip ? skip->pivlb : nullptr,
+                                                       &fit == &ref || (skip && skip->home) ? 1 : 0, skip ? skip->pivlb : nullptr,
                                                        skip ? skip->prad : nullptr, skip ? skip->rrad : nullptr,
                                                        skip ? skip->tlo : nullptr,
                                                        skip ? skip->piv2 : 0, skip ? skip->far_perm : nullptr,
                                                        dense, rowthr, nmax, pl.k + 1, ntiles, cand, cand_n, e,
-                                                       stall);
+                                                       stall, dense && seeded ? 1 : 0, skip ? skip->home : nullptr);
   MDS_CUDA(ctx, cudaGetLastError());
   if (derr) return MDS_OK;
   int herr = 0;
@@ -1156,7 +1164,78 @@ int tc_skip_bounds(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, co
   const int nct = (pv.nP + TC_FR_N - 1) / TC_FR_N;
   const int nseg = std::max(1, std::min(nct, (4 * ctx->num_sms + nrt - 1) / nrt));
   return launch_screen_tc(ctx, pp, fit, pv.tc, recf, pv.R.as<float>(), nfit, 32, nseg, nullptr, nullptr, derr,
-                          nullptr, lb, nullptr, nullptr, nullptr, rt0, nrt);
+                          nullptr, lb, nullptr, nullptr, nullptr, rt0, nrt, !pv.rowpiv);
+}
+
+// rowthr[i] = an upper bound of the (k+1)-th smallest RMSD^2 of fit frame i:
+// with RMSD(i, p_T) <= u and every frame of column tile T within prad[T] of
+// its pivot, the TC_FR_N frames of T lie within u + prad[T], so the m-th
+// smallest of these over the full tiles, m = ceil((k+1) / TC_FR_N), bounds the
+// (k+1)-th distance. u from the pivot pass's (tight) bound lb: the exact
+// RMSD^2 is at most lb^2 + 2g (|a_i|^2 + |a_p|^2). Lanes take rows, warps take
+// every 32nd pivot. home[rt] = the column tile nearest to the row tile's middle
+// frame, which the screen visits first. Without it the rows of a fit set start with no threshold:
+// 2,047 frames of 304 atoms against 20,011, k = 50: 15.1 M pairs computed in
+// 0.54 ms, with it 11.0 M in 0.43 ms.
+#define SEED_MAX 5  // (K' <= 352: k + 1 <= 336)
+#define SEED_WARPS 32
+__global__ void __launch_bounds__(SEED_WARPS * 32) k_seed_thr(const float* __restrict__ lb, const float* __restrict__ recf,
+                                                  const float* __restrict__ recp, const float* __restrict__ prad,
+                                                  int nfit, int nfull, int m, float guard, float* __restrict__ rowthr,
+                                                  int* __restrict__ home) {
+  __shared__ float sv[SEED_WARPS][SEED_MAX][32];
+  __shared__ int sp[SEED_WARPS][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, row = blockIdx.x * 32 + lane;
+  float v[SEED_MAX];
+#pragma unroll
+  for (int i = 0; i < SEED_MAX; ++i) v[i] = INFINITY;
+  auto insert = [&](float x) {
+#pragma unroll
+    for (int i = 0; i < SEED_MAX; ++i) {
+      const float lo = fminf(v[i], x);
+      x = fmaxf(v[i], x);
+      v[i] = lo;
+    }
+  };
+  int near = 0;
+  if (row < nfit) {
+    const float e = __ldg(recf + (int64_t)row * MDS_REC + 15);
+#pragma unroll 4
+    for (int p = w; p < nfull; p += SEED_WARPS) {
+      const float l = __ldg(lb + (int64_t)p * nfit + row);
+      const float u2 = fmaf(l, l, 2.0f * guard * (e + __ldg(recp + (int64_t)p * MDS_REC + 15)));
+      const float x = sqrtf(u2) * (1.0f + 1e-5f) + __ldg(prad + p);
+      if (x < v[0]) near = p;
+      insert(x);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < SEED_MAX; ++i) sv[w][i][lane] = v[i];
+  sp[w][lane] = near;
+  __syncthreads();
+  if (w || row >= nfit) return;
+  for (int o = 1; o < SEED_WARPS; ++o) {
+    if (sv[o][0][lane] < v[0]) near = sp[o][lane];
+    for (int i = 0; i < m; ++i) insert(sv[o][i][lane]);
+  }
+  // (the middle row of a row tile; the last one of a tile cut short)
+  if (row % TC_FR_M == TC_FR_M / 2 || (row == nfit - 1 && row % TC_FR_M < TC_FR_M / 2)) home[row / TC_FR_M] = near;
+  float t = INFINITY;
+#pragma unroll
+  for (int i = 0; i < SEED_MAX; ++i)
+    if (i == m - 1) t = v[i];
+  rowthr[row] = fminf(t * t * (1.0f + 1e-5f), 3.0e38f);
+}
+
+int tc_seed_rowthr(mds_ctx* ctx, const KnnRmsPlan& pl, const TcPivots& pv, const float* lb, const float* recf, int nfit,
+                   float* rowthr, int* home) {
+  const int nfull = pl.nref / TC_FR_N, m = (pl.k + TC_FR_N) / TC_FR_N;
+  if (pv.rowpiv || m > SEED_MAX) return mds_fail(ctx, MDS_ERR_INTERNAL, "thresholds need column-tile pivots");
+  ctx->stats.launches++;
+  k_seed_thr<<<(nfit + 31) / 32, SEED_WARPS * 32, 0, ctx->stream>>>(lb, recf, pv.R.as<float>(), pv.rad.as<float>(), nfit, nfull, m,
+                                                        pl.guard_tc, rowthr, home);
+  MDS_CUDA(ctx, cudaGetLastError());
+  return MDS_OK;
 }
 
 // Order of the non-diagonal items (row tile R, other segment s'), heaviest
@@ -1177,7 +1256,7 @@ __global__ void k_far_est(const float* __restrict__ lb, const float* __restrict_
     if (r2 != R) m = fminf(m, __ldg(lb + (int64_t)r2 * N + pf));
   for (int o = 16; o > 0; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
   const float t = 2.0f * m;
-  const int sd = diag_seg(R, nseg, nC);
+  const int sd = diag_seg(near_tile(R, nC, nullptr), nseg, nC);
   for (int sp = 0; sp < nseg - 1; ++sp) {
     const int seg = sp < sd ? sp : sp + 1;
     const int t0 = (int)((int64_t)nC * seg / nseg), t1 = (int)((int64_t)nC * (seg + 1) / nseg);

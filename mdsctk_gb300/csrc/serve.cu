@@ -120,7 +120,7 @@ struct Request {
 struct Slot {
   mds_ctx* ctx = nullptr;
   int cap = 0;
-  DevBuf raw, A, R, cand, cand_n, out_d, out_i, flagged, nflag, derr, ext, lb, rowthr;
+  DevBuf raw, A, R, cand, cand_n, out_d, out_i, flagged, nflag, derr, ext, lb, rowthr, home;
   DevBuf audit;  // the recheck's audit counters of the screen's bounds (4 x u64)
   RecheckScratch rs;
   TcOperands tcq;
@@ -214,10 +214,14 @@ static int launch_batch(mds_server* S, Slot& sl, int bucket) {
                              sl.derr.as<int>() + 2));
       sk.pivlb = sl.lb.as<float>();
       sk.prad = S->pv.rad.as<float>();
+      MDS_TRY(tc_seed_rowthr(c, pl, S->pv, sl.lb.as<float>(), sl.R.as<float>(), bucket, sl.rowthr.as<float>(),
+                             sl.home.as<int>()));
+      sk.home = sl.home.as<int>();
     }
     MDS_TRY(launch_screen_tc(c, pl, sl.tcq, S->tc, sl.R.as<float>(), S->R.as<float>(), bucket, S->Kp, nseg,
                              sl.cand.as<uint64_t>(), sl.cand_n.as<int>(), sl.derr.as<int>(),
-                             S->pv.nC > 0 ? &sk : nullptr, nullptr, sl.rowthr.as<float>(), S->nmax.as<float>()));
+                             S->pv.nC > 0 ? &sk : nullptr, nullptr, sl.rowthr.as<float>(), S->nmax.as<float>(), nullptr, 0,
+                             -1, S->pv.nC > 0));
   } else {
     nseg = std::min(choose_nseg_fp32(bucket, c->num_sms, S->n, S->Kp, false), segs);
     MDS_CUDA(c, cudaMemsetAsync(sl.derr.p, 0, sizeof(int), c->stream));
@@ -595,6 +599,7 @@ extern "C" int mds_server_create(const mds_server_config* cfg, const float* land
               sl.flagged.alloc(c, sizeof(int) * cap) == MDS_OK && sl.nflag.alloc(c, sizeof(int)) == MDS_OK &&
               sl.audit.alloc(c, 4 * sizeof(unsigned long long)) == MDS_OK &&
               sl.derr.alloc(c, 4 * sizeof(int)) == MDS_OK && sl.rowthr.alloc(c, sizeof(float) * cap) == MDS_OK &&
+              sl.home.alloc(c, sizeof(int) * (cap / TC_FR_M + 1)) == MDS_OK &&
               (S->pv.nC == 0 || sl.lb.alloc(c, sizeof(float) * (size_t)S->pv.nC * cap) == MDS_OK) &&
               sl.ext.alloc(c, sizeof(double) * (size_t)cap * S->nev) == MDS_OK &&
               recheck_scratch(c, cap, sl.rs) == MDS_OK;
@@ -638,6 +643,7 @@ extern "C" int mds_server_destroy(mds_server* S) {
     sl.raw.release(); sl.A.release(); sl.R.release(); sl.cand.release();
     sl.cand_n.release(); sl.out_d.release(); sl.out_i.release(); sl.flagged.release(); sl.nflag.release();
     sl.derr.release(); sl.ext.release(); sl.tcq.A.release(); sl.tcq.B.release(); sl.lb.release(); sl.rowthr.release();
+    sl.home.release();
     sl.audit.release(); sl.rs.rc.release(); sl.rs.meta.release(); sl.rs.cidx.release(); sl.rs.cbound.release();
     sl.rs.sums.release(); sl.rs.big.release(); sl.rs.nbig.release();
     mds_destroy(sl.ctx);
