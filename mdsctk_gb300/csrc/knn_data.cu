@@ -793,7 +793,9 @@ k_recheck_exact(const double* __restrict__ Xfit, const double* __restrict__ Xref
 // (k+1)-th exact value and that value lies below tau, or when every
 // candidate was rechecked (then dk < tau is required, else the row is
 // flagged); otherwise it goes to the block kernel, which rechecks all its
-// candidates.
+// candidates. PER: 32 PER slots hold the row's fw = k + 3 (bound by the sorting
+// network; 200,000 rows of 35: 268 us, 404 with 128 slots).
+template <int PER>
 __global__ void __launch_bounds__(RW_WARPS * 32)
 k_recheck_finish(int nrows, int k, int fw, const int* __restrict__ cidx, const int4* __restrict__ meta,
                  const double* __restrict__ ev, double* __restrict__ out_d, int* __restrict__ out_i,
@@ -806,16 +808,16 @@ k_recheck_finish(int nrows, int k, int fw, const int* __restrict__ cidx, const i
   if (first < 0) return;
   const float tau = __int_as_float(m.z), nxt = __int_as_float(m.w);
   const int k1 = k + 1;
-  uint64_t v[4];
-  int x[4];
+  uint64_t v[PER];
+  int x[PER];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = i * 32 + lane;
     v[i] = (e < first) ? (uint64_t)__double_as_longlong(ev[(int64_t)row * fw + e]) : 0x7ff0000000000000ull;
     x[i] = (e < first) ? cidx[(int64_t)row * fw + e] : 0x7fffffff;
   }
-  wsort_pair<4>(v, x, lane);
-  const uint64_t dkb = lane_elem<4>(v, k1 - 1);
+  wsort_pair<PER>(v, x, lane);
+  const uint64_t dkb = lane_elem<PER>(v, k1 - 1);
   const double dk = __longlong_as_double((long long)dkb);
   if (first < total && !(dk < (double)nxt && dk < (double)tau)) {
     if (lane == 0) big[atomicAdd(nbig, 1)] = row;
@@ -825,7 +827,7 @@ k_recheck_finish(int nrows, int k, int fw, const int* __restrict__ cidx, const i
   // dk < tau proves that no left-out pair ties with or beats the k+1-th
   if (lane == 0 && first == total && !(dk < (double)tau)) flagged[atomicAdd(nflag, 1)] = row;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < PER; ++i) {
     const int e = i * 32 + lane;
     if (e >= 1 && e <= k) {
       const bool have = e < first;
@@ -931,7 +933,8 @@ int knn_data_run(mds_ctx* ctx, const double* dref, int nref, const double* dfit,
       const int64_t slots = (int64_t)nrows * fw;
       k_recheck_exact<<<(int)((slots + 255) / 256), 256, 0, s>>>(ea, eb, sf, Sr.as<double>(), nrows, dim, corr, fw,
                                                                  cidx.as<int>(), meta.as<int4>(), evals.as<double>());
-      k_recheck_finish<<<wb, RW_WARPS * 32, 0, s>>>(nrows, k, fw, cidx.as<int>(), meta.as<int4>(),
+      auto finish = fw <= 32 ? k_recheck_finish<1> : fw <= 64 ? k_recheck_finish<2> : k_recheck_finish<4>;
+      finish<<<wb, RW_WARPS * 32, 0, s>>>(nrows, k, fw, cidx.as<int>(), meta.as<int4>(),
                                                     evals.as<double>(), dout_d, dout_i, flagged.as<int>(),
                                                     nflag.as<int>(), big.as<int>(), nbig.as<int>());
       MDS_CUDA(ctx, cudaGetLastError());
