@@ -562,6 +562,7 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     bool ok = true;
     int cur = -1, rt = 0, seg = 0, grow = 0, ntile = 0;
     bool rowok = false;
+    float far = 0.f;  // dense: the row tile's radius and that of its own frames' neighbours
     // The epilogue warps meet at named barrier 1 three times per tile: after
     // the task read (every warp has finished the previous tile, its
     // compactions and any publishing), after the accumulator is ready, and
@@ -586,6 +587,7 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         rt += rt0;
         grow = rt * TC_FR_M + rloc;
         rowok = (f < 10) && grow < nfit;
+        if (dense && !tight) far = __ldg(rrad + rt) + __ldg(prad + rt);
         ntile = 0;
         if (ew == 0)
           for (int r = lane; r < TC_FR_M; r += 32) {
@@ -712,9 +714,12 @@ k_screen_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             cr[4 * v4] = t.x; cr[4 * v4 + 1] = t.y; cr[4 * v4 + 2] = t.z; cr[4 * v4 + 3] = t.w;
           }
           if (dense) {
-            // (unless tight: no refinement, a loose bound only weakens a skip)
-            const float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]),
-                                                __builtin_huge_valf(), tight != 0);
+            // Unless tight: no refinement, and no quartic where the cheap bound
+            // already lies beyond what a skip of the pivot's frames needs
+            // (far + prad[j]): a loose bound only weakens a skip.
+            const float fj = tight ? INFINITY : far + __ldg(prad + j);
+            const float sv = screen_shifted_f32(G, rrec, cr, nofit != 0, guard * (rrec[15] + cr[15]), fj * fj,
+                                                tight != 0);
             dense[(int64_t)j * nfit + grow] = sqrtf(fmaxf(sv, 0.0f));
           } else {
             const float thr = fminf(*(volatile float*)&S->thr[rloc], S->gthr[rloc]);
@@ -1163,8 +1168,13 @@ int tc_skip_bounds(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, co
   // column segments (no lists in dense mode) so that there are >= 4 items per SM
   const int nct = (pv.nP + TC_FR_N - 1) / TC_FR_N;
   const int nseg = std::max(1, std::min(nct, (4 * ctx->num_sms + nrt - 1) / nrt));
+  TcSkip sk;
+  if (pv.rowpiv) {
+    sk.prad = pv.rad.as<float>();
+    sk.rrad = pv.rrad.as<float>();
+  }
   return launch_screen_tc(ctx, pp, fit, pv.tc, recf, pv.R.as<float>(), nfit, 32, nseg, nullptr, nullptr, derr,
-                          nullptr, lb, nullptr, nullptr, nullptr, rt0, nrt, !pv.rowpiv);
+                          &sk, lb, nullptr, nullptr, nullptr, rt0, nrt, !pv.rowpiv);
 }
 
 // rowthr[i] = an upper bound of the (k+1)-th smallest RMSD^2 of fit frame i:
