@@ -18,7 +18,7 @@
 //    landmark template, split-precision operands, candidate screen against
 //    the landmarks, exact recheck, Nystrom extension, result copies) is
 //    captured once per (slot, size bucket) and replayed; the batch is padded
-//    to its bucket with zero frames whose results are ignored.
+//    to its bucket with copies of its last frame, whose results are ignored.
 //  * the rare rows whose screen guard fails are finished on the host side of
 //    the slot (wider screen, exact rows) before results are published.
 //
@@ -49,6 +49,16 @@ double now_ms() {
 
 // Z [nev][n] / lambda -> Zl [n][nev]: the extension reads one landmark's
 // nev values in one piece. Once per model.
+// Frames m .. m + gridDim.x - 1 := frame m - 1. (Frames of zeros lie about as far
+// from one landmark as from another: they kept every column tile open for their
+// row tile, overflowed their lists and held the rotation's Newton for all its
+// steps. A batch of 533 frames padded to 768: PAD_A us, with copies PAD_B.)
+__global__ void k_pad_frames(float* __restrict__ raw, int64_t fr, int m) {
+  const float* a = raw + fr * (m - 1);
+  float* b = raw + fr * (m + blockIdx.x);
+  for (int64_t e = threadIdx.x; e < fr; e += blockDim.x) b[e] = a[e];
+}
+
 __global__ void k_serve_scale(const double* __restrict__ Z, const double* __restrict__ lam, int n, int nev,
                               double* __restrict__ Zl) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -333,9 +343,10 @@ static int start_batch(mds_server* S, Slot& sl) {
   }
   sl.bucket = std::min(bucket_for(sl.m), sl.cap);
   MDS_CUDA(c, cudaMemcpyAsync(sl.raw.p, sl.h_raw, sizeof(float) * fr * sl.m, cudaMemcpyHostToDevice, c->stream));
-  if (sl.bucket > sl.m)
-    MDS_CUDA(c, cudaMemsetAsync(sl.raw.as<float>() + fr * sl.m, 0, sizeof(float) * fr * (sl.bucket - sl.m),
-                                c->stream));
+  if (sl.bucket > sl.m) {
+    k_pad_frames<<<sl.bucket - sl.m, 256, 0, c->stream>>>(sl.raw.as<float>(), (int64_t)fr, sl.m);
+    MDS_CUDA(c, cudaGetLastError());
+  }
   auto it = sl.graphs.find(sl.bucket);
   if (it != sl.graphs.end()) {
     MDS_CUDA(c, cudaGraphLaunch(it->second, c->stream));
