@@ -328,9 +328,10 @@ __global__ void __launch_bounds__(128) k_prep_sums(const float* __restrict__ raw
 }
 
 // The rotation of every frame (one thread per frame, FP64 QCP): record
-// entries 3..12 (|y|^2, y mu^T) -> 3..11 (R, row-major). Bound by the FP64
-// pipe (1.6 multiply-adds per cycle and SM), so a warp is a block of its own:
-// 2,501 frames on all SMs RO_B us, on the 20 that blocks of 128 filled RO_A.
+// entries 3..12 (|y|^2, y mu^T) -> 3..11 (R, row-major). Bound by the latency
+// of the FP64 steps (67 cycles each) and by the FP64 pipe (1.6 multiply-adds
+// per cycle and SM), so a warp is a block of its own: 2,501 frames 17.3 us,
+// 18.5 in blocks of 128 on 20 SMs.
 __global__ void k_prep_rot(int n, const double* __restrict__ M0, float* __restrict__ rec) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= n) return;
@@ -1054,12 +1055,12 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
 //  3. k_rc_finish   a warp per row: the eigenvalue solves (a lane per pair), the
 //                   selection, guard check and audit, the output.
 // Rows with more candidates than that whose next bound does not settle them,
-// with more than RC3_LIST keys, or with fewer than k+1 below the threshold are
-// listed in big[] for k_recheck. 100,000 x 304, k = 64: 5.37 -> RC3_A ms;
-// 20,000 x 1,000, k = 100: 2.41 -> RC3_B ms, outputs bit-identical.
+// or with fewer than k+1 below the threshold are listed in big[] for k_recheck.
+// 100,000 x 304, k = 64: 5.37 -> 4.1 ms; 20,000 x 1,000, k = 100: 2.41 -> 2.3
+// ms, outputs bit-identical.
 #define RC3_CAP 128    // candidates per row (256: the rows with more are rechecked in full, 2.63 against 2.37 ms
                        // at 20,000 x 1,000)
-#define RC3_LIST 512   // keys per row that stage 1 holds
+#define RC3_LIST 512   // keys per row that stage 1 holds (K' <= 448 and one step of 32)
 #define RC3_MAXK1 120  // k + 1 (eight candidates to spare, as the block kernel's first chunk)
 #define RC3_WARPS 8
 
@@ -1112,24 +1113,30 @@ k_rc_cands(const uint64_t* __restrict__ cand, const int* __restrict__ cand_n, in
   const int t = __reduce_add_sync(0xffffffffu, segn);
   const float rthr = rowthr ? __ldcg(rowthr + row) : __int_as_float(0x7f800000);
   // the keys at or below the row's threshold (each list ascends, so a list is
-  // left at its first key above it)
+  // left at its first key above it); when the buffer fills, its K' smallest
+  // stay and the last of those is the limit from then on
   int m = 0;
+  float lim = rthr;
   for (int s = 0; s < nseg; ++s) {
     const int ns = __shfl_sync(0xffffffffu, segn, s);
     const uint64_t* src = cand + ((int64_t)row * nseg + s) * segstride;
     for (int x0 = 0; x0 < ns; x0 += 32) {
       const int x = x0 + lane;
       const uint64_t key = (x < ns) ? src[x] : MDS_KEY_INF;
-      const bool keep = x < ns && mds_key_value(key) <= rthr;
+      if (m > RC3_LIST - 32) {
+        warp_sort_keys(buf, m, lane);
+        m = Kp;
+        lim = fminf(lim, mds_key_value(buf[Kp - 1]));
+      }
+      const bool keep = x < ns && mds_key_value(key) <= lim;
       const unsigned bal = __ballot_sync(0xffffffffu, keep);
-      const int p = m + __popc(bal & ((1u << lane) - 1u));
-      if (keep && p < RC3_LIST) buf[p] = key;
+      if (keep) buf[m + __popc(bal & ((1u << lane) - 1u))] = key;
       m += __popc(bal);
       if (bal != 0xffffffffu) break;
     }
   }
   __syncwarp();
-  if (m > RC3_LIST || m < min(t, k1)) {
+  if (m < min(t, k1)) {
     if (lane == 0) {
       meta[rl] = make_int4(-1, 0, 0, 0);
       big[atomicAdd(nbig, 1)] = row;
@@ -1301,7 +1308,7 @@ k_rc_finish(const float* __restrict__ rc, const float* __restrict__ Ur, int row0
 // chunks of FR_KC through shared memory (two TMA boxes a chunk, FR_ST stages); a group of 8 lanes sums 2 rows x 2 frames, so each shared-memory load
 // serves two pairs and the FMA pipe, not the L1 pipe, is the bound. Twelve
 // warps of 160 registers. Per pair the sums run over the same atoms in the same
-// lanes and order as in recheck_chunk (bit-identical). 3,001 x 257 atoms: FR_B
+// lanes and order as in recheck_chunk (bit-identical). 3,001 x 257 atoms: 2.54
 // ms; one row per block, every frame read from L2 for it alone, 2.78 ms. (With
 // each thread issuing its own 16-byte copies 3.6 ms, with a bulk copy per 256
 // contiguous bytes 6.4 ms: the copies' own instructions were the limit.)
@@ -1828,7 +1835,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   MDS_TRY(Ur.alloc(ctx, sizeof(float) * MDS_USTRIDE * (size_t)nref));
   // Superposition, one upload chunk at a time, each chunk uploaded while the
   // one before it is superposed (2,047 frames of 304 atoms against 20,011 from
-  // pageable memory: UP_B us a call, UP_A with all copies issued first).
+  // pageable memory: 1,697 us a call, 2,100 with all copies issued first).
   auto prep_chunks = [&](const float* draw, const float* host, const std::vector<int>& cb, int nc, int ev0, float* A,
                          float* R, float* U, int* bad) -> int {
     for (int c = 0; c < nc; ++c) {

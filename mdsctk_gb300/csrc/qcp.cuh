@@ -113,13 +113,8 @@ __device__ inline double qcp_rotation_fp64(const double* S, double e0half, doubl
   c2 *= -2.0;
   double c1 = -8.0 * det3d(S[0], S[1], S[2], S[3], S[4], S[5], S[6], S[7], S[8]);
   double c0 = det4d(K);
-  // At rounding level the steps of some frames do not fall below 1e-15 but
-  // repeat a few values; a step depends on lam alone, so once a value returns
-  // the steps left are the same modulo the period (one such frame among a
-  // request's 533 held k_prep_rot for NW_A us, now NW_B).
-  double lam = e0half, mark = e0half;
-  int end = 60, mark_it = 0;
-  for (int it = 0; it < end; ++it) {
+  double lam = e0half;
+  for (int it = 0; it < 60; ++it) {
     double l2 = lam * lam;
     double p = (l2 + c2) * l2 + c1 * lam + c0;
     double dp = 4.0 * l2 * lam + 2.0 * c2 * lam + c1;
@@ -128,11 +123,6 @@ __device__ inline double qcp_rotation_fp64(const double* S, double e0half, doubl
     bool done = fabs(nl - lam) <= 1e-15 * fabs(nl) + 1e-300;
     lam = nl;
     if (done) break;
-    if (lam == mark && end == 60) end = it + 1 + (59 - it) % (it + 1 - mark_it);
-    if (it + 1 == 4 || it + 1 == 7 || it + 1 == 11 || it + 1 == 17 || it + 1 == 30) {
-      mark = lam;
-      mark_it = it + 1;
-    }
   }
   double A[16];
   for (int i = 0; i < 16; ++i) A[i] = K[i];

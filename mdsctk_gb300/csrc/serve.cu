@@ -47,18 +47,18 @@ double now_ms() {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-// Z [nev][n] / lambda -> Zl [n][nev]: the extension reads one landmark's
-// nev values in one piece. Once per model.
 // Frames m .. m + gridDim.x - 1 := frame m - 1. (Frames of zeros lie about as far
 // from one landmark as from another: they kept every column tile open for their
 // row tile, overflowed their lists and held the rotation's Newton for all its
-// steps. A batch of 533 frames padded to 768: PAD_A us, with copies PAD_B.)
+// steps, 55 us against 16.)
 __global__ void k_pad_frames(float* __restrict__ raw, int64_t fr, int m) {
   const float* a = raw + fr * (m - 1);
   float* b = raw + fr * (m + blockIdx.x);
   for (int64_t e = threadIdx.x; e < fr; e += blockDim.x) b[e] = a[e];
 }
 
+// Z [nev][n] / lambda -> Zl [n][nev]: the extension reads one landmark's
+// nev values in one piece. Once per model.
 __global__ void k_serve_scale(const double* __restrict__ Z, const double* __restrict__ lam, int n, int nev,
                               double* __restrict__ Zl) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

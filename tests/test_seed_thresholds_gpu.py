@@ -39,3 +39,19 @@ def test_seeded_copies(ctx, oracle):
     d, i = ctx.knn_rms(ref, x[:70], m, 5, precision="bf16x3")
     od, oi = oracle.knn_rms(ref, x[:70], m, 5)
     assert np.max(np.abs(d - od)) <= 1e-4  # the bound of the other tests against the oracle
+
+
+@pytest.mark.parametrize("precision", ["bf16x3", "fp32"])
+@pytest.mark.parametrize("k", [10, 80])
+def test_rows_with_overfull_lists(ctx, oracle, precision, k):
+    """Fit frames about as far from every reference frame as from any other:
+    the segments' lists hold more keys below the threshold than a row's buffer
+    in the recheck (512), which then keeps its K' smallest."""
+    ref = synth.trajectory(6000, 40, seed=3, basins=5, dwell=60)
+    fit = np.zeros((45, 40, 3), np.float32)
+    fit[20:] = ref[:25] + np.random.default_rng(4).normal(scale=0.6, size=(25, 40, 3)).astype(np.float32)
+    m = synth.uniform_masses(40)
+    d, _ = ctx.knn_rms(ref, fit, m, k, precision=precision)
+    od, _ = oracle.knn_rms(ref, fit, m, k)
+    assert np.all(np.diff(d, axis=1) >= 0)
+    assert np.max(np.abs(d - od)) <= 1e-4  # the bound of the other tests against the oracle
