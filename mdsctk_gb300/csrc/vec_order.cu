@@ -50,17 +50,19 @@ __global__ void k_vo_seed(const float* __restrict__ X, int n, int Dp, float* __r
 // keys/vals: (centroid << 12 | distance quantised against *dmax) and the
 // vector's index, for the sort; dist/dmax: the distance to the nearest
 // centroid and (float bits) the largest one, for that quantisation.
+// The block's sums: thread (g, d) adds component d of every G-th vector to its
+// own 16 accumulators, so no two threads share one. (One thread per vector,
+// Dp shared-memory FP64 atomics each, took 70 us a launch at 8,000 x 40, most
+// of the order's time; now 25.)
 __global__ void __launch_bounds__(256) k_vo_assign(const float* __restrict__ X, int n, int Dp, int stride,
                                                    const float* __restrict__ cent, double* __restrict__ sums,
                                                    int* __restrict__ counts, float* __restrict__ dist,
                                                    unsigned* __restrict__ dmax, int* __restrict__ label) {
-  __shared__ float cs[VO_CENT * VO_MAXDP];
-  __shared__ double ss[VO_CENT * VO_MAXDP];
+  __shared__ __align__(16) float cs[VO_CENT * VO_MAXDP];
+  __shared__ double ss[VO_CENT * 256];  // [centroid][thread]
   __shared__ int sc[VO_CENT];
-  for (int e = threadIdx.x; e < VO_CENT * Dp; e += blockDim.x) {
-    cs[e] = cent[e];
-    if (sums) ss[e] = 0.0;
-  }
+  __shared__ int sl[256];  // the block's labels (-1: no vector)
+  for (int e = threadIdx.x; e < VO_CENT * Dp; e += blockDim.x) cs[e] = cent[e];
   if (threadIdx.x < VO_CENT) sc[threadIdx.x] = 0;
   __syncthreads();
   const int64_t v = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x) * stride;
@@ -75,14 +77,14 @@ __global__ void __launch_bounds__(256) k_vo_assign(const float* __restrict__ X, 
       const float4 xv = x4[q];
 #pragma unroll
       for (int c = 0; c < VO_CENT; ++c) {
-        const float* cc = cs + c * Dp + 4 * q;
-        float e = xv.x - cc[0];
+        const float4 cc = *reinterpret_cast<const float4*>(cs + c * Dp + 4 * q);
+        float e = xv.x - cc.x;
         acc[c] = fmaf(e, e, acc[c]);
-        e = xv.y - cc[1];
+        e = xv.y - cc.y;
         acc[c] = fmaf(e, e, acc[c]);
-        e = xv.z - cc[2];
+        e = xv.z - cc.z;
         acc[c] = fmaf(e, e, acc[c]);
-        e = xv.w - cc[3];
+        e = xv.w - cc.w;
         acc[c] = fmaf(e, e, acc[c]);
       }
     }
@@ -92,10 +94,7 @@ __global__ void __launch_bounds__(256) k_vo_assign(const float* __restrict__ X, 
         best = acc[c];
         bl = c;
       }
-    if (sums) {
-      for (int d = 0; d < Dp; ++d) atomicAdd(&ss[bl * Dp + d], (double)X[(int64_t)v * Dp + d]);
-      atomicAdd(&sc[bl], 1);
-    }
+    if (sums) atomicAdd(&sc[bl], 1);
     if (dist) {
       const float dv = sqrtf(best);
       dist[v] = dv;
@@ -104,9 +103,27 @@ __global__ void __launch_bounds__(256) k_vo_assign(const float* __restrict__ X, 
     }
   }
   if (sums) {
+    sl[threadIdx.x] = v < n ? bl : -1;
     __syncthreads();
-    for (int e = threadIdx.x; e < VO_CENT * Dp; e += blockDim.x)
-      if (ss[e] != 0.0) atomicAdd(&sums[e], ss[e]);
+    const int G = 256 / Dp, g = threadIdx.x / Dp, d = threadIdx.x % Dp;
+    double* mine = ss + threadIdx.x;
+    if (g < G) {
+#pragma unroll
+      for (int c = 0; c < VO_CENT; ++c) mine[256 * c] = 0.0;
+      const int64_t v0 = (int64_t)blockIdx.x * 256;
+#pragma unroll 8
+      for (int i = g; i < 256; i += G) {
+        const int c = sl[i];
+        if (c >= 0) mine[256 * c] += (double)X[(v0 + i) * stride * Dp + d];
+      }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < VO_CENT * Dp; e += blockDim.x) {
+      const double* from = ss + 256 * (e / Dp) + e % Dp;
+      double t = 0.0;
+      for (int o = 0; o < G; ++o) t += from[o * Dp];
+      if (t != 0.0) atomicAdd(&sums[e], t);
+    }
     if (threadIdx.x < VO_CENT && sc[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sc[threadIdx.x]);
   }
 }
