@@ -1012,7 +1012,7 @@ int knn_data_run(mds_ctx* ctx, const double* dref, int nref, const double* dfit,
     // a warp per row and segment: enough warps for every SM, and lists that
     // the recheck can merge in registers
     const int seg = std::min({std::max(RW_MAXT / Kp, 1), pct, ctx->num_sms * 32 / nfit + 1});
-    prows = (int)std::min<int64_t>(nfit, std::max<int64_t>(DP_PANEL_BYTES / (ld * 4) / DP_T, 1) * DP_T);
+    prows = (int)std::min<int64_t>(nfit, std::max<int64_t>(DP_PANEL_BYTES / (ld * 4) / DP_TM, 1) * DP_TM);
     if (panel.alloc(ctx, sizeof(float) * (size_t)ld * prows) == MDS_OK && alloc_lists(seg) == MDS_OK) {
       nseg = seg;
     } else {  // (a small HBM budget)

@@ -422,6 +422,7 @@ __global__ void __launch_bounds__(128) k_prep_out(const float* __restrict__ raw,
 #define SC_KC 32
 #define SC_FS 98  // floats per frame per stage: 3*32 + 2 (bank spread)
 #define SC_THREADS 256
+#define SC_SKIP_TILES 22  // 80-frame column tiles from which a set against itself skips tiles
 #define SC_STATIC (4 * SC_TM * (MDS_REC + 1) + 1024)  // shared memory besides the dynamic part
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
@@ -1961,7 +1962,11 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       ex.ntiles = &dst->ntiles;
     }
     ex.diag = same ? 1 : 0;
-    const bool skipping = !keys_only && !pl.noskip && same && (nref + TC_FR_N - 1) / TC_FR_N >= 4;
+    // Below SC_SKIP_TILES column tiles the pivots cost more than the tiles they
+    // save (whole calls, host frames: 1,000 x 60 atoms 307 us with skipping, 265
+    // without; 1,500 x 304 824 / 740; 2,000 x 60 381 / 405; 2,000 x 304 767 /
+    // 1,045).
+    const bool skipping = !keys_only && !pl.noskip && same && (nref + TC_FR_N - 1) / TC_FR_N >= SC_SKIP_TILES;
     st.screen_launches = 1;
     if (skipping) {
       MDS_TRY(tc_skip_pivots(ctx, pl, Ar.as<float>(), Rr.as<float>(), f_pv, true));

@@ -18,6 +18,8 @@ pytestmark = pytest.mark.gpu
     (2100, 300, 50, 120),
     (900, None, 61, 16),
     (1500, None, 40, 100),
+    (1680, None, 40, 20),  # 21 column tiles: no skipping
+    (1690, None, 40, 20),  # 22: skipping
     (1300, None, 40, 200),
 ])
 @pytest.mark.parametrize("nofit", [False, True])
