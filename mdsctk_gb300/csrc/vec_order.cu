@@ -159,24 +159,37 @@ __global__ void k_vo_perm(const int64_t* __restrict__ vals, int n, int* __restri
 }
 
 // Column tile T = sorted vectors [T * tile, T * tile + tile): FP32 centre and
-// radius (rounded up). Block: `tile` threads.
+// radius (rounded up). Block: `tile` threads; for the centre, thread (g, d)
+// sums component d of every G-th vector, G = tile / Dp (one thread per
+// component, all vectors one after another: 77 us for both launches at 8,000
+// x 40; now 53).
 __global__ void k_vo_tile_geom(const float* __restrict__ X, const int* __restrict__ perm, int n, int Dp, int tile,
                                float* __restrict__ center, float* __restrict__ rad) {
   __shared__ float cf[VO_MAXDP];
+  __shared__ double part[256];
   __shared__ float red[32];
   const int T = blockIdx.x, t = threadIdx.x;
   const int j0 = T * tile, m = min(tile, n - j0);
-  for (int d = t; d < Dp; d += blockDim.x) {
+  const int G = tile / Dp, g = t / Dp;  // (Dp <= 128 <= tile)
+  if (g < G) {
     double s = 0.0;
-    for (int j = 0; j < m; ++j) s += (double)X[(int64_t)perm[j0 + j] * Dp + d];
-    cf[d] = (float)(s / m);
-    center[(int64_t)T * Dp + d] = cf[d];
+#pragma unroll 8
+    for (int j = g; j < m; j += G) s += (double)X[(int64_t)perm[j0 + j] * Dp + t % Dp];
+    part[t] = s;
+  }
+  __syncthreads();
+  if (t < Dp) {
+    double s = 0.0;
+    for (int o = 0; o < G; ++o) s += part[o * Dp + t];
+    cf[t] = (float)(s / m);
+    center[(int64_t)T * Dp + t] = cf[t];
   }
   __syncthreads();
   float r = 0.0f;
   if (t < m) {
     const float* y = X + (int64_t)perm[j0 + t] * Dp;
     double s = 0.0;
+#pragma unroll 8
     for (int d = 0; d < Dp; ++d) {
       const double e = (double)y[d] - (double)cf[d];
       s += e * e;
@@ -230,7 +243,9 @@ __device__ __forceinline__ void warp_sort128(float (&v)[4], int lane) {
 // FP32 arithmetic -- an upper bound of the row's k1-th smallest over the
 // whole reference set, which holds those members. Block: one row pair tile,
 // 8 warps taking its rows in turn (lane j: members j, j + 32, j + 64, j + 96).
-// Rows whose start tile has fewer than k1 members keep +inf.
+// Rows whose start tile has fewer than k1 members keep +inf. The rows of an item
+// are shared among gridDim.y blocks, so that a small set fills the GPU (8,000 x
+// 40: 123 us with one block per item, 36 with eight).
 __global__ void __launch_bounds__(256) k_vo_seed_rows(const float* __restrict__ Xr, const int* __restrict__ permr,
                                                       int nref, const float* __restrict__ Xf,
                                                       const int* __restrict__ permf, int nfit, int Dp,
@@ -250,7 +265,7 @@ __global__ void __launch_bounds__(256) k_vo_seed_rows(const float* __restrict__ 
   }
   __syncthreads();
   const float nm = __ldg(nmax);
-  for (int r = w; r < 256; r += 8) {
+  for (int r = w + 8 * blockIdx.y; r < 256; r += 8 * gridDim.y) {
     const int g = item * 256 + r;
     if (g >= nfit) break;
     const float* x = Xf + (int64_t)permf[g] * Dp;
@@ -600,8 +615,9 @@ int vec_seed_rows(mds_ctx* ctx, const float* Xr, const int* permr, int nref, con
   static size_t attr_limit = 0;
   MDS_TRY(mds_allow_dyn_smem(ctx, k_vo_seed_rows, &attr_done, &attr_limit));
   if (smem > attr_limit) return MDS_OK;
-  k_vo_seed_rows<<<nitems, 256, smem, ctx->stream>>>(Xr, permr, nref, Xf, permf, nfit, Dp, tdall, ncoltiles, k1,
-                                                      nmax, rowthr, devn);
+  const int parts = std::max(1, std::min(8, 4 * ctx->num_sms / std::max(nitems, 1)));
+  k_vo_seed_rows<<<dim3(nitems, parts), 256, smem, ctx->stream>>>(Xr, permr, nref, Xf, permf, nfit, Dp, tdall,
+                                                                  ncoltiles, k1, nmax, rowthr, devn);
   ctx->stats.launches++;
   MDS_CUDA(ctx, cudaGetLastError());
   return MDS_OK;
