@@ -189,8 +189,7 @@ struct TcShared {
   float gthr[TC_FR_M];              // rows' global thresholds, refreshed per tile
 };
 
-// per-warp shared scratch: the radix-select histogram, and the final sort of a
-// row's list when it holds at most TC_SCR keys
+// per-warp shared scratch of the radix select, in 8-byte words
 #define TC_SCR 256
 #define TC_SMEM_BYTES (TC_STAGES * TC_STAGE_BYTES + sizeof(TcShared) + TC_EPI_WARPS * TC_SCR * 8 + 1024)
 static_assert(TC_SMEM_BYTES <= 227 * 1024, "screen shared memory exceeds the per-block limit");
