@@ -157,11 +157,13 @@ __device__ inline double qcp_rotation_fp64(const double* S, double e0half, doubl
 // with U = sum a mu^T and M0 = sum mu mu^T.
 #define MDS_REC 16
 
-__device__ __forceinline__ float sqrt_approx(float x) {
+#ifdef __CUDACC__  // (a host build brings its own)
+__device__ __forceinline__ float sqrt_approx(float x) {  // within 2^-23 relative
   float r;
   asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+#endif
 
 // Screen value (lower bound of RMSD^2, nm^2) from the deviation Gram
 // G[3*c+d] = sum a_i^c a_j^d of fit frame i (row record r) and reference
@@ -172,8 +174,13 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 // returned without the quartic solve (the caller rejects such pairs anyway):
 // with g >= lambda_max(D') (Gershgorin), nu <= (g + sqrt(g^2 + 4|b|^2)) / 2,
 // the largest eigenvalue of [[0, |b|], [|b|, g]], which dominates K'.
-// The approximate square root and quotients (2 ulp) move the result by less
-// than 1e-6 nu, against guards of 1.5e-5 and 6e-5 of |a_i|^2 + |a_j|^2 >= nu.
+// In FP32 that bound is raised by 2^-21 (sqrt(g^2 + 4|b|^2) + |tr D'|): for
+// superposed frames g is about minus the radius of gyration squared and the sum
+// cancels, so its error is an ulp of g, not of nu, and so are the roundings of
+// g's own row sums. (Newton only comes down, so a start below the root stays
+// there: without the raise rigid frames had bounds up to 3 FP32 guards above
+// their exact value; with it, as from D/2, 0.03.) The approximate quotients (2
+// ulp) move a step, not where the steps end.
 __device__ __forceinline__ float screen_shifted_f32(const float* G, const float* r, const float* q,
                                                     bool nofit, float guard = 0.0f,
                                                     float thr = __builtin_huge_valf(), bool refine = true) {
@@ -193,19 +200,20 @@ __device__ __forceinline__ float screen_shifted_f32(const float* G, const float*
   // D' = lower-right block of K - tr(S) I
   float d00 = -2.0f * (syy + szz), d11 = -2.0f * (sxx + szz), d22 = -2.0f * (sxx + syy);
   float d01 = 2.0f * sxy, d02 = 2.0f * sxz, d12 = 2.0f * syz;
+  float t = d00 + d11 + d22;
   float beta0 = b0 * b0 + b1 * b1 + b2 * b2;
   float nu_up;
   {
     float g = fmaxf(fmaxf(d00 + fabsf(d01) + fabsf(d02), d11 + fabsf(d01) + fabsf(d12)),
                     d22 + fabsf(d02) + fabsf(d12));
-    nu_up = fmaxf(0.5f * (g + sqrt_approx(fmaf(g, g, 4.0f * beta0))), 0.0f);
+    float root = sqrt_approx(fmaf(g, g, 4.0f * beta0));
+    nu_up = fmaxf(fmaf(4.76837158e-7f, root + fabsf(t), 0.5f * (g + root)), 0.0f);
     float lb = D - 2.0f * nu_up - guard;
     if (lb >= thr) return lb;
   }
   // adjugate of D' (symmetric)
   float a00 = d11 * d22 - d12 * d12, a11 = d00 * d22 - d02 * d02, a22 = d00 * d11 - d01 * d01;
   float a01 = d02 * d12 - d01 * d22, a02 = d01 * d12 - d02 * d11, a12 = d01 * d02 - d00 * d12;
-  float t = d00 + d11 + d22;
   float m2 = a00 + a11 + a22;
   float det = d00 * a00 + d01 * a01 + d02 * a02;
   float Db0 = d00 * b0 + d01 * b1 + d02 * b2;
