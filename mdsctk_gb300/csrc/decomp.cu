@@ -990,9 +990,9 @@ static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, 
     MDS_TRY(h1.alloc(ctx, sizeof(double) * (nlock + m + 1)));
     MDS_TRY(h2.alloc(ctx, sizeof(double) * (nlock + m + 1)));
   } else {
-    static bool attr_done = false;
-    static size_t attr_limit = 0;
-    MDS_TRY(mds_allow_dyn_smem(ctx, k_lz_cycle, &attr_done, &attr_limit));
+    static PerDevice smem_attr;
+    size_t attr_limit = 0;
+    MDS_TRY(mds_allow_dyn_smem(ctx, k_lz_cycle, &smem_attr, &attr_limit));
     const int ncols = nlock + m;
     const size_t fixed = lz_fixed_smem(ncols);
     if (fixed > attr_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "ncv=%d too large", m);

@@ -796,9 +796,9 @@ int launch_screen_tcv(mds_ctx* ctx, const float* Xf, const float* nf, int nfit, 
   MDS_TRY(err.alloc(ctx, 4 * sizeof(int)));
   MDS_CUDA(ctx, cudaMemsetAsync(err.p, 0, 4 * sizeof(int), s));
   const int nst = (Dp <= 64) ? 4 : (Dp <= 96 ? 3 : 2);
-  static bool attr_done = false;
-  static size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_screen_tcv, &attr_done, &attr_limit));
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_screen_tcv, &attr, &attr_limit));
   // threshold heaps of k1 entries per (row, column half) where they fit
   int KH = (k + 1 <= TV_KHMAX) ? (k + 2) / 2 : 0;
   if (KH && tv_smem_bytes(Dp, nst, KH) > attr_limit) KH = 0;

@@ -679,9 +679,9 @@ int launch_screen_fp32(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, cons
                        const float* recf, const float* recr, int nrows, const int* rowlist, int Kp,
                        int nseg, uint64_t* cand, int* cand_n, const Fp32ScreenExtra* extra) {
   size_t smem = screen_fp32_smem(Kp);
-  static bool attr_set = false;  // once: launches may also happen while a stream is captured
-  static size_t limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_screen_fp32, &attr_set, &limit));
+  static PerDevice attr;
+  size_t limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_screen_fp32, &attr, &limit));
   if (smem > limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "screen shared memory %zu > %zu", smem, limit);
   int nrt = (nrows + SC_TM - 1) / SC_TM;
   ctx->stats.launches++;
@@ -1548,9 +1548,9 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
   }
   if (smem > 227 * 1024)
     return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "recheck needs %zu bytes of shared memory (natoms/k too large)", smem);
-  static bool attr_set = false;  // once: launches may also happen while a stream is captured
-  static size_t limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_recheck, &attr_set, &limit));
+  static PerDevice attr;
+  size_t limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_recheck, &attr, &limit));
   if (smem > limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "recheck shared memory %zu > %zu", smem, limit);
   if (nrows <= 0) return MDS_OK;
   const float* recf = audit ? audit->recf : nullptr;
@@ -1561,9 +1561,9 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
   const int* nrows_dev = nullptr;
   int grid = nrows;
   if (rs && rs->panel > 0 && mode == 0 && !rowlist && k + 1 <= RC3_MAXK1 && nseg <= 32) {
-    static bool sums_done = false;
-    static size_t sums_limit = 0;
-    MDS_TRY(mds_allow_dyn_smem(ctx, k_rc_sums, &sums_done, &sums_limit));
+    static PerDevice sums_attr;
+    size_t sums_limit = 0;
+    MDS_TRY(mds_allow_dyn_smem(ctx, k_rc_sums, &sums_attr, &sums_limit));
     MDS_CUDA(ctx, cudaMemsetAsync(rs->nbig.p, 0, sizeof(int), s));
     for (int r0 = 0; r0 < nrows; r0 += rs->panel) {
       const int nr = std::min(rs->panel, nrows - r0), wb = (nr + RC3_WARPS - 1) / RC3_WARPS;
@@ -1628,9 +1628,9 @@ static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af,
   const int ny = std::max(1, std::min(std::min(ntile, 65535), (8 * ctx->num_sms + nrt - 1) / nrt));
   ctx->stats.launches += 2;
   k_row_const<<<nfit, RC_THREADS, 0, ctx->stream>>>(Af, mu, 0, pl.Ap, pl.natoms, pl.nofit, rc.as<float>());
-  static bool attr_done = false;
-  static size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_full_rows, &attr_done, &attr_limit));
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_full_rows, &attr, &attr_limit));
   CUtensorMap mF, mR;
   MDS_TRY(encode_map_f32(ctx, &mF, Af, (int64_t)3 * nfit, pl.Ap, FR_KC, 3 * FR_R));
   MDS_TRY(encode_map_f32(ctx, &mR, Ar, (int64_t)3 * pl.nref, pl.Ap, FR_KC, 3 * FR_C));

@@ -894,11 +894,10 @@ int launch_screen_tc(mds_ctx* ctx, const KnnRmsPlan& pl, const TcOperands& fit, 
   if (nitems <= 0) return MDS_OK;
   const int grid = std::min(nitems, ctx->num_sms);
   const size_t smem = TC_SMEM_BYTES;
-  static bool attr_set = false;  // set once: the call is also made while a stream is being captured
-  if (!attr_set) {
-    MDS_CUDA(ctx, cudaFuncSetAttribute(k_screen_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_screen_tc, &attr, &attr_limit));
+  if (smem > attr_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "screen shared memory %zu > %zu", smem, attr_limit);
   // With an external error flag the caller checks it after the stream is
   // synchronised (the launch can then be captured in a CUDA graph).
   DevBuf err(ctx);

@@ -514,9 +514,9 @@ extern "C" int mds_knn_data_sparse(mds_ctx* ctx, const int64_t* ref_off, const i
   const int W = mds_round_up(std::max(dmax + 1, 1), 32 * BN_KW) / 32;
   if (binary && (size_t)W * 4 * ((size_t)n_ref + (same ? 0 : n_fit)) <= ((size_t)8 << 30)) {
     const size_t bsm = bin_knn_smem(k);
-    static bool bin_done = false;
-    static size_t bin_limit = 0;
-    MDS_TRY(mds_allow_dyn_smem(ctx, k_bin_knn, &bin_done, &bin_limit));
+    static PerDevice bin_attr;
+    size_t bin_limit = 0;
+    MDS_TRY(mds_allow_dyn_smem(ctx, k_bin_knn, &bin_attr, &bin_limit));
     DevBuf br(ctx), bf(ctx), cr(ctx), cf(ctx), bad(ctx);
     MDS_TRY(bad.alloc(ctx, sizeof(int)));
     MDS_CUDA(ctx, cudaMemsetAsync(bad.p, 0, sizeof(int), s));
@@ -604,9 +604,9 @@ extern "C" int mds_knn_data_sparse(mds_ctx* ctx, const int64_t* ref_off, const i
     }
   }
   const size_t smem = sparse_knn_smem(k, mode);
-  static bool attr_done = false;
-  static size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_sparse_knn, &attr_done, &attr_limit));
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_sparse_knn, &attr, &attr_limit));
   if (smem > attr_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "k=%d too large", k);
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
   ctx->stats.launches = 1;

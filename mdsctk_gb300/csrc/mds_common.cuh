@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/mdsgpu.h"
+#include "per_device.h"
 
 #define MDS_MAX_CHUNKS 8  // chunks of a pipelined frame upload
 
@@ -128,12 +129,14 @@ struct DevBuf {
     if (_r != MDS_OK) return _r;   \
   } while (0)
 
-// Let `kernel` use all the dynamic shared memory the device allows next to its
-// static shared memory. Done once per kernel (*done), so that later launches
-// (also those made while a stream is captured) need no attribute call.
+// Let `kernel` use all the dynamic shared memory the context's device (the
+// current one) allows next to its static shared memory; *limit = that size.
+// Done once per kernel and device (`set`, a static of the caller), so that
+// later launches (also those made while a stream is captured) need no
+// attribute call.
 template <class Kernel>
-int mds_allow_dyn_smem(mds_ctx* ctx, Kernel kernel, bool* done, size_t* limit) {
-  if (!*done) {
+int mds_allow_dyn_smem(mds_ctx* ctx, Kernel kernel, PerDevice* set, size_t* limit) {
+  return set->get(ctx->device, limit, [&](size_t* value) -> int {
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return mds_fail(ctx, MDS_ERR_CUDA, "cudaFuncGetAttributes");
     int optin = 0;
@@ -142,10 +145,9 @@ int mds_allow_dyn_smem(mds_ctx* ctx, Kernel kernel, bool* done, size_t* limit) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
     if (e != cudaSuccess)
       return mds_fail(ctx, MDS_ERR_CUDA, "cudaFuncSetAttribute(%d): %s", dyn, cudaGetErrorString(e));
-    *limit = (size_t)dyn;
-    *done = true;
-  }
-  return MDS_OK;
+    *value = (size_t)dyn;
+    return MDS_OK;
+  });
 }
 
 static inline int mds_round_up(int x, int m) { return (x + m - 1) / m * m; }

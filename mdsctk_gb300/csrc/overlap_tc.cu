@@ -421,9 +421,9 @@ int overlap_count_pad(int n) { return mds_round_up(n, OV_N); }
 int launch_rows_e4m3(mds_ctx* ctx, const int64_t* off, const int* idx, const double* val, int n, int64_t K,
                      unsigned char* out, int* cnt, int* bad) {
   const size_t smem = (size_t)std::min<int64_t>(K, OV_ROWCHUNK);
-  static bool attr_done = false;
-  static size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_rows_e4m3, &attr_done, &attr_limit));
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_rows_e4m3, &attr, &attr_limit));
   ctx->stats.launches++;
   k_rows_e4m3<<<n, 256, smem, ctx->stream>>>(off, idx, val, K, out, cnt, bad);
   MDS_CUDA(ctx, cudaGetLastError());
@@ -436,10 +436,10 @@ int overlap_knn(mds_ctx* ctx, const unsigned char* Bf, const int* cf, int nfit, 
   CUtensorMap mA, mB;
   MDS_TRY(ov_map(ctx, &mA, Bf, nfit, K, OV_M));
   MDS_TRY(ov_map(ctx, &mB, Br, nref, K, OV_N));
-  static bool attr_done = false, sel_done = false;
-  static size_t attr_limit = 0, sel_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_overlap, &attr_done, &attr_limit));
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_select_rows, &sel_done, &sel_limit));
+  static PerDevice attr, sel_attr;
+  size_t attr_limit = 0, sel_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_overlap, &attr, &attr_limit));
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_select_rows, &sel_attr, &sel_limit));
   // panels of rows whose distances take about a gigabyte at most
   const int64_t ld = mds_round_up(nref, OV_N);
   int panel = (int)std::max<int64_t>(OV_M, std::min<int64_t>(mds_round_up(nfit, OV_M),

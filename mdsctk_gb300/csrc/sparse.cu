@@ -333,9 +333,9 @@ int radix_sort(mds_ctx* ctx, unsigned long long* k0, int64_t* v0, unsigned long 
   MDS_TRY(hist.alloc(ctx, sizeof(unsigned) * 256 * ((size_t)nblocks + 1)));
   unsigned* tot = hist.as<unsigned>() + (size_t)256 * nblocks;
   const size_t smem = (size_t)RS_TILE * (sizeof(unsigned long long) + sizeof(int64_t));
-  static bool attr_done = false;
-  static size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_rs_scatter, &attr_done, &attr_limit));
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_rs_scatter, &attr, &attr_limit));
   unsigned long long* ka = k0;
   int64_t* va = v0;
   unsigned long long* kb = k1;

@@ -611,9 +611,9 @@ int vec_seed_rows(mds_ctx* ctx, const float* Xr, const int* permr, int nref, con
   if (k1 > 128) return MDS_OK;
   const int ncoltiles = (nref + 127) / 128, nitems = (nfit + 255) / 256;
   const size_t smem = sizeof(float) * ((size_t)128 * (Dp + 1) + 8 * (size_t)Dp);
-  static bool attr_done = false;
-  static size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_vo_seed_rows, &attr_done, &attr_limit));
+  static PerDevice attr;
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, k_vo_seed_rows, &attr, &attr_limit));
   if (smem > attr_limit) return MDS_OK;
   const int parts = std::max(1, std::min(8, 4 * ctx->num_sms / std::max(nitems, 1)));
   k_vo_seed_rows<<<dim3(nitems, parts), 256, smem, ctx->stream>>>(Xr, permr, nref, Xf, permf, nfit, Dp, tdall,
