@@ -211,6 +211,7 @@ struct TcSkip {
   const float* tlo = nullptr;    // [nrowtiles][ncoltiles] bounds of the tiles' pairs, or null
   int piv2 = 0;                  // pivots are the row tiles' (two per column tile)
   const int* far_perm = nullptr; // order of the non-diagonal items, or null
+  int known = 0;                 // pivot pass: pivots whose radii are final (the first ones)
 };
 // The pivots of a reference set (their deviations, records and split
 // operands) and the radii: the middle frame of every column tile (nP = nC),
