@@ -99,9 +99,13 @@ int mds_get_knn_stats(const mds_ctx* ctx, mds_knn_stats* out);
  *   end-of-work marker, so the kernel's bounded waits run out after about a
  *   second; the kernel then releases its resources and reports it, and the
  *   call returns MDS_ERR_TIMEOUT. The context stays usable.
+ *   MDS_INJECT_FULL_STALL: in the next full-matrix launch (sort off) one warp
+ *   of each block gives up on its last chunk as if its wait had run out; the
+ *   call returns MDS_ERR_TIMEOUT.
  * what = 0 disarms.
  */
 #define MDS_INJECT_SCREEN_STALL 0x1u
+#define MDS_INJECT_FULL_STALL 0x2u
 int mds_test_inject(mds_ctx* ctx, unsigned what);
 
 /*

@@ -1326,7 +1326,7 @@ k_rc_finish(const float* __restrict__ rc, const float* __restrict__ Ur, int row0
 __global__ void __launch_bounds__(FR_THREADS, 1)
 k_full_rows(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUtensorMap tmR,
             const float* __restrict__ rc, const float* __restrict__ Ur, int nfit, int Nr, int Ap, int nofit, double* __restrict__ out_d,
-            int* __restrict__ out_i, int* __restrict__ err) {
+            int* __restrict__ out_i, int* __restrict__ err, int stall) {
   extern __shared__ __align__(128) float sm[];
   __shared__ uint64_t full[FR_ST], empty[FR_ST];
   __shared__ int s_abort;
@@ -1381,6 +1381,9 @@ k_full_rows(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUt
         if (ok) load(issued++);
       }
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&full[st], (n / FR_ST) & 1, &s_abort));
+      // (stall: an injected fault for the failure-path tests -- the last warp
+      // gives up on its last chunk, which every other warp still gets)
+      if (stall && warp == FR_THREADS / 32 - 1 && n == total - 1) ok = false;
       if (!ok) break;
       const float* xf = sf + st * FR_STAGE + rp * FR_FS;
       const float* yf = sf + st * FR_STAGE + (FR_R + cp) * FR_FS;
@@ -1433,15 +1436,18 @@ k_full_rows(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUt
     }
     __syncwarp();
   }
-  if (!ok && threadIdx.x == 0) {
+  // every warp reports for itself: the others may have got the chunk it gave up on
+  if (!ok && lane == 0) {
     atomicMax(err, 1);
+    s_abort = 1;
+  }
+  if (!ok && threadIdx.x == 0) {
     // the copies in flight end, or time out, before the block leaves
     for (int x = n; x < issued; ++x) {
       volatile int dummy = 0;
       mbar_wait(&full[x % FR_ST], (x / FR_ST) & 1, &dummy, 50000000ull);
     }
   }
-  if (!ok && lane == 0) s_abort = 1;
   __syncthreads();
 }
 
@@ -1617,12 +1623,11 @@ size_t recheck_scratch_bytes(int nrows) {
 }
 
 // The full matrix of exact distances (rc: the rows' constants, [nfit][24]).
+// *derr (device, zeroed by the caller) is set when a wait timed out.
 static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const float* Ar, const float* mu,
-                            const float* Ur, int nfit, double* out_d, int* out_i) {
-  DevBuf rc(ctx), err(ctx);
+                            const float* Ur, int nfit, double* out_d, int* out_i, int* derr) {
+  DevBuf rc(ctx);
   MDS_TRY(rc.alloc(ctx, sizeof(float) * 24 * (size_t)nfit));
-  MDS_TRY(err.alloc(ctx, sizeof(int)));
-  MDS_CUDA(ctx, cudaMemsetAsync(err.p, 0, sizeof(int), ctx->stream));
   const int nrt = (nfit + FR_R - 1) / FR_R, ntile = (pl.nref + FR_C - 1) / FR_C;
   // column ranges so that there are about 8 blocks per SM
   const int ny = std::max(1, std::min(std::min(ntile, 65535), (8 * ctx->num_sms + nrt - 1) / nrt));
@@ -1634,13 +1639,11 @@ static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af,
   CUtensorMap mF, mR;
   MDS_TRY(encode_map_f32(ctx, &mF, Af, (int64_t)3 * nfit, pl.Ap, FR_KC, 3 * FR_R));
   MDS_TRY(encode_map_f32(ctx, &mR, Ar, (int64_t)3 * pl.nref, pl.Ap, FR_KC, 3 * FR_C));
+  const int stall = (ctx->inject & MDS_INJECT_FULL_STALL) ? 1 : 0;
+  ctx->inject &= ~MDS_INJECT_FULL_STALL;
   k_full_rows<<<dim3(nrt, ny), FR_THREADS, FR_SMEM, ctx->stream>>>(mF, mR, rc.as<float>(), Ur, nfit, pl.nref, pl.Ap,
-                                                                   pl.nofit, out_d, out_i, err.as<int>());
+                                                                   pl.nofit, out_d, out_i, derr, stall);
   MDS_CUDA(ctx, cudaGetLastError());
-  int herr = 0;
-  MDS_CUDA(ctx, cudaMemcpyAsync(&herr, err.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  MDS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (herr) return mds_fail(ctx, MDS_ERR_TIMEOUT, "full matrix: a bounded wait timed out");
   return MDS_OK;
 }
 
@@ -1713,8 +1716,8 @@ struct RmsStatus {
   unsigned long long ntiles;    // tiles the screen computed
   int nflag;                    // flagged rows
   int bad[2];                   // smallest frame with a non-finite coordinate (reference set, fit set)
-  // error words of the tensor-core launches: [0..1] the pivot pass, [2..3]
-  // the screen, then two per staged chunk's pivot pass
+  // error words of the tensor-core launches: [0..1] the pivot pass (or the
+  // full matrix), [2..3] the screen, then two per staged chunk's pivot pass
   int tcerr[4 + 2 * MDS_MAX_CHUNKS];
 };
 
@@ -1898,20 +1901,20 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   }
   if (pl.full) {
     MDS_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
-    MDS_TRY(launch_full_rows(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, dout_d, dout_i));
+    MDS_TRY(launch_full_rows(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, dout_d, dout_i, dst->tcerr));
     MDS_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
-    int hbad[2] = {0, 0};
-    MDS_CUDA(ctx, cudaMemcpyAsync(hbad, dst->bad, sizeof(hbad), cudaMemcpyDeviceToHost, s));
+    MDS_CUDA(ctx, cudaMemcpyAsync(&hst, dst, sizeof(hst), cudaMemcpyDeviceToHost, s));
     MDS_CUDA(ctx, cudaEventSynchronize(ctx->ev[2]));
     MDS_CUDA(ctx, cudaStreamSynchronize(s));
     float ms = 0;
     cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
     st.recheck_ms = ms;
     st.passes = 0;
-    if (hbad[0] != 0x7f7f7f7f)
-      return mds_fail(ctx, MDS_ERR_ARG, "reference frame %d has a non-finite coordinate", hbad[0]);
-    if (hbad[1] != 0x7f7f7f7f)
-      return mds_fail(ctx, MDS_ERR_ARG, "fit frame %d has a non-finite coordinate", hbad[1]);
+    if (hst.tcerr[0]) return mds_fail(ctx, MDS_ERR_TIMEOUT, "full matrix: a bounded wait timed out");
+    if (hst.bad[0] != 0x7f7f7f7f)
+      return mds_fail(ctx, MDS_ERR_ARG, "reference frame %d has a non-finite coordinate", hst.bad[0]);
+    if (hst.bad[1] != 0x7f7f7f7f)
+      return mds_fail(ctx, MDS_ERR_ARG, "fit frame %d has a non-finite coordinate", hst.bad[1]);
     return MDS_OK;
   }
   // tensor-core operands (split hi/lo), when that screen is selected

@@ -1,0 +1,28 @@
+"""Bounded device waits that run out, in forms that fault or hang nothing
+(mds_test_inject): the call reports MDS_ERR_TIMEOUT and the same context then
+computes the same result as before."""
+import numpy as np
+import pytest
+
+from mdsctk_gb300 import _lib as L
+from mdsctk_gb300 import synth
+
+
+def _expect_timeout(ctx, what, call):
+    L.check(ctx.h, ctx._lib.mds_test_inject(ctx.h, what))
+    with pytest.raises(L.MdsError) as e:
+        call()
+    assert e.value.code == L.MDS_ERR_TIMEOUT, e.value
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,atoms", [(8, 20), (100, 200)])
+def test_full_matrix_reports_any_warp(ctx, n, atoms):
+    """One warp gives up on a chunk that every other warp still gets: the
+    rows it leaves out must not be returned as if they were there."""
+    x = synth.trajectory(n, atoms, seed=n)
+    m = synth.uniform_masses(atoms)
+    d0, i0 = ctx.knn_rms(x, None, m, 0, sort=False)
+    _expect_timeout(ctx, L.MDS_INJECT_FULL_STALL, lambda: ctx.knn_rms(x, None, m, 0, sort=False))
+    d1, i1 = ctx.knn_rms(x, None, m, 0, sort=False)
+    assert np.array_equal(d0, d1) and np.array_equal(i0, i1)
