@@ -667,13 +667,11 @@ extern "C" int mds_contact_profile(mds_ctx* ctx, const float* xyz, int nframes, 
   MDS_CUDA(ctx, cudaMemcpyAsync(dg1.p, g1, sizeof(int) * n1, cudaMemcpyHostToDevice, s));
   MDS_CUDA(ctx, cudaMemcpyAsync(dg2.p, g2, sizeof(int) * n2, cudaMemcpyHostToDevice, s));
   const int words = (int)(((int64_t)n1 * n2 + 31) / 32);
-  // the masks of all frames where they take at most a gigabyte (else they are
-  // made for as many frames at a time as fit, once the offsets are known)
+  // the masks of all frames where they take at most a gigabyte and fit (else
+  // they are made for as many frames at a time as do, once the offsets are known)
   DevBuf mask(ctx);
-  int at_once = idx ? (int)std::min<int64_t>(nframes, std::max<int64_t>(1, ((int64_t)1 << 28) / words)) : 0;
-  while (at_once > 1 && mask.alloc(ctx, sizeof(unsigned) * (size_t)words * at_once) != MDS_OK) at_once /= 2;
-  if (at_once == 1) MDS_TRY(mask.alloc(ctx, sizeof(unsigned) * (size_t)words));
-  const bool all = at_once == nframes;
+  int at_once = (int)std::min<int64_t>(nframes, std::max<int64_t>(1, ((int64_t)1 << 28) / words));
+  bool all = idx && at_once == nframes && mask.alloc(ctx, sizeof(unsigned) * (size_t)words * nframes) == MDS_OK;
   k_contact_mask<<<nframes, SP_THREADS, 0, s>>>(dx.as<float>(), natoms, dg1.as<int>(), n1, dg2.as<int>(), n2, eps,
                                                 words, all ? mask.as<unsigned>() : nullptr, dcnt.as<int64_t>());
   MDS_CUDA(ctx, cudaGetLastError());
@@ -687,8 +685,23 @@ extern "C" int mds_contact_profile(mds_ctx* ctx, const float* xyz, int nframes, 
     return mds_fail(ctx, MDS_ERR_ARG, "index buffer holds %lld entries, %lld needed", (long long)idx_cap,
                     (long long)total);
   if (total == 0) return MDS_OK;
-  MDS_TRY(doff.alloc(ctx, sizeof(int64_t) * (nframes + 1)));
-  MDS_TRY(didx.alloc(ctx, sizeof(int) * total));
+  // the masks give way to the indices, and take what these leave
+  auto alloc_lists = [&]() -> int {
+    MDS_TRY(doff.alloc(ctx, sizeof(int64_t) * (nframes + 1)));
+    return didx.alloc(ctx, sizeof(int) * total);
+  };
+  int rc = alloc_lists();
+  if (rc == MDS_ERR_NOMEM && all) {
+    mask.release();
+    mds_trim_cache(ctx, 0);
+    all = false;
+    rc = alloc_lists();
+  }
+  MDS_TRY(rc);
+  if (!all) {
+    while (at_once > 1 && mask.alloc(ctx, sizeof(unsigned) * (size_t)words * at_once) != MDS_OK) at_once /= 2;
+    if (at_once == 1) MDS_TRY(mask.alloc(ctx, sizeof(unsigned) * (size_t)words));
+  }
   MDS_CUDA(ctx, cudaMemcpyAsync(doff.p, offsets, sizeof(int64_t) * (nframes + 1), cudaMemcpyHostToDevice, s));
   for (int f0 = 0; f0 < nframes; f0 += at_once) {
     const int nf = std::min(at_once, nframes - f0);
