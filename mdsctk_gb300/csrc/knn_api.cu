@@ -159,7 +159,20 @@ static int knn_rms_impl(mds_ctx* ctx, const float* ref_xyz, int n_ref, const flo
   for (int a = 0; a < natoms; ++a)
     if (!(hmass[a] >= 0.f) || !std::isfinite(hmass[a]))
       return mds_fail(ctx, MDS_ERR_ARG, "mass[%d] is negative or not finite", a);
-  MDS_TRY(knn_rms_run(ctx, pl, pref, fit_xyz ? pfit : nullptr, hmass.data(), pd, pi));
+  int rc = knn_rms_run(ctx, pl, pref, fit_xyz ? pfit : nullptr, hmass.data(), pd, pi);
+  if (rc == MDS_ERR_NOMEM && !full) {
+    // What the screen's and the recheck's faster paths take beside the frames
+    // (several lists a row, bounds to the pivots, the recheck's stages) did not
+    // fit: the same result with the least that one needs.
+    mds_trim_cache(ctx, 0);
+    const long long pairs = ctx->stats.pairs;
+    ctx->stats = mds_knn_stats{};
+    ctx->stats.pairs = pairs;
+    ctx->stats.kprime = pl.kprime;
+    pl.lean = pl.noskip = 1;
+    rc = knn_rms_run(ctx, pl, pref, fit_xyz ? pfit : nullptr, hmass.data(), pd, pi);
+  }
+  MDS_TRY(rc);
   if (!dev && !hooks.screen_keys && !hooks.prep_dev) {
     MDS_CUDA(ctx, cudaMemcpyAsync(out_d, pd, sizeof(double) * width * n_fit, cudaMemcpyDeviceToHost, s));
     MDS_CUDA(ctx, cudaMemcpyAsync(out_i, pi, sizeof(int) * width * n_fit, cudaMemcpyDeviceToHost, s));

@@ -26,6 +26,7 @@ struct KnnRmsPlan {
   int kprime = 0;  // candidates kept per row by the screen
   int nofit = 0, full = 0;
   int noskip = 0;  // MDS_NO_SKIP: the tensor-core screen computes every tile
+  int lean = 0;    // least workspace: one column segment, recheck by blocks
   unsigned prec = MDS_PREC_FP32;
   float guard_fp32 = 0.f;  // lower-bound margin per unit of |a_i|^2+|a_j|^2
   float guard_tc = 0.f;

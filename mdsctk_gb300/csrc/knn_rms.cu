@@ -1602,21 +1602,21 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
 
 int recheck_scratch(mds_ctx* ctx, int nrows, RecheckScratch& rs) {
   int panel = std::max(1, std::min(nrows, 16384));  // 100 MB: the pairs' sums stay in L2
-  while (true) {
+  rs.panel = 0;
+  if (rs.big.alloc(ctx, sizeof(int) * (size_t)std::max(nrows, 1)) != MDS_OK || rs.nbig.alloc(ctx, sizeof(int)) != MDS_OK)
+    return MDS_OK;
+  for (; panel > 0; panel = panel > 256 ? panel / 4 : 0) {
     const size_t slots = (size_t)panel * RC3_CAP;
     if (rs.rc.alloc(ctx, sizeof(float) * 24 * (size_t)panel) == MDS_OK &&
         rs.meta.alloc(ctx, sizeof(int4) * (size_t)panel) == MDS_OK &&
         rs.cidx.alloc(ctx, sizeof(int) * slots) == MDS_OK && rs.cbound.alloc(ctx, sizeof(float) * slots) == MDS_OK &&
-        rs.sums.alloc(ctx, sizeof(float) * 10 * slots) == MDS_OK)
-      break;
-    rs.panel = 0;
-    if (panel <= 256) return MDS_OK;  // (a small HBM budget: the block kernel takes every row)
-    panel /= 4;
+        rs.sums.alloc(ctx, sizeof(float) * 10 * slots) == MDS_OK) {
+      rs.panel = panel;
+      return MDS_OK;
+    }
+    for (DevBuf* b : {&rs.rc, &rs.meta, &rs.cidx, &rs.cbound, &rs.sums}) b->release();
   }
-  MDS_TRY(rs.big.alloc(ctx, sizeof(int) * (size_t)std::max(nrows, 1)));
-  MDS_TRY(rs.nbig.alloc(ctx, sizeof(int)));
-  rs.panel = panel;
-  return MDS_OK;
+  return MDS_OK;  // (a small HBM budget: the block kernel takes every row)
 }
 size_t recheck_scratch_bytes(int nrows) {
   return (size_t)std::min(nrows, 16384) * (96 + 16 + RC3_CAP * 48) + sizeof(int) * (size_t)nrows + 4096;
@@ -1626,24 +1626,33 @@ size_t recheck_scratch_bytes(int nrows) {
 // *derr (device, zeroed by the caller) is set when a wait timed out.
 static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const float* Ar, const float* mu,
                             const float* Ur, int nfit, double* out_d, int* out_i, int* derr) {
+  // all rows at once, or as many as the constants' memory allows
   DevBuf rc(ctx);
-  MDS_TRY(rc.alloc(ctx, sizeof(float) * 24 * (size_t)nfit));
-  const int nrt = (nfit + FR_R - 1) / FR_R, ntile = (pl.nref + FR_C - 1) / FR_C;
-  // column ranges so that there are about 8 blocks per SM
-  const int ny = std::max(1, std::min(std::min(ntile, 65535), (8 * ctx->num_sms + nrt - 1) / nrt));
-  ctx->stats.launches += 2;
-  k_row_const<<<nfit, RC_THREADS, 0, ctx->stream>>>(Af, mu, 0, pl.Ap, pl.natoms, pl.nofit, rc.as<float>());
+  int panel = nfit;
+  while (rc.alloc(ctx, sizeof(float) * 24 * (size_t)panel) != MDS_OK) {
+    if (panel <= FR_R) return MDS_ERR_NOMEM;
+    panel = (panel / 2 + FR_R - 1) / FR_R * FR_R;
+  }
+  const int ntile = (pl.nref + FR_C - 1) / FR_C;
   static PerDevice attr;
   size_t attr_limit = 0;
   MDS_TRY(mds_allow_dyn_smem(ctx, k_full_rows, &attr, &attr_limit));
   CUtensorMap mF, mR;
-  MDS_TRY(encode_map_f32(ctx, &mF, Af, (int64_t)3 * nfit, pl.Ap, FR_KC, 3 * FR_R));
   MDS_TRY(encode_map_f32(ctx, &mR, Ar, (int64_t)3 * pl.nref, pl.Ap, FR_KC, 3 * FR_C));
   const int stall = (ctx->inject & MDS_INJECT_FULL_STALL) ? 1 : 0;
   ctx->inject &= ~MDS_INJECT_FULL_STALL;
-  k_full_rows<<<dim3(nrt, ny), FR_THREADS, FR_SMEM, ctx->stream>>>(mF, mR, rc.as<float>(), Ur, nfit, pl.nref, pl.Ap,
-                                                                   pl.nofit, out_d, out_i, derr, stall);
-  MDS_CUDA(ctx, cudaGetLastError());
+  for (int r0 = 0; r0 < nfit; r0 += panel) {
+    const int nr = std::min(panel, nfit - r0), nrt = (nr + FR_R - 1) / FR_R;
+    // column ranges so that there are about 8 blocks per SM
+    const int ny = std::max(1, std::min(std::min(ntile, 65535), (8 * ctx->num_sms + nrt - 1) / nrt));
+    MDS_TRY(encode_map_f32(ctx, &mF, Af + (int64_t)r0 * 3 * pl.Ap, (int64_t)3 * nr, pl.Ap, FR_KC, 3 * FR_R));
+    ctx->stats.launches += 2;
+    k_row_const<<<nr, RC_THREADS, 0, ctx->stream>>>(Af, mu, r0, pl.Ap, pl.natoms, pl.nofit, rc.as<float>());
+    k_full_rows<<<dim3(nrt, ny), FR_THREADS, FR_SMEM, ctx->stream>>>(
+        mF, mR, rc.as<float>(), Ur, nr, pl.nref, pl.Ap, pl.nofit, out_d + (int64_t)r0 * pl.nref,
+        out_i + (int64_t)r0 * pl.nref, derr, stall);
+    MDS_CUDA(ctx, cudaGetLastError());
+  }
   return MDS_OK;
 }
 
@@ -1936,7 +1945,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       nseg = std::min(std::max(nseg, (24 * ctx->num_sms + nrt - 1) / nrt), std::min(8, nct));
     }
   }
-  if (pl.screen_keys) nseg = 1;
+  if (pl.screen_keys || pl.lean) nseg = 1;
   DevBuf cand(ctx), cand_n(ctx), rows(ctx);
   const int segstride = (pl.prec == MDS_PREC_FP32) ? Kp : tc_seg_stride();
   if (nseg > 8 && cand.alloc(ctx, sizeof(uint64_t) * (size_t)nfit * nseg * segstride) != MDS_OK)
@@ -2064,7 +2073,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   audit.guard = (pl.prec == MDS_PREC_FP32) ? pl.guard_fp32 : pl.guard_tc;
   audit.counters = dst->audit;
   RecheckScratch rs;
-  MDS_TRY(recheck_scratch(ctx, nfit, rs));
+  if (!pl.lean) MDS_TRY(recheck_scratch(ctx, nfit, rs));
   MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, nullptr, 0,
                          cand.as<uint64_t>(), cand_n.as<int>(), nseg, segstride, Kp, k, dout_d, dout_i,
                          flagged.as<int>(), &dst->nflag, rowthr.p ? rowthr.as<float>() : nullptr, &audit, 0,
