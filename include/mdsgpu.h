@@ -102,10 +102,13 @@ int mds_get_knn_stats(const mds_ctx* ctx, mds_knn_stats* out);
  *   MDS_INJECT_FULL_STALL: in the next full-matrix launch (sort off) one warp
  *   of each block gives up on its last chunk as if its wait had run out; the
  *   call returns MDS_ERR_TIMEOUT.
+ *   MDS_INJECT_OVERLAP_STALL: the next tensor-core product of binary vectors
+ *   leaves out a load, so its bounded waits run out; MDS_ERR_TIMEOUT.
  * what = 0 disarms.
  */
 #define MDS_INJECT_SCREEN_STALL 0x1u
 #define MDS_INJECT_FULL_STALL 0x2u
+#define MDS_INJECT_OVERLAP_STALL 0x4u
 int mds_test_inject(mds_ctx* ctx, unsigned what);
 
 /*

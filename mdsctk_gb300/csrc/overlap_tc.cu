@@ -106,7 +106,7 @@ __device__ __forceinline__ int2 ov_tile(int item, int nrt, int nct) {
 __global__ void __launch_bounds__(OV_THREADS, 1)
 k_overlap(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const int* __restrict__ cf,
           const int* __restrict__ cr, int row0, int nrows, int nref, int nkb, uint32_t idesc, int64_t ld,
-          unsigned* __restrict__ out, int* __restrict__ err) {
+          unsigned* __restrict__ out, int* __restrict__ err, int stall) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   unsigned char* stages = smem_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -148,10 +148,14 @@ k_overlap(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             ok = false;
             break;
           }
-          unsigned char* st = stages + stage * OV_STAGE_BYTES;
-          mbar_expect_tx(&S->full[stage], OV_STAGE_BYTES);
-          tma_load_2d(st, &tmA, &S->full[stage], kb * OV_KB, row0 + t.x * OV_M);
-          tma_load_2d(st + OV_A_BYTES, &tmB, &S->full[stage], kb * OV_KB, t.y * OV_N);
+          // (stall: an injected fault for the failure-path tests -- the first
+          // K-block is not loaded, so the MMA thread's wait for it runs out)
+          if (!stall || kb > 0 || item >= (int)gridDim.x) {
+            unsigned char* st = stages + stage * OV_STAGE_BYTES;
+            mbar_expect_tx(&S->full[stage], OV_STAGE_BYTES);
+            tma_load_2d(st, &tmA, &S->full[stage], kb * OV_KB, row0 + t.x * OV_M);
+            tma_load_2d(st + OV_A_BYTES, &tmB, &S->full[stage], kb * OV_KB, t.y * OV_N);
+          }
           if (++stage == OV_STAGES) {
             stage = 0;
             phase ^= 1;
@@ -305,16 +309,18 @@ k_select_rows(const unsigned* __restrict__ d2, int64_t ld, int row0, int nref, i
     hi = max(hi, wb[w]);
   }
   const unsigned* v = staged ? row_s : g;
-  unsigned base = lo, less = 0;  // the (k+1)-th value lies in [base, base + span); `less` values below base
-  unsigned span = hi - lo + 1;
+  // the (k+1)-th value lies in [base, base + width]; `less` values below base
+  // (an inclusive width: the panel of a product that timed out holds anything,
+  // and the counts have to be right for any values, since they place the writes)
+  unsigned base = lo, less = 0, width = hi - lo;
   while (true) {
     int sh = 0;
-    while (((span - 1) >> sh) >= OV_BINS) ++sh;
+    while ((width >> sh) >= OV_BINS) ++sh;
     for (int i = tid; i < OV_BINS; i += OV_SEL_THREADS) hist[i] = 0;
     __syncthreads();
     for (int j = tid; j < nref; j += OV_SEL_THREADS) {
       const unsigned x = v[j] - base;
-      if (v[j] >= base && x < span) atomicAdd(&hist[x >> sh], 1u);
+      if (v[j] >= base && x <= width) atomicAdd(&hist[x >> sh], 1u);
     }
     __syncthreads();
     // bins 16 t .. 16 t + 15 by thread t
@@ -345,7 +351,7 @@ k_select_rows(const unsigned* __restrict__ d2, int64_t ld, int row0, int nref, i
     base += s_bin << sh;
     less = s_less;
     if (sh == 0) break;
-    span = 1u << sh;
+    width = (1u << sh) - 1;
     __syncthreads();
   }
   const unsigned vk = base;            // the (k+1)-th smallest value
@@ -456,12 +462,14 @@ int overlap_knn(mds_ctx* ctx, const unsigned char* Bf, const int* cf, int nfit, 
   const bool staged = fixed + sizeof(unsigned) * (size_t)nref <= 100 * 1024;
   const size_t sel_smem = fixed + (staged ? sizeof(unsigned) * (size_t)nref : 0);
   if (sel_smem > sel_limit) return mds_fail(ctx, MDS_ERR_UNSUPPORTED, "k=%d too large", k);
+  const int stall = (ctx->inject & MDS_INJECT_OVERLAP_STALL) ? 1 : 0;
+  ctx->inject &= ~MDS_INJECT_OVERLAP_STALL;
   for (int r0 = 0; r0 < nfit; r0 += panel) {
     const int nr = std::min(panel, nfit - r0);
     const int grid = std::min(overlap_tiles(nr, nref), ctx->num_sms);
     ctx->stats.launches += 2;
     k_overlap<<<grid, OV_THREADS, OV_SMEM, s>>>(mA, mB, cf, cr, r0, nr, nref, (int)(K / OV_KB),
-                                                umma_idesc_e4m3(OV_M, OV_N), ld, d2.as<unsigned>(), err.as<int>());
+                                                umma_idesc_e4m3(OV_M, OV_N), ld, d2.as<unsigned>(), err.as<int>(), stall);
     k_select_rows<<<nr, OV_SEL_THREADS, sel_smem, s>>>(d2.as<unsigned>(), ld, r0, nref, k, staged ? 1 : 0, out_d,
                                                        out_i);
     MDS_CUDA(ctx, cudaGetLastError());

@@ -26,3 +26,16 @@ def test_full_matrix_reports_any_warp(ctx, n, atoms):
     _expect_timeout(ctx, L.MDS_INJECT_FULL_STALL, lambda: ctx.knn_rms(x, None, m, 0, sort=False))
     d1, i1 = ctx.knn_rms(x, None, m, 0, sort=False)
     assert np.array_equal(d0, d1) and np.array_equal(i0, i1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim", [100, 5000])  # one K-block of a row, and more than the pipeline's stages
+def test_binary_product_times_out(ctx, dim):
+    r = np.random.default_rng(dim)
+    idx = np.sort(np.stack([r.choice(dim, 20, replace=False) for _ in range(2300)]), axis=1).astype(np.int32)
+    a = (np.arange(2301, dtype=np.int64) * 20, idx.ravel(), np.ones(idx.size))
+    d0, i0 = ctx.knn_data_sparse(a, None, 12)
+    assert ctx.stats()["launches"] == 3
+    _expect_timeout(ctx, L.MDS_INJECT_OVERLAP_STALL, lambda: ctx.knn_data_sparse(a, None, 12))
+    d1, i1 = ctx.knn_data_sparse(a, None, 12)
+    assert np.array_equal(d0, d1) and np.array_equal(i0, i1)
