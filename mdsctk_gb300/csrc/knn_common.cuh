@@ -154,11 +154,14 @@ struct RecheckScratch {
 };
 int recheck_scratch(mds_ctx* ctx, int nrows, RecheckScratch& rs);
 size_t recheck_scratch_bytes(int nrows);
+// serr (optional): the error word of the screen that made the lists. When a
+// wait of it ran out the lists are not all written; then nothing is rechecked
+// (the caller reports the error).
 int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const float* Ar, const float* mu,
                    const float* Ur, int nrows, const int* rowlist, int mode, const uint64_t* cand,
                    const int* cand_n, int nseg, int segstride, int Kp, int k, double* out_d, int* out_i,
                    int* flagged, int* nflag, const float* rowthr = nullptr, const RecheckAudit* audit = nullptr,
-                   int cand_by_row = 0, RecheckScratch* rs = nullptr);
+                   int cand_by_row = 0, RecheckScratch* rs = nullptr, const int* serr = nullptr);
 
 int choose_nseg_fp32(int nfit, int num_sms, int nref, int Kp, bool same);
 

@@ -914,7 +914,7 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
           double* __restrict__ out_d, int* __restrict__ out_i, int* __restrict__ flagged, int* __restrict__ nflag,
           const float* __restrict__ rowthr, const float* __restrict__ recf, const float* __restrict__ recr,
           float guard, unsigned long long* __restrict__ audit, int cand_by_row,
-          const int* __restrict__ nrows_dev) {
+          const int* __restrict__ nrows_dev, const int* __restrict__ serr) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* sa = reinterpret_cast<float*>(smem_raw);                 // [3*Ap] a_i
   float* sd = sa + 3 * Ap;                                        // [CHUNK]
@@ -927,6 +927,7 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
   __shared__ float ui[18];                              // the row's U as double-float pairs
   __shared__ float redu[(RC_THREADS / 32) * 18];
 
+  if (serr && __ldcg(serr)) return;  // (the lists are not all written)
   if (nrows_dev) nrows = min(nrows, *nrows_dev);
   for (int lr = blockIdx.x; lr < nrows; lr += gridDim.x) {
   __syncthreads();  // (the row before is done with the shared memory)
@@ -1103,11 +1104,16 @@ __device__ __forceinline__ void rc_sort_write(uint64_t* buf, int m, int Kp, floa
 __global__ void __launch_bounds__(RC3_WARPS * 32)
 k_rc_cands(const uint64_t* __restrict__ cand, const int* __restrict__ cand_n, int row0, int rows, int nseg,
            int segstride, int Kp, int k1, const float* __restrict__ rowthr, int* __restrict__ cidx,
-           float* __restrict__ cbound, int4* __restrict__ meta, int* __restrict__ big, int* __restrict__ nbig) {
+           float* __restrict__ cbound, int4* __restrict__ meta, int* __restrict__ big, int* __restrict__ nbig,
+           const int* __restrict__ serr) {
   __shared__ uint64_t s_buf[RC3_WARPS][RC3_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int rl = blockIdx.x * RC3_WARPS + w;
   if (rl >= rows) return;
+  if (serr && __ldcg(serr)) {  // (the lists are not all written: no candidates, no row for k_recheck)
+    if (lane == 0) meta[rl] = make_int4(-1, 0, 0, 0);
+    return;
+  }
   const int row = row0 + rl;
   uint64_t* buf = s_buf[w];
   const int segn = (lane < nseg) ? min(cand_n[(int64_t)row * nseg + lane], Kp) : 0;
@@ -1542,7 +1548,7 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
                    const float* Ur, int nrows, const int* rowlist, int mode,
                    const uint64_t* cand, const int* cand_n, int nseg, int segstride, int Kp, int k,
                    double* out_d, int* out_i, int* flagged, int* nflag, const float* rowthr,
-                   const RecheckAudit* audit, int cand_by_row, RecheckScratch* rs) {
+                   const RecheckAudit* audit, int cand_by_row, RecheckScratch* rs, const int* serr) {
   size_t smem = recheck_smem(pl.Ap, Kp, k, mode);
   if (mode == 0) {
     // the streaming merge works on the best K' plus one segment's K'
@@ -1577,7 +1583,7 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
       k_row_const<<<nr, RC_THREADS, 0, s>>>(Af, mu, r0, pl.Ap, pl.natoms, pl.nofit, rs->rc.as<float>());
       k_rc_cands<<<wb, RC3_WARPS * 32, 0, s>>>(cand, cand_n, r0, nr, nseg, segstride, Kp, k + 1, rowthr,
                                                rs->cidx.as<int>(), rs->cbound.as<float>(), rs->meta.as<int4>(),
-                                               rs->big.as<int>(), rs->nbig.as<int>());
+                                               rs->big.as<int>(), rs->nbig.as<int>(), serr);
       k_rc_sums<<<nr, RC_THREADS, sizeof(float) * 3 * pl.Ap, s>>>(
           Af, Ar, r0, pl.Ap, pl.nofit, rs->cidx.as<int>(), rs->meta.as<int4>(), rs->sums.as<float>());
       k_rc_finish<<<wb, RC3_WARPS * 32, 0, s>>>(rs->rc.as<float>(), Ur, r0, nr, pl.nofit, k, rs->cidx.as<int>(),
@@ -1595,7 +1601,7 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
   ctx->stats.launches++;
   k_recheck<<<grid, RC_THREADS, smem, s>>>(Af, Ar, mu, Ur, nrows, rowlist, pl.nref, pl.Ap, pl.natoms, pl.nofit, mode,
                                            cand, cand_n, nseg, segstride, Kp, k, out_d, out_i, flagged, nflag, rowthr,
-                                           recf, recr, guard, counters, cand_by_row, nrows_dev);
+                                           recf, recr, guard, counters, cand_by_row, nrows_dev, serr);
   MDS_CUDA(ctx, cudaGetLastError());
   return MDS_OK;
 }
@@ -2077,7 +2083,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, nullptr, 0,
                          cand.as<uint64_t>(), cand_n.as<int>(), nseg, segstride, Kp, k, dout_d, dout_i,
                          flagged.as<int>(), &dst->nflag, rowthr.p ? rowthr.as<float>() : nullptr, &audit, 0,
-                         &rs));
+                         &rs, dst->tcerr + 2));
   MDS_CUDA(ctx, cudaEventRecord(ctx->ev[3], s));
   MDS_CUDA(ctx, cudaMemcpyAsync(&hst, dst, sizeof(hst), cudaMemcpyDeviceToHost, s));
   MDS_CUDA(ctx, cudaStreamSynchronize(s));

@@ -250,7 +250,8 @@ static int launch_batch(mds_server* S, Slot& sl, int bucket) {
   MDS_TRY(launch_recheck(c, pl, sl.A.as<float>(), S->A.as<float>(), S->dmu.as<float>(), S->U.as<float>(), bucket,
                          nullptr, 0, sl.cand.as<uint64_t>(), sl.cand_n.as<int>(), nseg, segstride, S->Kp, S->k,
                          sl.out_d.as<double>(), sl.out_i.as<int>(), sl.flagged.as<int>(), sl.nflag.as<int>(),
-                         S->prec == MDS_PREC_FP32 ? nullptr : sl.rowthr.as<float>(), &audit, 0, &sl.rs));
+                         S->prec == MDS_PREC_FP32 ? nullptr : sl.rowthr.as<float>(), &audit, 0, &sl.rs,
+                         sl.derr.as<int>()));
   c->stats.launches++;
   k_serve_ext<<<(bucket + SE_WARPS - 1) / SE_WARPS, SE_WARPS * 32, serve_ext_smem(S->k), c->stream>>>(
       sl.out_d.as<double>(), sl.out_i.as<int>(), bucket, S->k, S->cfg.sigma, S->ddinv.as<double>(),

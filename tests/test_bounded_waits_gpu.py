@@ -39,3 +39,27 @@ def test_binary_product_times_out(ctx, dim):
     _expect_timeout(ctx, L.MDS_INJECT_OVERLAP_STALL, lambda: ctx.knn_data_sparse(a, None, 12))
     d1, i1 = ctx.knn_data_sparse(a, None, 12)
     assert np.array_equal(d0, d1) and np.array_equal(i0, i1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [10, 200])  # the recheck in stages; the block kernel alone
+@pytest.mark.parametrize("n", [200, 2000])
+def test_no_recheck_of_a_screen_that_timed_out(ctx, n, k):
+    """A screen that gave up leaves lists unwritten: whatever they hold, the
+    recheck must not follow their indices. Seen from the result arrays, which
+    stay as they were."""
+    import torch
+
+    x = torch.from_numpy(synth.trajectory(n, 96, seed=90 + n, basins=2, dwell=100)).cuda()
+    m = torch.ones(96, device="cuda")
+    kk = min(k, n - 1)
+    d0, i0 = (t.clone() for t in ctx.knn_rms(x, None, m, k, precision="bf16x3"))
+    out = (torch.full((n, kk), -7.0, dtype=torch.float64, device="cuda"),
+           torch.full((n, kk), -7, dtype=torch.int32, device="cuda"))
+    # (skip=False: no pivot pass, which would take the fault)
+    call = lambda: ctx.knn_rms(x, None, m, k, precision="bf16x3", out=out, skip=False)
+    torch.cuda.synchronize()
+    _expect_timeout(ctx, L.MDS_INJECT_SCREEN_STALL, call)
+    assert bool((out[0] == -7).all()) and bool((out[1] == -7).all())
+    d1, i1 = call()
+    assert torch.equal(d0, d1) and torch.equal(i0, i1)
