@@ -104,11 +104,14 @@ int mds_get_knn_stats(const mds_ctx* ctx, mds_knn_stats* out);
  *   call returns MDS_ERR_TIMEOUT.
  *   MDS_INJECT_OVERLAP_STALL: the next tensor-core product of binary vectors
  *   leaves out a load, so its bounded waits run out; MDS_ERR_TIMEOUT.
+ *   MDS_INJECT_LANCZOS_STALL: a block of the next Lanczos cycle does not arrive
+ *   at its grid barrier, whose waits run out; MDS_ERR_TIMEOUT.
  * what = 0 disarms.
  */
 #define MDS_INJECT_SCREEN_STALL 0x1u
 #define MDS_INJECT_FULL_STALL 0x2u
 #define MDS_INJECT_OVERLAP_STALL 0x4u
+#define MDS_INJECT_LANCZOS_STALL 0x8u
 int mds_test_inject(mds_ctx* ctx, unsigned what);
 
 /*

@@ -31,6 +31,7 @@ MDS_NO_SKIP = 0x100
 MDS_INJECT_SCREEN_STALL = 0x1
 MDS_INJECT_FULL_STALL = 0x2
 MDS_INJECT_OVERLAP_STALL = 0x4
+MDS_INJECT_LANCZOS_STALL = 0x8
 
 PRECISIONS = {"fp32": MDS_PREC_FP32, "bf16x3": MDS_PREC_BF16X3, "fp16x3": MDS_PREC_FP16X3}
 

@@ -63,3 +63,17 @@ def test_no_recheck_of_a_screen_that_timed_out(ctx, n, k):
     assert bool((out[0] == -7).all()) and bool((out[1] == -7).all())
     d1, i1 = call()
     assert torch.equal(d0, d1) and torch.equal(i0, i1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [150, 3000])  # two clusters of blocks; most of the device
+def test_lanczos_cycle_times_out(ctx, n):
+    r = np.random.default_rng(n)
+    p = r.uniform(size=(n, 2))
+    d, i = ctx.knn_data(p, None, 10)
+    g = ctx.sysparse(d, i)
+    call = lambda: ctx.decomp_sparse(*g, 0.3, 4)
+    e0, v0, _, _ = call()
+    _expect_timeout(ctx, L.MDS_INJECT_LANCZOS_STALL, call)
+    e1, v1, _, _ = call()
+    assert np.array_equal(e0, e1) and np.array_equal(v0, v1)
