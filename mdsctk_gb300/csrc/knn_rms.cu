@@ -29,6 +29,7 @@
 
 #include "knn_common.cuh"
 #include "qcp.cuh"
+#include "screen_plan.h"
 #include "tc_ptx.cuh"
 #include "warp_sort.cuh"
 
@@ -1059,11 +1060,10 @@ k_recheck(const float* __restrict__ Af, const float* __restrict__ Ar, const floa
 // Rows with more candidates than that whose next bound does not settle them,
 // or with fewer than k+1 below the threshold are listed in big[] for k_recheck.
 // 100,000 x 304, k = 64: 5.37 -> 4.1 ms; 20,000 x 1,000, k = 100: 2.41 -> 2.3
-// ms, outputs bit-identical.
+// ms, outputs bit-identical. Which calls take it: staged_recheck (screen_plan.h).
 #define RC3_CAP 128    // candidates per row (256: the rows with more are rechecked in full, 2.63 against 2.37 ms
                        // at 20,000 x 1,000)
 #define RC3_LIST 512   // keys per row that stage 1 holds (K' <= 448 and one step of 32)
-#define RC3_MAXK1 120  // k + 1 (eight candidates to spare, as the block kernel's first chunk)
 #define RC3_WARPS 8
 
 __global__ void __launch_bounds__(RC_THREADS) k_row_const(const float* __restrict__ Af, const float* __restrict__ mu,
@@ -1572,7 +1572,8 @@ int launch_recheck(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af, const fl
   cudaStream_t s = ctx->stream;
   const int* nrows_dev = nullptr;
   int grid = nrows;
-  if (rs && rs->panel > 0 && mode == 0 && !rowlist && k + 1 <= RC3_MAXK1 && nseg <= 32) {
+  if (rs && rs->panel > 0 && mode == 0 && !rowlist && nseg <= 32 &&
+      staged_recheck(nrows, k, Af == Ar, pl.prec == MDS_PREC_FP32)) {
     static PerDevice sums_attr;
     size_t sums_limit = 0;
     MDS_TRY(mds_allow_dyn_smem(ctx, k_rc_sums, &sums_attr, &sums_limit));
@@ -2079,7 +2080,7 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   audit.guard = (pl.prec == MDS_PREC_FP32) ? pl.guard_fp32 : pl.guard_tc;
   audit.counters = dst->audit;
   RecheckScratch rs;
-  if (!pl.lean) MDS_TRY(recheck_scratch(ctx, nfit, rs));
+  if (!pl.lean && staged_recheck(nfit, k, same, pl.prec == MDS_PREC_FP32)) MDS_TRY(recheck_scratch(ctx, nfit, rs));
   MDS_TRY(launch_recheck(ctx, pl, Afp, Ar.as<float>(), dmu, Ur.as<float>(), nfit, nullptr, 0,
                          cand.as<uint64_t>(), cand_n.as<int>(), nseg, segstride, Kp, k, dout_d, dout_i,
                          flagged.as<int>(), &dst->nflag, rowthr.p ? rowthr.as<float>() : nullptr, &audit, 0,

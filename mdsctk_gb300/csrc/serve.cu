@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "knn_common.cuh"
+#include "screen_plan.h"
 #include "qcp.cuh"
 
 int decomp_resident(mds_ctx* ctx, int n, const int* dpcol, const int* dirow, const double* ddist, double sigma,
@@ -470,7 +471,7 @@ static size_t slot_bytes(const mds_server* S, int cap) {
   b += (size_t)cap * S->nseg_max * S->segstride * 8 + (size_t)cap * S->nseg_max * 4;
   b += (size_t)cap * S->k * 12 + (size_t)cap * S->nev * 8 + (size_t)cap * 4;
   b += (size_t)cap * S->pv.nC * 4;                            // pivot bounds
-  b += recheck_scratch_bytes(cap);
+  if (staged_recheck(cap, S->k, false, S->prec == MDS_PREC_FP32)) b += recheck_scratch_bytes(cap);
   return b + (64u << 20);
 }
 
@@ -614,7 +615,7 @@ extern "C" int mds_server_create(const mds_server_config* cfg, const float* land
               sl.home.alloc(c, sizeof(int) * (cap / TC_FR_M + 1)) == MDS_OK &&
               (S->pv.nC == 0 || sl.lb.alloc(c, sizeof(float) * (size_t)S->pv.nC * cap) == MDS_OK) &&
               sl.ext.alloc(c, sizeof(double) * (size_t)cap * S->nev) == MDS_OK &&
-              recheck_scratch(c, cap, sl.rs) == MDS_OK;
+              (!staged_recheck(cap, S->k, false, S->prec == MDS_PREC_FP32) || recheck_scratch(c, cap, sl.rs) == MDS_OK);
     if (!ok) {
       S->last_error = mds_last_error(c);
       return MDS_ERR_NOMEM;
