@@ -423,7 +423,6 @@ __global__ void __launch_bounds__(128) k_prep_out(const float* __restrict__ raw,
 #define SC_KC 32
 #define SC_FS 98  // floats per frame per stage: 3*32 + 2 (bank spread)
 #define SC_THREADS 256
-#define SC_SKIP_TILES 22  // 80-frame column tiles from which a set against itself skips tiles
 #define SC_STATIC (4 * SC_TM * (MDS_REC + 1) + 1024)  // shared memory besides the dynamic part
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
@@ -1696,23 +1695,6 @@ int launch_prep(mds_ctx* ctx, const float* draw, int n, int natoms, int Ap, cons
   return MDS_OK;
 }
 
-// Segments of nct column tiles for nrt row tiles on `slots` blocks at a time:
-// the fewest (of at most smax) that leave the last wave nearly full.
-static int choose_nseg(int nrt, int slots, int nct, int smax) {
-  int best = 1;
-  double besteff = 0;
-  for (int s = 1; s <= smax && s <= nct; ++s) {
-    double waves = (double)nrt * s / slots;
-    double eff = waves / std::ceil(waves);
-    if (eff > besteff + 0.02) {
-      besteff = eff;
-      best = s;
-    }
-    if (eff >= 0.95) break;
-  }
-  return best;
-}
-
 // Segments of the FP32 screen; two of its blocks share an SM where the lists of
 // K' allow it. The few row tiles of a small fit set take up to 32
 // segments (100 fit frames against 12,000 of 304 atoms, K' = 96: 0.39 ms, 1.49
@@ -1721,7 +1703,8 @@ static int choose_nseg(int nrt, int slots, int nct, int smax) {
 // frames of 60 atoms: 0.18 ms, 0.23 with up to 32).
 int choose_nseg_fp32(int nfit, int num_sms, int nref, int Kp, bool same) {
   const int per_sm = 2 * (screen_fp32_smem(Kp) + SC_STATIC) <= 228 * 1024 ? 2 : 1;
-  return choose_nseg((nfit + SC_TM - 1) / SC_TM, per_sm * num_sms, (nref + SC_TN - 1) / SC_TN, same ? 8 : TC_MAX_SEGS);
+  return choose_segments((nfit + SC_TM - 1) / SC_TM, per_sm * num_sms, (nref + SC_TN - 1) / SC_TN,
+                         same ? 8 : TC_MAX_SEGS);
 }
 
 // Counters and error words of one call, in one device block: one copy sets
@@ -1942,6 +1925,8 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
   // first pass
   int Kp = pl.kprime;
   int nseg = choose_nseg_fp32(nfit, ctx->num_sms, nref, Kp, same);
+  const bool f_skip = !pl.screen_keys && !pl.noskip && same && fp32_skips(nref, natoms, k);  // (FP32 screen)
+  if (f_skip) nseg = fp32_skip_segments((nfit + SC_TM - 1) / SC_TM, ctx->num_sms, natoms, k, nseg);
   if (pl.prec != MDS_PREC_FP32) {
     nseg = tc_choose_nseg(ctx, pl, nfit);
     // A set screened against itself skips most tiles and its items differ
@@ -1981,13 +1966,8 @@ int knn_rms_run(mds_ctx* ctx, KnnRmsPlan& pl, const float* draw_ref, const float
       ex.ntiles = &dst->ntiles;
     }
     ex.diag = same ? 1 : 0;
-    // Below SC_SKIP_TILES column tiles the pivots cost more than the tiles they
-    // save (whole calls, host frames: 1,000 x 60 atoms 307 us with skipping, 265
-    // without; 1,500 x 304 824 / 740; 2,000 x 60 381 / 405; 2,000 x 304 767 /
-    // 1,045).
-    const bool skipping = !keys_only && !pl.noskip && same && (nref + TC_FR_N - 1) / TC_FR_N >= SC_SKIP_TILES;
     st.screen_launches = 1;
-    if (skipping) {
+    if (f_skip) {
       MDS_TRY(tc_skip_pivots(ctx, pl, Ar.as<float>(), Rr.as<float>(), f_pv, true));
       MDS_TRY(f_lb.alloc(ctx, sizeof(float) * (size_t)f_pv.nP * nfit));
       Fp32ScreenExtra dx;

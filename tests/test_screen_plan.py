@@ -27,9 +27,39 @@ def plan(tmp_path_factory):
 @pytest.mark.parametrize("nrows,k,same,fp32,staged", [
     (20000, 100, 1, 0, 1), (3000, 20, 1, 0, 1), (100000, 119, 1, 0, 1), (100000, 120, 1, 0, 0), (1000, 50, 1, 0, 0),
     (600, 20, 0, 0, 0), (600, 110, 0, 0, 0), (2047, 20, 0, 0, 1), (2047, 50, 0, 0, 0), (2047, 100, 0, 0, 0),
-    (10000, 50, 0, 0, 1), (10000, 100, 0, 0, 0), (3000, 60, 0, 1, 1), (3000, 60, 0, 0, 0), (3000, 119, 0, 1, 0)])
+    (10000, 50, 0, 0, 1), (10000, 100, 0, 0, 0), (3000, 60, 0, 1, 1), (3000, 60, 0, 0, 0), (3000, 119, 0, 1, 0),
+    (1500, 20, 1, 0, 1), (1500, 80, 1, 0, 0), (600, 20, 1, 1, 0), (1000, 20, 1, 1, 1), (1000, 119, 1, 1, 0),
+    (1500, 100, 1, 1, 1), (1500, 10, 0, 1, 1)])
 def test_staged_recheck(plan, nrows, k, same, fp32, staged):
     assert plan.plan_staged_recheck(nrows, k, same, fp32) == staged
+
+
+@pytest.mark.parametrize("nrt,slots,nct,smax,best", [
+    (5, 304, 3, 8, (3,)), (13, 304, 7, 8, (7, 8)), (22, 304, 11, 8, (6, 8)), (32, 304, 16, 8, (8,)), (32, 152, 16, 8, (4, 8)),
+    (44, 304, 22, 8, (6,)), (1, 304, 188, 32, (32,)), (13, 152, 94, 32, (23,))])
+def test_segments(plan, nrt, slots, nct, smax, best):
+    assert plan.plan_choose_segments(nrt, slots, nct, smax) in best
+
+
+def test_segments_use_what_there_is(plan):
+    """Few tiles: a segment each, whatever share of the device they fill."""
+    for nct in range(1, 9):
+        for nrt in range(1, 8):
+            assert plan.plan_choose_segments(nrt, 304, nct, 8) == nct, (nrt, nct)
+
+
+@pytest.mark.parametrize("nref,natoms,k,skips", [
+    (1000, 60, 20, 0), (1600, 60, 20, 0), (1600, 200, 20, 0), (1600, 400, 20, 1), (1600, 1200, 20, 1), (1600, 1000, 60, 0),
+    (1450, 1200, 10, 1), (1450, 1200, 20, 0), (1200, 1200, 10, 0), (1740, 60, 20, 1), (1700, 1000, 60, 1)])
+def test_fp32_skips(plan, nref, natoms, k, skips):
+    assert plan.plan_fp32_skips(nref, natoms, k) == skips
+
+
+@pytest.mark.parametrize("n,natoms,k,segs", [(2200, 1200, 20, 2), (1800, 200, 20, 2), (1450, 1200, 10, 3), (2200, 60, 20, 5),
+                                             (2000, 1000, 80, 5), (4800, 400, 30, 5), (8000, 400, 20, 5)])
+def test_fp32_skip_segments(plan, n, natoms, k, segs):
+    """(5 stands for what choose_segments gave)"""
+    assert plan.plan_fp32_skip_segments((n + 31) // 32, 152, natoms, k, 5) == segs
 
 
 @pytest.mark.gpu
