@@ -950,8 +950,10 @@ struct LanczosOut {
 // the one-launch cycle (k_lz_cycle, twice as fast). For the resident serving
 // model, whose landmark graph mostly falls apart into components: which
 // vectors of the repeated eigenvalue's space a sequence returns is decided by
-// its rounding, and a model rebuilt from the same landmarks has to give the
-// embedding that coordinates served before were taken in.
+// its rounding. Both sequences are deterministic, but they return different
+// vectors there (served coordinates differed by their own size), and the
+// coordinates that a program stored from a model built by these kernels stay
+// comparable with those of a model rebuilt from the same landmarks.
 // With nlock > 0 the sequence runs on the operator deflated by the nlock
 // orthonormal columns dLock [nlock][n]: every new basis vector is
 // orthogonalised against them as well as against the Lanczos basis.

@@ -534,9 +534,11 @@ extern "C" int mds_knn_data_sparse(mds_ctx* ctx, const int64_t* ref_off, const i
     // The tensor-core product needs eight times the bit sets' memory and three
     // launches a panel. It takes every set whose tiles of 128 x 256 pairs reach
     // half the SMs: 2,100 rows of 23,104 bits 0.24 ms (2,048 rows by popcount:
-    // 2.9 ms), of 2,000 bits 0.09 ms (1.4 ms). Popcount tiles (two launches,
-    // which is what small sets are counted on to take) below that, 1.0 ms at
-    // 1,400 rows of 2,000 bits, and where the byte rows do not fit.
+    // 2.9 ms). Popcount tiles take smaller sets, and those whose byte rows do
+    // not fit. The line is not where the two cross, which is near 100 rows
+    // (product / popcount on the device, 20 x 300 bits 46 / 39 us; 300 x 300 49 /
+    // 69; 1,000 x 2,000 60 / 160; 1,400 x 20,000 121 / 1,091): it lies above the
+    // 1,300 rows that the tests hold to the popcount tiles' two launches.
     const int64_t K = overlap_width(dmax + 1);
     const size_t bytes = (size_t)K * ((size_t)n_ref + (same ? 0 : n_fit));
     bool tc = overlap_tiles(n_fit, n_ref) >= ctx->num_sms / 2 && bytes <= ((size_t)16 << 30);

@@ -4,7 +4,10 @@
 // The reference's distance of two binary vectors is sqrt(|A| + |B| - 2|A & B|)
 // bit for bit (knn_sparse.cu). The rows become e4m3 bytes (0 or 1.0), every
 // product is 0 or 1 and the FP32 accumulator holds integers below 2^24, so
-// the overlaps are exact whatever the order of the sums.
+// the overlaps are exact whatever the order of the sums (compared with counts
+// on the CPU up to overlaps of 5 million in rows of 10,000,003 indices, the
+// widest that 16 GiB of byte rows hold for the fewest rows that come here:
+// tests/test_overlap_range_gpu.py).
 //
 //  1. k_rows_e4m3    CSR rows -> byte rows [n][K], with the check that they
 //                    are binary (every value 1.0, indices strictly ascending).
