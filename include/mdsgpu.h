@@ -104,8 +104,8 @@ int mds_get_knn_stats(const mds_ctx* ctx, mds_knn_stats* out);
  *   call returns MDS_ERR_TIMEOUT.
  *   MDS_INJECT_OVERLAP_STALL: the next tensor-core product of binary vectors
  *   leaves out a load, so its bounded waits run out; MDS_ERR_TIMEOUT.
- *   MDS_INJECT_LANCZOS_STALL: a block of the next Lanczos cycle does not arrive
- *   at its grid barrier, whose waits run out; MDS_ERR_TIMEOUT.
+ *   MDS_INJECT_LANCZOS_STALL: the grid barrier of the next Lanczos cycle misses
+ *   an arrival, so its waits run out; MDS_ERR_TIMEOUT.
  * what = 0 disarms.
  */
 #define MDS_INJECT_SCREEN_STALL 0x1u

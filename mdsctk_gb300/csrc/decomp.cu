@@ -504,8 +504,6 @@ struct LzArgs {
   int* brk;
   unsigned* bar;     // arrivals at the grid barrier (zeroed before the launch)
   int* err;
-  int stall;         // (an injected fault for the failure-path tests: one block
-                     // never arrives at the grid barrier, so every wait runs out)
 };
 
 // Shared memory besides the basis: h, partial sums of the projections (at
@@ -526,8 +524,7 @@ __device__ __forceinline__ bool lz_grid_sync(const LzArgs& a, unsigned& arrivals
   if (threadIdx.x == 0) {
     int ok = 1;
     __threadfence();
-    if (!a.stall || blockIdx.x != 0)
-      asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.bar), "r"(1u) : "memory");
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(a.bar), "r"(1u) : "memory");
     const long long t0 = clock64();
     unsigned v;
     while (true) {
@@ -1161,9 +1158,14 @@ static int lanczos(mds_ctx* ctx, const SymOp& op, int nev, int ncv, double tol, 
         MDS_CUDA(ctx, cudaGetLastError());
       } else {
         MDS_CUDA(ctx, cudaMemsetAsync(sync.p, 0, 2 * sizeof(int), s));
+        if (ctx->inject & MDS_INJECT_LANCZOS_STALL) {
+          // an injected fault for the failure-path tests: the count starts one
+          // below zero, so a block's arrival is missing and every wait runs out
+          // (a block reads the count after its own arrival, so never below zero)
+          ctx->inject &= ~MDS_INJECT_LANCZOS_STALL;
+          MDS_CUDA(ctx, cudaMemsetAsync(sync.p, 0xff, sizeof(unsigned), s));
+        }
         lz.j0 = j0;
-        lz.stall = (ctx->inject & MDS_INJECT_LANCZOS_STALL) ? 1 : 0;
-        ctx->inject &= ~MDS_INJECT_LANCZOS_STALL;
         MDS_CUDA(ctx, cudaLaunchKernelEx(&cfg, k_lz_cycle, lz));
         ctx->stats.launches++;
       }

@@ -1328,10 +1328,13 @@ k_rc_finish(const float* __restrict__ rc, const float* __restrict__ Ur, int row0
 #define FR_AHEAD 2  // chunks in flight ahead of the one in use (the other stages let the warps drift apart)
 #define FR_SMEM (sizeof(float) * (FR_ST * FR_STAGE + 2 * FR_R * FR_C * 10 + FR_R * 24))
 
+// STALL: an injected fault for the failure-path tests (a test in the loop over
+// the chunks took 0.8% of a call).
+template <bool STALL>
 __global__ void __launch_bounds__(FR_THREADS, 1)
 k_full_rows(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUtensorMap tmR,
             const float* __restrict__ rc, const float* __restrict__ Ur, int nfit, int Nr, int Ap, int nofit, double* __restrict__ out_d,
-            int* __restrict__ out_i, int* __restrict__ err, int stall) {
+            int* __restrict__ out_i, int* __restrict__ err) {
   extern __shared__ __align__(128) float sm[];
   __shared__ uint64_t full[FR_ST], empty[FR_ST];
   __shared__ int s_abort;
@@ -1386,9 +1389,8 @@ k_full_rows(const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUt
         if (ok) load(issued++);
       }
       ok = __all_sync(0xffffffffu, ok && mbar_wait(&full[st], (n / FR_ST) & 1, &s_abort));
-      // (stall: an injected fault for the failure-path tests -- the last warp
-      // gives up on its last chunk, which every other warp still gets)
-      if (stall && warp == FR_THREADS / 32 - 1 && n == total - 1) ok = false;
+      // (the last warp gives up on its last chunk, which every other warp still gets)
+      if (STALL && warp == FR_THREADS / 32 - 1 && n == total - 1) ok = false;
       if (!ok) break;
       const float* xf = sf + st * FR_STAGE + rp * FR_FS;
       const float* yf = sf + st * FR_STAGE + (FR_R + cp) * FR_FS;
@@ -1640,13 +1642,14 @@ static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af,
     panel = (panel / 2 + FR_R - 1) / FR_R * FR_R;
   }
   const int ntile = (pl.nref + FR_C - 1) / FR_C;
-  static PerDevice attr;
-  size_t attr_limit = 0;
-  MDS_TRY(mds_allow_dyn_smem(ctx, k_full_rows, &attr, &attr_limit));
-  CUtensorMap mF, mR;
-  MDS_TRY(encode_map_f32(ctx, &mR, Ar, (int64_t)3 * pl.nref, pl.Ap, FR_KC, 3 * FR_C));
   const int stall = (ctx->inject & MDS_INJECT_FULL_STALL) ? 1 : 0;
   ctx->inject &= ~MDS_INJECT_FULL_STALL;
+  auto kernel = stall ? k_full_rows<true> : k_full_rows<false>;
+  static PerDevice attr[2];
+  size_t attr_limit = 0;
+  MDS_TRY(mds_allow_dyn_smem(ctx, kernel, &attr[stall], &attr_limit));
+  CUtensorMap mF, mR;
+  MDS_TRY(encode_map_f32(ctx, &mR, Ar, (int64_t)3 * pl.nref, pl.Ap, FR_KC, 3 * FR_C));
   for (int r0 = 0; r0 < nfit; r0 += panel) {
     const int nr = std::min(panel, nfit - r0), nrt = (nr + FR_R - 1) / FR_R;
     // column ranges so that there are about 8 blocks per SM
@@ -1654,9 +1657,9 @@ static int launch_full_rows(mds_ctx* ctx, const KnnRmsPlan& pl, const float* Af,
     MDS_TRY(encode_map_f32(ctx, &mF, Af + (int64_t)r0 * 3 * pl.Ap, (int64_t)3 * nr, pl.Ap, FR_KC, 3 * FR_R));
     ctx->stats.launches += 2;
     k_row_const<<<nr, RC_THREADS, 0, ctx->stream>>>(Af, mu, r0, pl.Ap, pl.natoms, pl.nofit, rc.as<float>());
-    k_full_rows<<<dim3(nrt, ny), FR_THREADS, FR_SMEM, ctx->stream>>>(
+    kernel<<<dim3(nrt, ny), FR_THREADS, FR_SMEM, ctx->stream>>>(
         mF, mR, rc.as<float>(), Ur, nr, pl.nref, pl.Ap, pl.nofit, out_d + (int64_t)r0 * pl.nref,
-        out_i + (int64_t)r0 * pl.nref, derr, stall);
+        out_i + (int64_t)r0 * pl.nref, derr);
     MDS_CUDA(ctx, cudaGetLastError());
   }
   return MDS_OK;
