@@ -462,6 +462,7 @@ static void worker_loop(mds_server* S) {
   }
 }
 
+// (without the recheck's stages)
 static size_t slot_bytes(const mds_server* S, int cap) {
   size_t ap = S->Ap;
   size_t b = 0;
@@ -471,7 +472,6 @@ static size_t slot_bytes(const mds_server* S, int cap) {
   b += (size_t)cap * S->nseg_max * S->segstride * 8 + (size_t)cap * S->nseg_max * 4;
   b += (size_t)cap * S->k * 12 + (size_t)cap * S->nev * 8 + (size_t)cap * 4;
   b += (size_t)cap * S->pv.nC * 4;                            // pivot bounds
-  if (staged_recheck(cap, S->k, false, S->prec == MDS_PREC_FP32)) b += recheck_scratch_bytes(cap);
   return b + (64u << 20);
 }
 
@@ -596,6 +596,11 @@ extern "C" int mds_server_create(const mds_server_config* cfg, const float* land
   int cap = S->cfg.max_batch_frames;
   size_t per = slot_bytes(S.get(), cap);
   int nslots = (int)std::max<size_t>(1, std::min<size_t>(budget / per, cfg->slots > 0 ? cfg->slots : 3));
+  // the recheck's stages where they leave the number of slots as it is (the
+  // block kernel otherwise)
+  const size_t per_staged = per + recheck_scratch_bytes(cap);
+  const bool staged = staged_recheck(cap, S->k, false, S->prec == MDS_PREC_FP32) && budget / per_staged >= (size_t)nslots;
+  if (staged) per = per_staged;
   for (int i = 0; i < nslots; ++i) S->slots.emplace_back();
   for (auto& sl : S->slots) {
     if ((rc = mds_create(cfg->device, 0, &sl.ctx))) return rc;
@@ -615,7 +620,7 @@ extern "C" int mds_server_create(const mds_server_config* cfg, const float* land
               sl.home.alloc(c, sizeof(int) * (cap / TC_FR_M + 1)) == MDS_OK &&
               (S->pv.nC == 0 || sl.lb.alloc(c, sizeof(float) * (size_t)S->pv.nC * cap) == MDS_OK) &&
               sl.ext.alloc(c, sizeof(double) * (size_t)cap * S->nev) == MDS_OK &&
-              (!staged_recheck(cap, S->k, false, S->prec == MDS_PREC_FP32) || recheck_scratch(c, cap, sl.rs) == MDS_OK);
+              (!staged || recheck_scratch(c, cap, sl.rs) == MDS_OK);
     if (!ok) {
       S->last_error = mds_last_error(c);
       return MDS_ERR_NOMEM;
